@@ -92,6 +92,8 @@ struct MGHierarchy {
   int small_kernel = 0;                          // mg_small_kernel of the configuration
   int apply_kernel = 2;                          // mixed_apply_kernel of the configuration
   SmallPlan small_plan{};                        // their split over the cluster's CTAs
+  bool resident = false;                         // the small levels fit the resident cycle
+  ResidentPlan res_plan{};                       // its layout
   void *small_plan_dev = nullptr;                // device copy of small_plan
   float omega = 0.9f;                            // damping of the block-Jacobi smoother
   float correction = 1.2f;                       // scaling of the coarse-grid correction

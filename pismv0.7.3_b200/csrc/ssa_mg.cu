@@ -1097,6 +1097,335 @@ __global__ void __cluster_dims__(SMALL_CLUSTER, 1, 1) __launch_bounds__(CTA_THRE
   cluster.sync();
 }
 
+// ---------------------------------------------------------------------------
+// The resident small-level cycle (ResidentPlan, ssa_small_plan.h): the L2-staged cycle above
+// is a chain of ten dependent steps, each waiting on two rounds of loads from L2 (D^-1 and b,
+// then the operator).  Here every operator is on chip before the right-hand side is read: the
+// lead CTA keeps its finest level's blocks in registers and the coarser levels' in shared
+// memory, so its steps run at shared-memory latency, and the first small level of a large
+// grid is spread over the other seven CTAs' registers, which compute the halo they need from
+// b themselves: two exchanges through distributed shared memory (the restricted residual to
+// the lead, its correction back) are all that crosses CTAs.
+//
+// Bound: latency, about 45 dependent shared-memory or shuffle rounds and the two cluster
+// exchanges; the data are 0.5 MB.  Whole fast solves with this cycle against the L2-staged one,
+// one B200: 101^2 57.6 against 68.8 ms, 801^2 93.2 / 101.7, FP64 at 401^2 207 / 240, eight
+// members at 401^2 314 / 367, the same bits.  Every item takes the arithmetic of k_mg_small_cycle in the
+// same order, so the results are the same bits.
+// ---------------------------------------------------------------------------
+struct SmallResident {
+  LevelView lev[MG_MAX_LEVELS];
+  ResidentPlan P;
+  const double *invT;   // dense inverse of the coarsest operator (transposed)
+  int n;                // unknowns of the coarsest level
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// y = A x from the nine blocks a(b) and the nine neighbour values x(b), in block order
+template <class AB, class XB>
+__device__ __forceinline__ float2 apply_blocks(const AB &a, const XB &x) {
+  float y1 = 0.0f, y2 = 0.0f;
+#pragma unroll
+  for (int b = 0; b < 9; ++b) {
+    const float4 ab = a(b);
+    const float2 xv = x(b);
+    y1 += ab.x * xv.x + ab.y * xv.y;
+    y2 += ab.z * xv.x + ab.w * xv.y;
+  }
+  return make_float2(y1, y2);
+}
+
+// the sum of an aggregate's four residuals, held by four neighbouring lanes
+__device__ __forceinline__ float2 aggregate_sum(float2 r) {
+  r.x += __shfl_xor_sync(0xffffffffu, r.x, 1);
+  r.y += __shfl_xor_sync(0xffffffffu, r.y, 1);
+  r.x += __shfl_xor_sync(0xffffffffu, r.x, 2);
+  r.y += __shfl_xor_sync(0xffffffffu, r.y, 2);
+  return r;
+}
+
+// omega v + corr c, rounded as the other cycles' omega * v + corr * c (the second product first);
+// written out because v's product is also a value of its own here
+__device__ __forceinline__ float2 up_iterate(float omega, const float2 &v, float corr, const float2 &c) {
+  return make_float2(__fmaf_rn(omega, v.x, __fmul_rn(corr, c.x)), __fmaf_rn(omega, v.y, __fmul_rn(corr, c.y)));
+}
+
+template <bool WIDE>
+__global__ void __cluster_dims__(WIDE ? SMALL_CLUSTER : 1, 1, 1) __launch_bounds__(SR_THREADS, 1)
+    k_mg_small_resident(const __grid_constant__ SmallResident S, float omega, float corr, const KState *st) {
+  extern __shared__ __align__(128) unsigned char sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int part = WIDE ? (int)cluster.block_rank() : 0;
+  const bool lead = part == 0;
+  const ResidentPlan &P = S.P;
+  if (WIDE) cluster_arrive();   // 0: this CTA runs, its shared memory may be written
+  const int lv = lead ? P.reg : P.first;   // the level this CTA holds in registers
+  const LevelView &L = S.lev[lv], &C = S.lev[lv + 1];
+  const int Mx = L.Mx, My = L.My;
+  auto vb = [&](int l) { return reinterpret_cast<float2 *>(sm + P.vec[l]); };   // lead: b of level l
+  auto vx = [&](int l) { return vb(l) + S.lev[l].N; };                         // its iterate
+  auto vz = [&](int l) { return vb(l) + 2 * S.lev[l].N; };                     // its smoothed iterate
+  // ---- before the right-hand side: this CTA's items, their operators, the staged levels ----
+  int b0 = 0, b1 = small_span(C.N), w0 = 0, nrows = Mx;
+  if (WIDE && !lead) {
+    small_chunk(small_span(C.N), SMALL_CLUSTER - 1, part - 1, 32, b0, b1);
+    if (b1 > b0) {
+      int r0, r1;
+      small_down_rows(L.ax, C.My, C.N, b0, b1, r0, r1);
+      small_window(Mx, r0, r1, w0, nrows);
+    } else {
+      nrows = 0;
+    }
+  }
+  const int nwin = WIDE && !lead ? nrows * My : 0;
+  float4 *const dw = reinterpret_cast<float4 *>(sm);                  // the others: D^-1 of the window,
+  float2 *const vw = reinterpret_cast<float2 *>(sm + 16 * nwin);      // D^-1 b,
+  float2 *const xw = reinterpret_cast<float2 *>(sm + 24 * nwin);      // and the iterate
+  float2 *const xs = lead ? vx(P.reg) : xw;
+  float4 a[SR_ITEMS][9], d[SR_ITEMS];
+  int cellk[SR_ITEMS], row[SR_ITEMS][3], col[SR_ITEMS][3], kcs[SR_ITEMS];   // cell (-1: none), neighbours
+#pragma unroll
+  for (int q = 0; q < SR_ITEMS; ++q) {
+    const int it = b0 + tid + q * SR_THREADS, kc = it >> 2, pi = (it >> 1) & 1, pj = it & 1;
+    const int I = kc / C.My, J = kc - I * C.My, i = I * L.ax + pi, j = J * L.ay + pj;
+    const bool ok = it < b1 && kc < C.N && pi < L.ax && pj < L.ay && i < Mx && j < My;
+    kcs[q] = it < b1 && kc < C.N ? kc : -1;
+    cellk[q] = ok ? i * My + j : -1;
+    const int ii[3] = {wrap(i - 1, Mx), i, wrap(i + 1, Mx)}, jj[3] = {wrap(j - 1, My), j, wrap(j + 1, My)};
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      int r = ii[s] - w0;
+      if (r < 0) r += Mx;
+      else if (r >= nrows) r -= Mx;
+      row[q][s] = r * My;
+      col[q][s] = jj[s];
+    }
+    const int k = ok ? cellk[q] : 0;
+#pragma unroll
+    for (int b = 0; b < 9; ++b) a[q][b] = L.A[b * L.N + k];
+    d[q] = L.dinv[k];
+  }
+  // the neighbour of item q in block b (NW N NE / W C E / SW S SE), in xs
+  auto at = [&](int q, int b) { return row[q][b % 3] + col[q][2 - b / 3]; };
+  double inv[2 * MG_MAX_COARSE_CELLS / (SR_THREADS / 32)];
+  if (lead) {
+    for (int l = P.reg + 1; l < P.last; ++l) {
+      const LevelView &F = S.lev[l], &G = S.lev[l + 1];
+      const int items = small_span(G.N);
+      if (tid < items) {
+        const int kc = tid >> 2, pi = (tid >> 1) & 1, pj = tid & 1;
+        const int I = kc / G.My, J = kc - I * G.My, i = I * F.ax + pi, j = J * F.ay + pj;
+        const bool ok = kc < G.N && pi < F.ax && pj < F.ay && i < F.Mx && j < F.My;
+        float4 *A = reinterpret_cast<float4 *>(sm + P.op[l]);
+        uint16_t *nb = reinterpret_cast<uint16_t *>(sm + P.nb[l]);
+        const int k = ok ? i * F.My + j : 0;
+#pragma unroll
+        for (int b = 0; b < 9; ++b) {
+          A[b * items + tid] = F.A[b * F.N + k];
+          const int ni = wrap(i + (b % 3) - 1, F.Mx), nj = wrap(j + 1 - b / 3, F.My);
+          nb[b * items + tid] = ok ? (uint16_t)(ni * F.My + nj) : (uint16_t)0xffffu;
+        }
+        A[9 * items + tid] = F.dinv[k];
+      }
+    }
+    // row r = warp (+ 16) of the coarsest inverse, one column a lane
+#pragma unroll
+    for (int q = 0; q < (int)(sizeof(inv) / sizeof(double)); ++q) {
+      const int r = warp + q * (SR_THREADS / 32);
+      inv[q] = r < S.n && lane < S.n ? S.invT[lane * S.n + r] : 0.0;
+    }
+  } else {
+    for (int q = tid; q < nwin; q += SR_THREADS) {
+      int k = w0 * My + q;
+      if (k < 0) k += L.N;
+      else if (k >= L.N) k -= L.N;
+      dw[q] = L.dinv[k];
+    }
+  }
+  if (WIDE) cluster_wait();
+  if (st && st->done) return;   // the same answer in every CTA
+  float2 bk[SR_ITEMS], v[SR_ITEMS];
+  if (WIDE && !lead) {
+    // ---- the first small level, down: x0 = omega D^-1 b on the window, R (b - A x0) to the lead ----
+#pragma unroll
+    for (int q = 0; q < SR_ITEMS; ++q) bk[q] = L.b[cellk[q] < 0 ? 0 : cellk[q]];
+#pragma unroll 2
+    for (int q = tid; q < nwin; q += SR_THREADS) {
+      int k = w0 * My + q;
+      if (k < 0) k += L.N;
+      else if (k >= L.N) k -= L.N;
+      const float2 t = fmul4(dw[q], L.b[k]);
+      vw[q] = t;
+      xw[q] = make_float2(omega * t.x, omega * t.y);
+    }
+    __syncthreads();
+    float2 *const bl = cluster.map_shared_rank(vb(P.reg), 0);
+#pragma unroll
+    for (int q = 0; q < SR_ITEMS; ++q) {
+      if (b0 + q * SR_THREADS >= b1) break;
+      float2 r = make_float2(0.0f, 0.0f);
+      if (cellk[q] >= 0) {
+        const float2 y = apply_blocks([&](int b) { return a[q][b]; }, [&](int b) { return xs[at(q, b)]; });
+        r = make_float2(bk[q].x - y.x, bk[q].y - y.y);
+      }
+      r = aggregate_sum(r);
+      if (kcs[q] >= 0 && (tid & 3) == 0) bl[kcs[q]] = r;
+    }
+    cluster_arrive();   // 1: the lead's b is complete
+    cluster_wait();
+    cluster_arrive();   // 2: the lead's correction is complete
+    cluster_wait();
+    // ---- up: x = omega D^-1 b + s P x_c; z = x + omega D^-1 (b - A x) ----
+    const float2 *const zl = cluster.map_shared_rank(vz(P.reg), 0);
+#pragma unroll 2
+    for (int q = tid; q < nwin; q += SR_THREADS) {
+      const int r = q / My, j = q - r * My;
+      int i = w0 + r;
+      if (i < 0) i += Mx;
+      else if (i >= Mx) i -= Mx;
+      const float2 t = vw[q], c = zl[(i / L.ax) * C.My + j / L.ay];
+      xw[q] = up_iterate(omega, t, corr, c);
+    }
+    cluster_arrive();   // 3: the lead's shared memory is no longer read
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < SR_ITEMS; ++q)
+      if (cellk[q] >= 0) {
+        const float2 xk = xs[at(q, 4)];
+        const float2 y = apply_blocks([&](int b) { return a[q][b]; }, [&](int b) { return xs[at(q, b)]; });
+        const float2 dd = fmul4(d[q], make_float2(bk[q].x - y.x, bk[q].y - y.y));
+        L.x[cellk[q]] = make_float2(xk.x + omega * dd.x, xk.y + omega * dd.y);
+      }
+    cluster_wait();
+    return;
+  }
+  // ---- the lead: its register level, down ----
+  if (WIDE) {
+    cluster_arrive();   // 1
+    cluster_wait();
+  }
+#pragma unroll
+  for (int q = 0; q < SR_ITEMS; ++q)
+    if (cellk[q] >= 0) {
+      bk[q] = WIDE ? vb(P.reg)[cellk[q]] : L.b[cellk[q]];
+      v[q] = fmul4(d[q], bk[q]);
+      xs[cellk[q]] = make_float2(omega * v[q].x, omega * v[q].y);
+    }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < SR_ITEMS; ++q) {
+    if (q * SR_THREADS >= b1) break;
+    float2 r = make_float2(0.0f, 0.0f);
+    if (cellk[q] >= 0) {
+      const float2 y = apply_blocks([&](int b) { return a[q][b]; }, [&](int b) { return xs[at(q, b)]; });
+      r = make_float2(bk[q].x - y.x, bk[q].y - y.y);
+    }
+    r = aggregate_sum(r);
+    if (kcs[q] >= 0 && (tid & 3) == 0) vb(P.reg + 1)[kcs[q]] = r;
+  }
+  __syncthreads();
+  // ---- the coarser levels, down ----
+  for (int l = P.reg + 1; l < P.last; ++l) {
+    const int items = small_span(S.lev[l + 1].N);
+    const float4 *A = reinterpret_cast<const float4 *>(sm + P.op[l]);
+    const uint16_t *nb = reinterpret_cast<const uint16_t *>(sm + P.nb[l]);
+    float2 *const x = vx(l);
+    float2 b = make_float2(0.0f, 0.0f);
+    int k = 0xffff;
+    if (tid < items) {
+      k = nb[4 * items + tid];
+      if (k != 0xffff) {
+        b = vb(l)[k];
+        const float2 t = fmul4(A[9 * items + tid], b);
+        x[k] = make_float2(omega * t.x, omega * t.y);
+      }
+    }
+    __syncthreads();
+    if (tid < items) {   // whole warps
+      float2 r = make_float2(0.0f, 0.0f);
+      if (k != 0xffff) {
+        const float2 y = apply_blocks([&](int q) { return A[q * items + tid]; },
+                                      [&](int q) { return x[nb[q * items + tid]]; });
+        r = make_float2(b.x - y.x, b.y - y.y);
+      }
+      r = aggregate_sum(r);
+      if ((tid & 3) == 0 && (tid >> 2) < S.lev[l + 1].N) vb(l + 1)[tid >> 2] = r;
+    }
+    __syncthreads();
+  }
+  // ---- the coarsest level: x = A^-1 b ----
+  {
+    const float *b = reinterpret_cast<const float *>(vb(P.last));
+    float *z = reinterpret_cast<float *>(vz(P.last));
+#pragma unroll
+    for (int q = 0; q < (int)(sizeof(inv) / sizeof(double)); ++q) {
+      const int r = warp + q * (SR_THREADS / 32);
+      if (r >= S.n) break;
+      double acc = 0.0;
+      if (lane < S.n) acc += inv[q] * (double)b[lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) z[r] = (float)acc;
+    }
+    __syncthreads();
+  }
+  // ---- up ----
+  for (int l = P.last - 1; l > P.reg; --l) {
+    const int items = small_span(S.lev[l + 1].N);
+    const float4 *A = reinterpret_cast<const float4 *>(sm + P.op[l]);
+    const uint16_t *nb = reinterpret_cast<const uint16_t *>(sm + P.nb[l]);
+    float2 *const x = vx(l);
+    float2 b = make_float2(0.0f, 0.0f), xk = b;
+    float4 dl = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int k = 0xffff;
+    if (tid < items) {
+      k = nb[4 * items + tid];
+      if (k != 0xffff) {
+        b = vb(l)[k];
+        dl = A[9 * items + tid];
+        const float2 t = fmul4(dl, b), c = vz(l + 1)[tid >> 2];
+        xk = up_iterate(omega, t, corr, c);
+        x[k] = xk;
+      }
+    }
+    __syncthreads();
+    if (k != 0xffff) {
+      const float2 y = apply_blocks([&](int q) { return A[q * items + tid]; },
+                                      [&](int q) { return x[nb[q * items + tid]]; });
+      const float2 dd = fmul4(dl, make_float2(b.x - y.x, b.y - y.y));
+      vz(l)[k] = make_float2(xk.x + omega * dd.x, xk.y + omega * dd.y);
+    }
+    __syncthreads();
+  }
+  // the lead's register level
+  float2 xk[SR_ITEMS];
+#pragma unroll
+  for (int q = 0; q < SR_ITEMS; ++q)
+    if (cellk[q] >= 0) {
+      xk[q] = up_iterate(omega, v[q], corr, vz(P.reg + 1)[kcs[q]]);
+      xs[cellk[q]] = xk[q];
+    }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < SR_ITEMS; ++q)
+    if (cellk[q] >= 0) {
+      const float2 y = apply_blocks([&](int b) { return a[q][b]; }, [&](int b) { return xs[at(q, b)]; });
+      const float2 dd = fmul4(d[q], make_float2(bk[q].x - y.x, bk[q].y - y.y));
+      const float2 z = make_float2(xk[q].x + omega * dd.x, xk[q].y + omega * dd.y);
+      if (WIDE) vz(P.reg)[cellk[q]] = z;
+      else L.x[cellk[q]] = z;
+    }
+  if (WIDE) {
+    cluster_arrive();   // 2
+    cluster_wait();
+    cluster_arrive();   // 3
+    cluster_wait();
+  }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1137,6 +1466,17 @@ int mg_plan(int Mx, int My, MGHierarchy &H) {
   H.small_smem = (int)sizeof(float2) *
                  std::max(small_window_cells(H.lev, H.small_first, H.nlev, SMALL_CLUSTER, CTA_THREADS),
                           small_window_cells(H.lev, H.small_first_wide, H.nlev, SMALL_CLUSTER, CTA_THREADS));
+  // the resident cycle when the levels fit its registers and shared memory
+  {
+    int mx[MG_MAX_LEVELS], my[MG_MAX_LEVELS], ax[MG_MAX_LEVELS], ay[MG_MAX_LEVELS];
+    for (int l = 0; l < H.nlev; ++l) {
+      mx[l] = H.lev[l].Mx;
+      my[l] = H.lev[l].My;
+      ax[l] = H.lev[l].ax;
+      ay[l] = H.lev[l].ay;
+    }
+    H.resident = resident_plan(H.small_first, H.nlev - 1, mx, my, ax, ay, SMALL_DSMEM_MAX_BYTES, H.res_plan);
+  }
   // the shared-memory cycle when every small level's block fits (ssa_small_plan.h)
   {
     int mx[SC_MAX_LEV], my[SC_MAX_LEV], ax[SC_MAX_LEV], ay[SC_MAX_LEV];
@@ -1197,6 +1537,10 @@ int mg_allocate(MGHierarchy &H, int fine_cells) {
     if (cudaMemcpy(H.views, v, sizeof(LevelView) * H.nlev, cudaMemcpyHostToDevice) != cudaSuccess) return 1;
   }
   if (raise_dynamic_smem((const void *)k_mg_small_cycle, H.small_smem) != 0) return 1;
+  if (H.resident && raise_dynamic_smem(H.res_plan.wide ? (const void *)k_mg_small_resident<true>
+                                                       : (const void *)k_mg_small_resident<false>,
+                                       H.res_plan.smem) != 0)
+    return 1;
   if (H.small_dsmem) {
     if (cudaMalloc(&H.small_plan_dev, sizeof(SmallPlan)) != cudaSuccess) return 1;
     if (cudaMemcpy(H.small_plan_dev, &H.small_plan, sizeof(SmallPlan), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1346,6 +1690,18 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     S.invT = H.cinv;
     S.n = 2 * H.lev[H.nlev - 1].N;
     k_mg_small_dsmem<<<SMALL_CLUSTER, CTA_THREADS, H.small_plan.smem, Lc.stream>>>(S, omega, corr, st);
+    ++launches;
+  } else if (H.resident && H.small_kernel != 2) {
+    // every level set that fits (all but grids with long thin small levels)
+    SmallResident S;
+    for (int l = H.res_plan.first; l < H.nlev; ++l) S.lev[l] = view(H.lev[l]);
+    S.P = H.res_plan;
+    S.invT = H.cinv;
+    S.n = 2 * H.lev[H.nlev - 1].N;
+    if (H.res_plan.wide)
+      k_mg_small_resident<true><<<SMALL_CLUSTER, SR_THREADS, H.res_plan.smem, Lc.stream>>>(S, omega, corr, st);
+    else
+      k_mg_small_resident<false><<<1, SR_THREADS, H.res_plan.smem, Lc.stream>>>(S, omega, corr, st);
     ++launches;
   } else {
     SmallLevels S;

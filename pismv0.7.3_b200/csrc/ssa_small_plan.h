@@ -139,4 +139,68 @@ SMALL_HD void small_down_rows(int ax, int Myc, int Nc, int b0, int b1, int &r0, 
   r1 = (k1 / Myc) * ax + ax - 1;
 }
 
+// The resident small-level cycle: every operator of the small levels is on chip before the
+// cycle's input arrives.  One CTA (the lead) holds level `reg` in registers (two items a
+// thread) and every coarser level in its shared memory; where the first small level has more
+// items than the lead can hold, the other SC_CTAS - 1 CTAs of a cluster hold that level in
+// registers and the lead starts one level below it (wide).  An item is one fine cell of an
+// aggregate, four per coarse cell, as in a down step above.
+constexpr int SR_THREADS = 512, SR_ITEMS = 2;
+constexpr int SR_MAX_LEV = 16;
+
+struct ResidentPlan {
+  int first, reg, last;   // levels: the first small one, the lead's register level, the coarsest
+  int wide;               // level first is held by the CTAs beside the lead (reg = first + 1)
+  int vec[SR_MAX_LEV];    // lead: byte offset of the level's b, x, z (float2, N each)
+  int op[SR_MAX_LEV];     // lead: byte offset of the level's nine blocks and D^-1 by item
+  int nb[SR_MAX_LEV];     // lead: byte offset of the level's neighbour table (9 x uint16 by item)
+  int smem;               // bytes of dynamic shared memory, the larger of the lead's and the others'
+};
+
+// Plan levels first .. last (sizes Mx, My, N = Mx My; aggregation ax, ay).  False where the
+// levels do not fit: the caller then stages them from L2 at every step.
+inline bool resident_plan(int first, int last, const int *Mx, const int *My, const int *ax, const int *ay,
+                          int max_smem, ResidentPlan &P) {
+  P = ResidentPlan{};
+  if (last >= SR_MAX_LEV || first >= last) return false;
+  auto cells = [&](int l) { return Mx[l] * My[l]; };
+  auto items = [&](int l) { return small_span(cells(l + 1)); };   // level l < last
+  const int cap = SR_THREADS * SR_ITEMS;
+  P.first = first;
+  P.last = last;
+  P.wide = items(first) > cap ? 1 : 0;
+  P.reg = first + P.wide;
+  if (P.reg >= last || items(P.reg) > cap) return false;
+  for (int l = first; l < last; ++l)
+    if (ax[l] < 1 || ax[l] > 2 || ay[l] < 1 || ay[l] > 2) return false;
+  int bytes = 0;
+  auto take = [&](int n) {
+    const int at = bytes;
+    bytes += (n + 15) / 16 * 16;
+    return at;
+  };
+  for (int l = P.reg; l <= last; ++l) P.vec[l] = take(3 * 8 * cells(l));
+  for (int l = P.reg + 1; l < last; ++l) {
+    if (items(l) > SR_THREADS || cells(l) >= 65535) return false;
+    P.op[l] = take(10 * 16 * items(l));
+    P.nb[l] = take(9 * 2 * items(l));
+  }
+  P.smem = bytes;
+  if (P.wide) {
+    const int parts = SC_CTAS - 1, span = items(first);
+    if ((span + parts - 1) / parts > cap) return false;
+    for (int c = 0; c < parts; ++c) {
+      int b0, b1, r0, r1, w0, nrows;
+      small_chunk(span, parts, c, 32, b0, b1);
+      if (b1 <= b0) continue;
+      if (b1 - b0 > cap) return false;
+      small_down_rows(ax[first], My[first + 1], cells(first + 1), b0, b1, r0, r1);
+      small_window(Mx[first], r0, r1, w0, nrows);
+      const int w = nrows * My[first] * (16 + 8 + 8);   // D^-1, D^-1 b and x of the window
+      if (w > P.smem) P.smem = w;
+    }
+  }
+  return P.smem <= max_smem;
+}
+
 }  // namespace pism_gpu
