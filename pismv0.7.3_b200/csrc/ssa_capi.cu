@@ -261,7 +261,7 @@ int run_iterations(pism_gpu_ssa *h, int kind, const void *x, int count, const ON
     cudaGraph_t graph = nullptr;
     bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
-      for (int q = 0; q < GRAPH_ITERS; ++q) one();
+      for (int q = 0; q < GRAPH_ITERS; ++q) one(0);
       ok = cudaStreamEndCapture(h->stream, &graph) == cudaSuccess && graph != nullptr;
     }
     if (ok) ok = cudaGraphInstantiate(&G.exec, graph, 0) == cudaSuccess;
@@ -282,13 +282,13 @@ int run_iterations(pism_gpu_ssa *h, int kind, const void *x, int count, const ON
       CK(h, cudaGraphLaunch(G.exec, h->stream));
       h->stats.kernel_launches += G.kernels;
     }
-  for (; q < count; ++q) one();
+  for (; q < count; ++q) one(0);
   return PISM_GPU_SSA_OK;
 }
 
 // A Krylov solve as one graph: a kernel sets a conditional handle from st->done, and a
-// WHILE node runs the loop body (one or a few iterations) plus that kernel again until the
-// solve is done, so the whole solve is one graph launch and one read-back.  Iterations of a
+// WHILE node runs the loop body (one or a few iterations, the last kernel of each setting the
+// handle again) until the solve is done, so the whole solve is one graph launch and one read-back.  Iterations of a
 // pass that start after convergence return at once.  Built once per handle and kind.
 template <class ONE>
 bool build_loop(pism_gpu_ssa *h, pism_gpu_ssa::LoopGraph &G, const KState *st, const ONE &one) {
@@ -325,8 +325,7 @@ bool build_loop(pism_gpu_ssa *h, pism_gpu_ssa::LoopGraph &G, const KState *st, c
                                              cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
     h->L.stream = bs;
-    one();
-    launch_loop_condition(h->L, cond, st);
+    one(cond);   // its last kernel sets the condition
     h->L.stream = s;
     const bool launched = cudaGetLastError() == cudaSuccess;
     ok = cudaStreamEndCapture(bs, nullptr) == cudaSuccess && launched;
@@ -359,9 +358,9 @@ int run_until_done(pism_gpu_ssa *h, int kind, const void *x, KState *st, int chu
   if (h->cfg.graphs >= 2 && !G.exec && !G.failed) {
     const long long before = h->stats.kernel_launches;
     long long per = 0;
-    G.failed = !build_loop(h, G, st, [&] {
+    G.failed = !build_loop(h, G, st, [&](cudaGraphConditionalHandle cond) {
       const long long b0 = h->stats.kernel_launches;
-      for (int q = 0; q < body_iters; ++q) one();
+      for (int q = 0; q < body_iters; ++q) one(cond);
       per = (h->stats.kernel_launches - b0) / body_iters;
     });
     G.x = x;
@@ -374,7 +373,7 @@ int run_until_done(pism_gpu_ssa *h, int kind, const void *x, KState *st, int chu
     CK(h, cudaMemcpyAsync(h->st_host, st, sizeof(KState), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     const long long passes = (h->st_host->iter + G.body_iters - 1) / G.body_iters;
-    h->stats.kernel_launches += 1 + passes * (G.body_iters * G.per_iteration + 1);
+    h->stats.kernel_launches += 1 + passes * G.body_iters * G.per_iteration;
     return PISM_GPU_SSA_OK;
   }
   // graphs == 0 (kernel profiling): one read-back per iteration, so that no iteration is
@@ -395,12 +394,12 @@ int run_until_done(pism_gpu_ssa *h, int kind, const void *x, KState *st, int chu
 // Inside an active capture on h->L.stream: add a conditional node (WHILE or IF) after the
 // capture's current dependencies.  `set(cond)` launches the kernel that gives the node its
 // value, once before the node and, for a WHILE node, again at the end of each pass of the
-// body; `body()` launches the body on h->L.stream (itself capturing into the node's body
-// graph, so bodies nest).  *body_kernels gets the kernels of one pass, nested bodies
+// body (unless body_sets: the body's last kernel does); `body(cond)` launches the body on
+// h->L.stream (itself capturing into the node's body graph, so bodies nest).  *body_kernels gets the kernels of one pass, nested bodies
 // included.  The capture continues after the node.
 template <class SET, class BODY>
 bool add_conditional(pism_gpu_ssa *h, cudaGraphConditionalNodeType type, const SET &set, const BODY &body,
-                     long long *body_kernels) {
+                     long long *body_kernels, bool body_sets = false) {
   const cudaStream_t s = h->L.stream;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaGraph_t cg = nullptr;
@@ -427,8 +426,8 @@ bool add_conditional(pism_gpu_ssa *h, cudaGraphConditionalNodeType type, const S
   if (ok) {
     const long long b0 = h->stats.kernel_launches;
     h->L.stream = bs;
-    ok = body();
-    if (type == cudaGraphCondTypeWhile) set(cond);
+    ok = body(cond);
+    if (type == cudaGraphCondTypeWhile && !body_sets) set(cond);
     h->L.stream = s;
     *body_kernels = h->stats.kernel_launches - b0;
     ok = cudaGetLastError() == cudaSuccess && ok;
@@ -509,7 +508,7 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
     return [&h, flag](cudaGraphConditionalHandle cond) { launch_flag_condition(h->L, cond, flag, true); };
   };
   const long long before_loop = h->stats.kernel_launches;
-  bool ok = add_conditional(h, cudaGraphCondTypeWhile, not_done(&P->done), [&] {
+  bool ok = add_conditional(h, cudaGraphCondTypeWhile, not_done(&P->done), [&](cudaGraphConditionalHandle) {
     bool inner_ok = true, rebuild_ok = true;
     launch_picard_begin(h->L, P, pc, h->zd_dev);
     bool residual_queued = false;
@@ -537,7 +536,7 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
       rebuild_ok = add_conditional(
           h, cudaGraphCondTypeIf,
           [&](cudaGraphConditionalHandle cond) { launch_flag_condition(h->L, cond, &P->rebuild, false); },
-          [&] {
+          [&](cudaGraphConditionalHandle) {
             mg_setup_coarse(h->L, g, f, h->mg);
             return true;
           },
@@ -549,21 +548,21 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
     if (line) line_setup(h->L, g, f, h->K.dinv, h->line);
     if (mixed) {
       if (!residual_queued) launch_residual32(h->L, g, f, h->rhs, h->vel, h->K32.rhs, h->res_dev);
-      inner_ok = add_conditional(h, cudaGraphCondTypeWhile, not_done(&P->refine_done), [&] {
+      inner_ok = add_conditional(h, cudaGraphCondTypeWhile, not_done(&P->refine_done), [&](cudaGraphConditionalHandle) {
         launch_mixed_init_dev(h->L, N, h->K32, h->res_dev, &P->rtol, c.mixed_inner_rtol, c.ksp_max_it);
         bool ok2 = add_conditional(
             h, cudaGraphCondTypeWhile,
             [&](cudaGraphConditionalHandle cond) { launch_loop_condition(h->L, cond, h->K32.st); },
-            [&] {
-              launch_mixed_iteration(h->L, g, f, *mg, h->K32);
+            [&](cudaGraphConditionalHandle cond) {
+              launch_mixed_iteration(h->L, g, f, *mg, h->K32, cond);
               return true;
             },
-            &inc_inner);
+            &inc_inner, true);
         launch_refine_end(h->L, P, h->K32.st, 60);
         ok2 = ok2 && add_conditional(
                          h, cudaGraphCondTypeIf,
                          [&](cudaGraphConditionalHandle cond) { launch_flag_condition(h->L, cond, &P->go, false); },
-                         [&] {
+                         [&](cudaGraphConditionalHandle) {
                            launch_axpy32(h->L, N, h->K32.d, h->vel);
                            launch_residual32(h->L, g, f, h->rhs, h->vel, h->K32.rhs, h->res_dev);
                            return true;
@@ -577,15 +576,15 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
       inner_ok = add_conditional(
           h, cudaGraphCondTypeWhile,
           [&](cudaGraphConditionalHandle cond) { launch_loop_condition(h->L, cond, h->K.st); },
-          [&] {
-            for (int q = 0; q < 4; ++q) launch_bicg_iteration(h->L, g, f, h->K, h->vel, mg, line);
+          [&](cudaGraphConditionalHandle cond) {
+            for (int q = 0; q < 4; ++q) launch_bicg_iteration(h->L, g, f, h->K, h->vel, mg, line, cond);
             return true;
           },
-          &inc_inner);
+          &inc_inner, true);
       launch_ksp_end(h->L, P, h->K.st, 4);
     }
     launch_picard_after_solve(h->L, P, h->zd_dev);
-    inner_ok = inner_ok && add_conditional(h, cudaGraphCondTypeIf, not_done(&P->done), [&] {
+    inner_ok = inner_ok && add_conditional(h, cudaGraphCondTypeIf, not_done(&P->done), [&](cudaGraphConditionalHandle) {
       launch_nuH(h->L, g, c, f, reg, underrelax, true, h->norm_dev);
       launch_picard_test(h->L, P, h->norm_dev, pc);
       return true;
@@ -707,7 +706,7 @@ int linear_solve(pism_gpu_ssa *h, double2 *x, double rtol, int *its_out, int *st
   const int kind = mg ? GRAPH_BICG_MG : line ? GRAPH_BICG_LINE : GRAPH_BICG_JACOBI;
   // long FP64 solves: four iterations per pass of the loop body
   RET(run_until_done(h, kind, x, h->K.st, std::max(8, (int)(0.8 * h->last_ksp_its)), 4,
-                     [&] { launch_bicg_iteration(h->L, g, f, h->K, x, mg, line); }));
+                     [&](cudaGraphConditionalHandle cond) { launch_bicg_iteration(h->L, g, f, h->K, x, mg, line, cond); }));
   h->last_ksp_its = h->st_host->iter;
   *its_out = h->st_host->iter;
   *status_out = h->st_host->status;
@@ -822,7 +821,7 @@ int linear_solve_mixed(pism_gpu_ssa *h, double2 *x, double rtol, int *its_out, i
     launch_mixed_init(h->L, g.Mx * g.My, h->K32, h->res_dev, rtol, h->cfg.mixed_inner_rtol, h->cfg.ksp_max_it);
     // short inner solves (a few iterations each): one iteration per pass
     RET(run_until_done(h, GRAPH_MIXED, nullptr, h->K32.st, 8, 1,
-                       [&] { launch_mixed_iteration(h->L, g, f, *mg, h->K32); }));
+                       [&](cudaGraphConditionalHandle cond) { launch_mixed_iteration(h->L, g, f, *mg, h->K32, cond); }));
     const double rn = sqrt(h->st_host->outer_r2), bn = sqrt(h->st_host->outer_b2);
     h->stats.final_linear_residual = bn > 0 ? rn / bn : rn;
     if (!std::isfinite(rn)) { status = KSP_NAN; break; }

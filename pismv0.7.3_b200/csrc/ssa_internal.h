@@ -129,8 +129,9 @@ void launch_apply(const Launch &L, const GridDev &g, const Fields &f, const doub
 void launch_diag_setup(const Launch &L, const GridDev &g, const Fields &f, double4 *dinv, int *zero_diag_cell);
 void launch_bicg_init(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, const double2 *b,
                       const double2 *x);
+// (cond: the WHILE condition of a graph-resident loop, set by the iteration's last kernel; 0: none)
 void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
-                           const MGHierarchy *mg, const LinePC *line);
+                           const MGHierarchy *mg, const LinePC *line, cudaGraphConditionalHandle cond = 0);
 // FGMRES: r0 = b - A x into V0 (init) / after a restart; one Arnoldi step j; the end of a cycle
 void launch_gmres_residual(const Launch &L, const GridDev &g, const Fields &f, const Gmres &G, const double2 *b,
                            const double2 *x, int init);
@@ -219,7 +220,7 @@ void launch_loop_condition(const Launch &L, cudaGraphConditionalHandle cond, con
 void launch_mixed_init(const Launch &L, int N, const Krylov32 &K, const double *res2, double outer_rtol,
                        double inner_min, int maxit);
 void launch_mixed_iteration(const Launch &L, const GridDev &g, const Fields &f, const MGHierarchy &H,
-                            const Krylov32 &K);
+                            const Krylov32 &K, cudaGraphConditionalHandle cond = 0);
 // r32 = (float) (b - A x) with FP64 arithmetic; out2 = {||b - A x||^2, ||b||^2}
 void launch_residual32(const Launch &L, const GridDev &g, const Fields &f, const double2 *b, const double2 *x,
                        float2 *r32, double *out2);

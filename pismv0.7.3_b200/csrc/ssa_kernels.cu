@@ -12,6 +12,7 @@
 #include <cstdio>
 
 #include "ssa_internal.h"
+#include "ssa_pdl.cuh"
 #include "ssa_stencil.cuh"
 #include "ssa_reduce.cuh"
 
@@ -564,10 +565,15 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_init(GridDev g, TileMap tm, Sten
 // p = r + beta (p - omega v);  phat = M^-1 p (block Jacobi; with multigrid phat is
 // written by the V-cycle instead)
 template <bool JAC>
-__global__ void __launch_bounds__(NT) k_bicg_p(int N, const double2 *__restrict__ r, const double2 *__restrict__ v,
-                                               const double4 *__restrict__ dinv, double2 *__restrict__ p,
-                                               double2 *__restrict__ phat, const KState *st) {
+__global__ void __launch_bounds__(NT) k_bicg_p(int N, const double2 *r_, const double2 *v_,
+                                               const double4 *__restrict__ dinv, double2 *p_, double2 *phat_,
+                                               const KState *st_) {
+  pdl_wait();
+  const KState *st = after_wait(st_);
   if (st->done) return;
+  pdl_release();
+  const double2 *__restrict__ r = after_wait(r_), *__restrict__ v = after_wait(v_);
+  double2 *__restrict__ p = after_wait(p_), *__restrict__ phat = after_wait(phat_);
   const double bta = st->beta, om = st->omega;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 rk = r[k], pk = p[k], vk = v[k];
@@ -580,10 +586,14 @@ __global__ void __launch_bounds__(NT) k_bicg_p(int N, const double2 *__restrict_
 // v = A phat; alpha = rho / (rhat . v)
 __global__ void __launch_bounds__(NT, 4) k_bicg_v(GridDev g, TileMap tm, StencilConst s, const uint32_t *__restrict__ flags,
                                                const double2 *__restrict__ nuH, const double *__restrict__ beta,
-                                               const double2 *__restrict__ phat, const double2 *__restrict__ rhat,
-                                               double2 *__restrict__ v, double *partials, unsigned *ticket,
-                                               KState *st) {
+                                               const double2 *phat_, const double2 *rhat_, double2 *v_,
+                                               double *partials, unsigned *ticket, KState *st_) {
+  pdl_wait();
+  KState *st = after_wait(st_);
   if (st->done) return;
+  pdl_release();
+  const double2 *__restrict__ phat = after_wait(phat_), *__restrict__ rhat = after_wait(rhat_);
+  double2 *__restrict__ v = after_wait(v_);
   double acc[1] = {0.0};
   __shared__ HaloTile<double2> xT, nT;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -609,10 +619,15 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_v(GridDev g, TileMap tm, Stencil
 
 // s = r - alpha v;  shat = M^-1 s
 template <bool JAC>
-__global__ void __launch_bounds__(NT) k_bicg_s(int N, const double2 *__restrict__ r, const double2 *__restrict__ v,
-                                               const double4 *__restrict__ dinv, double2 *__restrict__ sv,
-                                               double2 *__restrict__ shat, const KState *st) {
+__global__ void __launch_bounds__(NT) k_bicg_s(int N, const double2 *r_, const double2 *v_,
+                                               const double4 *__restrict__ dinv, double2 *sv_, double2 *shat_,
+                                               const KState *st_) {
+  pdl_wait();
+  const KState *st = after_wait(st_);
   if (st->done) return;
+  pdl_release();
+  const double2 *__restrict__ r = after_wait(r_), *__restrict__ v = after_wait(v_);
+  double2 *__restrict__ sv = after_wait(sv_), *__restrict__ shat = after_wait(shat_);
   const double al = st->alpha;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 rk = r[k], vk = v[k];
@@ -625,10 +640,14 @@ __global__ void __launch_bounds__(NT) k_bicg_s(int N, const double2 *__restrict_
 // t = A shat; omega = (t . s) / (t . t)
 __global__ void __launch_bounds__(NT, 4) k_bicg_t(GridDev g, TileMap tm, StencilConst s, const uint32_t *__restrict__ flags,
                                                const double2 *__restrict__ nuH, const double *__restrict__ beta,
-                                               const double2 *__restrict__ shat, const double2 *__restrict__ sv,
-                                               double2 *__restrict__ tv, double *partials, unsigned *ticket,
-                                               KState *st) {
+                                               const double2 *shat_, const double2 *sv_, double2 *tv_,
+                                               double *partials, unsigned *ticket, KState *st_) {
+  pdl_wait();
+  KState *st = after_wait(st_);
   if (st->done) return;
+  pdl_release();
+  const double2 *__restrict__ shat = after_wait(shat_), *__restrict__ sv = after_wait(sv_);
+  double2 *__restrict__ tv = after_wait(tv_);
   double acc[2] = {0.0, 0.0};
   __shared__ HaloTile<double2> xT, nT;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -646,14 +665,24 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_t(GridDev g, TileMap tm, Stencil
   if (grid_reduce<2>(acc, partials, ticket, tot)) st->omega = (tot[1] != 0.0) ? tot[0] / tot[1] : 0.0;
 }
 
-// x += alpha phat + omega shat;  r = s - omega t;  convergence test
-__global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *__restrict__ phat, const double2 *__restrict__ shat,
-                                               const double2 *__restrict__ sv, const double2 *__restrict__ tv,
-                                               const double2 *__restrict__ rhat, double2 *__restrict__ x,
-                                               double2 *__restrict__ r, double *partials, unsigned *ticket,
-                                               KState *st) {
-  if (st->done) return;
+// x += alpha phat + omega shat;  r = s - omega t;  convergence test, and the WHILE condition
+// of a graph-resident loop (cond, 0: none)
+__global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *phat_, const double2 *shat_, const double2 *sv_,
+                                               const double2 *tv_, const double2 *rhat_, double2 *x_, double2 *r_,
+                                               double *partials, unsigned *ticket, KState *st_,
+                                               cudaGraphConditionalHandle cond) {
+  pdl_wait();
+  KState *st = after_wait(st_);
+  if (st->done) {
+    if (cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
+    return;
+  }
+  pdl_release();
   const double al = st->alpha, om = st->omega;
+  const double2 *__restrict__ phat = after_wait(phat_), *__restrict__ shat = after_wait(shat_);
+  const double2 *__restrict__ sv = after_wait(sv_), *__restrict__ tv = after_wait(tv_);
+  const double2 *__restrict__ rhat = after_wait(rhat_);
+  double2 *__restrict__ x = after_wait(x_), *__restrict__ r = after_wait(r_);
   double acc[2] = {0.0, 0.0};
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 ph = phat[k], sh = shat[k], sk = sv[k], tk = tv[k];
@@ -672,18 +701,22 @@ __global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *__restrict_
     st->rnorm2 = tot[1];
     st->iter += 1;
     const double rn = sqrt(tot[1]), tol = st->rtol * sqrt(st->bnorm2);
+    int done = 1;
     if (!isfinite(rn)) {
-      st->done = 1; st->status = KSP_NAN;
+      st->status = KSP_NAN;
     } else if (rn <= tol) {
-      st->done = 1; st->status = 0;
+      st->status = 0;
     } else if (st->iter >= st->maxit) {
-      st->done = 1; st->status = KSP_MAXIT;
+      st->status = KSP_MAXIT;
     } else if (om == 0.0 || rho_new == 0.0) {
-      st->done = 1; st->status = KSP_BREAKDOWN;
+      st->status = KSP_BREAKDOWN;
     } else {
+      done = 0;
       st->beta = (rho_new / st->rho) * (al / om);
       st->rho = rho_new;
     }
+    st->done = done;
+    if (cond) cudaGraphSetConditional(cond, done ? 0u : 1u);
   }
 }
 
@@ -822,34 +855,23 @@ void launch_bicg_init(const Launch &L, const GridDev &g, const Fields &f, const 
 }
 
 void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
-                           const MGHierarchy *mg, const LinePC *line) {
+                           const MGHierarchy *mg, const LinePC *line, cudaGraphConditionalHandle cond) {
   L.tick(5);
   TileMap tm = make_tiles(g);
   const int N = g.Mx * g.My;
   const StencilConst s = stencil_const(g, f);
   const int bt = grid_for_tiles(L, tm.tiles), bv = grid_for(L, N);
-  if (mg) {
-    k_bicg_p<false><<<bv, NT, 0, L.stream>>>(N, K.r, K.v, K.dinv, K.p, K.phat, K.st);
-    mg_vcycle(L, g, f, *mg, K.p, K.phat, K.st);
-  } else if (line) {
-    k_bicg_p<false><<<bv, NT, 0, L.stream>>>(N, K.r, K.v, K.dinv, K.p, K.phat, K.st);
-    line_apply(L, g, *line, K.p, K.phat, K.st);
-  } else {
-    k_bicg_p<true><<<bv, NT, 0, L.stream>>>(N, K.r, K.v, K.dinv, K.p, K.phat, K.st);
-  }
-  k_bicg_v<<<bt, NT, 0, L.stream>>>(g, tm, s, f.flags, f.nuH, f.beta, K.phat, K.rhat, K.v, L.partials, L.ticket,
-                                    K.st);
-  if (mg) {
-    k_bicg_s<false><<<bv, NT, 0, L.stream>>>(N, K.r, K.v, K.dinv, K.s, K.shat, K.st);
-    mg_vcycle(L, g, f, *mg, K.s, K.shat, K.st);
-  } else if (line) {
-    k_bicg_s<false><<<bv, NT, 0, L.stream>>>(N, K.r, K.v, K.dinv, K.s, K.shat, K.st);
-    line_apply(L, g, *line, K.s, K.shat, K.st);
-  } else {
-    k_bicg_s<true><<<bv, NT, 0, L.stream>>>(N, K.r, K.v, K.dinv, K.s, K.shat, K.st);
-  }
-  k_bicg_t<<<bt, NT, 0, L.stream>>>(g, tm, s, f.flags, f.nuH, f.beta, K.shat, K.s, K.t, L.partials, L.ticket, K.st);
-  k_bicg_x<<<bv, NT, 0, L.stream>>>(N, K.phat, K.shat, K.s, K.t, K.rhat, x, K.r, L.partials, L.ticket, K.st);
+  const bool jac = !mg && !line;
+  launch_pdl(L, jac ? k_bicg_p<true> : k_bicg_p<false>, bv, NT, 0, N, K.r, K.v, K.dinv, K.p, K.phat, K.st);
+  if (mg) mg_vcycle(L, g, f, *mg, K.p, K.phat, K.st);
+  else if (line) line_apply(L, g, *line, K.p, K.phat, K.st);
+  launch_pdl(L, k_bicg_v, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.phat, K.rhat, K.v, L.partials, L.ticket,
+             K.st);
+  launch_pdl(L, jac ? k_bicg_s<true> : k_bicg_s<false>, bv, NT, 0, N, K.r, K.v, K.dinv, K.s, K.shat, K.st);
+  if (mg) mg_vcycle(L, g, f, *mg, K.s, K.shat, K.st);
+  else if (line) line_apply(L, g, *line, K.s, K.shat, K.st);
+  launch_pdl(L, k_bicg_t, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.shat, K.s, K.t, L.partials, L.ticket, K.st);
+  launch_pdl(L, k_bicg_x, bv, NT, 0, N, K.phat, K.shat, K.s, K.t, K.rhat, x, K.r, L.partials, L.ticket, K.st, cond);
 }
 
 void launch_residual32(const Launch &L, const GridDev &g, const Fields &f, const double2 *b, const double2 *x,

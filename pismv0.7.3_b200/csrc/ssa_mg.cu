@@ -36,6 +36,7 @@
 
 #include "ssa_fine32.cuh"
 #include "ssa_krylov32.cuh"
+#include "ssa_pdl.cuh"
 #include "ssa_small_plan.h"
 
 namespace pism_gpu {
@@ -443,7 +444,9 @@ __device__ __forceinline__ void store_aggregates(float2 (&rsh)[TILE_I][TILE_J], 
 template <int AX, int AY, class BA>
 __global__ void __launch_bounds__(NTm) k_mg0_restrict(FineF F, BA b_in, float omega, int Mxc,
                                                       int Myc, TileM tm, float2 *__restrict__ bc, const KState *st) {
+  pdl_wait();
   if (st && st->done) return;
+  pdl_release();
   const auto b = b_in.bind();
   __shared__ HaloTile<float2> xT, nT;
   __shared__ float2 rsh[TILE_I][TILE_J];
@@ -479,9 +482,12 @@ __global__ void __launch_bounds__(NTm) k_mg0_restrict(FineF F, BA b_in, float om
 // fine level: x = omega D^-1 b + s P x_1;  z = x + omega D^-1 (b - A x)
 template <int AX, int AY, class BA, class ZV>
 __global__ void __launch_bounds__(NTm) k_mg0_post(FineF F, BA b_in, float omega, float corr,
-                                                  int Myc, const float2 *__restrict__ xc, TileM tm,
+                                                  int Myc, const float2 *xc_, TileM tm,
                                                   ZV *__restrict__ z, const KState *st) {
+  pdl_wait();
   if (st && st->done) return;
+  pdl_release();
+  const float2 *__restrict__ xc = after_wait(xc_);
   const auto b = b_in.bind();
   __shared__ HaloTile<float2> xT, nT;
   const GridDev &g = F.g;
@@ -524,9 +530,12 @@ constexpr int H2I = TIm + 4, H2J = TJm + 4;   // the two-cell-halo region of a t
 
 template <int AX, int AY, class BA, class EPI>
 __global__ void __launch_bounds__(NTm) k_mg0_post_apply(FineF F, BA b_in, float omega, float corr, int Myc,
-                                                        const float2 *__restrict__ xc, TileM tm,
+                                                        const float2 *xc_, TileM tm,
                                                         float2 *__restrict__ z, EPI e) {
+  pdl_wait();
   if (e.st->done) return;
+  pdl_release();
+  const float2 *__restrict__ xc = after_wait(xc_);
   e.begin();
   const auto b = b_in.bind();
   __shared__ float2 xs[H2I][H2J], ns[H2I][H2J], zs[TIm + 2][TJm + 2];
@@ -568,29 +577,59 @@ __global__ void __launch_bounds__(NTm) k_mg0_post_apply(FineF F, BA b_in, float 
   e.finish();
 }
 
-// coarse level l: b_{l+1} = R (b_l - A_l x0), x0 = omega D^-1 b_l
+// The halo element of a tile that thread (ti, tj) loads beside its own cell (load_halo_tile's
+// assignment): its place (ha, hb) in the tile, ha < 0 for none, and its wrapped cell.
+struct HaloCell {
+  int ha, hb, q;
+};
+__device__ __forceinline__ HaloCell halo_cell(int i0, int j0, int Mx, int My) {
+  const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
+  HaloCell h{-1, 0, 0};
+  if (ti < 2) {
+    h.ha = ti == 0 ? 0 : TILE_I + 1;
+    h.hb = tj;
+  } else if (ti < 4 && tj < 2) {
+    h.ha = ti == 2 ? 0 : TILE_I + 1;
+    h.hb = 32 + tj;
+  } else if (ti < 6 && tj < TILE_I) {
+    h.ha = tj + 1;
+    h.hb = ti == 4 ? 0 : TILE_J + 1;
+  }
+  if (h.ha >= 0) h.q = pmod(i0 - 1 + h.ha, Mx) * My + pmod(j0 - 1 + h.hb, My);
+  return h;
+}
+
+// coarse level l: b_{l+1} = R (b_l - A_l x0), x0 = omega D^-1 b_l.  Of a block's first tile the
+// operator (nine blocks and D^-1, 160 of the 170 B a cell) is read before the wait for the
+// kernel that writes b_l.
 template <int AX, int AY>
-__global__ void __launch_bounds__(NTm) k_mgc_restrict(LevelView L, float omega, int Mxc, int Myc, TileM tm,
-                                                      float2 *__restrict__ bc, const KState *st) {
-  if (st && st->done) return;
+__global__ void __launch_bounds__(NTm, 4) k_mgc_restrict(LevelView L, float omega, int Mxc, int Myc, TileM tm,
+                                                         float2 *__restrict__ bc, const KState *st) {
   __shared__ HaloTile<float2> xT;
   __shared__ float2 rsh[TILE_I][TILE_J];
   const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
+  bool first = true;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
     const int i0 = (t / tm.tiles_j) * TILE_I, j0 = (t % tm.tiles_j) * TILE_J;
     const int i = i0 + ti, j = j0 + tj;
     const bool inside = i < L.Mx && j < L.My;
-    const int k = inside ? i * L.My + j : 0;
-    float4 a[9];   // issued with the tile loads: one round trip per tile
+    const int q = pmod(i, L.Mx) * L.My + pmod(j, L.My);   // a cell past the edge wraps
+    const HaloCell hc = halo_cell(i0, j0, L.Mx, L.My);
+    float4 a[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) a[q] = L.A[q * L.N + k];
-    const float2 bk = L.b[k];
+    for (int n = 0; n < 9; ++n) a[n] = L.A[n * L.N + q];
+    const float4 dq = L.dinv[q], dh = L.dinv[hc.q];
+    if (first) {
+      pdl_wait();
+      if (st && st->done) return;
+      pdl_release();
+      first = false;
+    }
+    const float2 bk = L.b[q], bh = L.b[hc.q];
+    const float2 v = fmul4(dq, bk), vh = fmul4(dh, bh);
     __syncthreads();
-    load_halo_tile<float2>(xT, i0, j0, L.Mx, L.My, [&](int ii, int jj) {
-      const int q = ii * L.My + jj;
-      const float2 v = fmul4(L.dinv[q], L.b[q]);
-      return make_float2(omega * v.x, omega * v.y);
-    });
+    xT[ti + 1][tj + 1] = make_float2(omega * v.x, omega * v.y);
+    if (hc.ha >= 0) xT[hc.ha][hc.hb] = make_float2(omega * vh.x, omega * vh.y);
     __syncthreads();
     float2 r = make_float2(0.0f, 0.0f);
     if (inside) {
@@ -603,36 +642,43 @@ __global__ void __launch_bounds__(NTm) k_mgc_restrict(LevelView L, float omega, 
   }
 }
 
-// coarse level l: x = omega D^-1 b + s P x_{l+1};  x <- x + omega D^-1 (b - A x)
+// coarse level l: x = omega D^-1 b + s P x_{l+1};  x <- x + omega D^-1 (b - A x).  Of a block's
+// first tile everything but x_{l+1} is read before the wait (b_l was written on the way down).
 template <int AX, int AY>
-__global__ void __launch_bounds__(NTm) k_mgc_post(LevelView L, float omega, float corr, int Myc,
-                                                  const float2 *__restrict__ xc, TileM tm, const KState *st) {
-  if (st && st->done) return;
+__global__ void __launch_bounds__(NTm, 4) k_mgc_post(LevelView L, float omega, float corr, int Myc,
+                                                     const float2 *xc, TileM tm, const KState *st) {
   __shared__ HaloTile<float2> xT;
   const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
+  bool first = true;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
     const int i0 = (t / tm.tiles_j) * TILE_I, j0 = (t % tm.tiles_j) * TILE_J;
     const int i = i0 + ti, j = j0 + tj;
     const bool inside = i < L.Mx && j < L.My;
-    const int k = inside ? i * L.My + j : 0;
-    float4 a[9];   // issued with the tile loads: one round trip per tile
+    const int iw = pmod(i, L.Mx), jw = pmod(j, L.My), q = iw * L.My + jw;
+    const HaloCell hc = halo_cell(i0, j0, L.Mx, L.My);
+    const int hi = hc.q / L.My, hj = hc.q - hi * L.My;
+    float4 a[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) a[q] = L.A[q * L.N + k];
-    const float2 bk = L.b[k];
-    const float4 dk = L.dinv[k];
+    for (int n = 0; n < 9; ++n) a[n] = L.A[n * L.N + q];
+    const float2 bk = L.b[q], bh = L.b[hc.q];
+    const float4 dk = L.dinv[q], dh = L.dinv[hc.q];
+    const float2 v = fmul4(dk, bk), vh = fmul4(dh, bh);
+    if (first) {
+      pdl_wait();
+      if (st && st->done) return;
+      pdl_release();
+      first = false;
+    }
+    const float2 c = xc[(iw / AX) * Myc + jw / AY], ch = xc[(hi / AX) * Myc + hj / AY];
     __syncthreads();
-    load_halo_tile<float2>(xT, i0, j0, L.Mx, L.My, [&](int ii, int jj) {
-      const int q = ii * L.My + jj;
-      const float2 v = fmul4(L.dinv[q], L.b[q]);
-      const float2 c = xc[(ii / AX) * Myc + jj / AY];
-      return make_float2(omega * v.x + corr * c.x, omega * v.y + corr * c.y);
-    });
+    const float2 xk = make_float2(omega * v.x + corr * c.x, omega * v.y + corr * c.y);
+    xT[ti + 1][tj + 1] = xk;
+    if (hc.ha >= 0) xT[hc.ha][hc.hb] = make_float2(omega * vh.x + corr * ch.x, omega * vh.y + corr * ch.y);
     __syncthreads();
     if (inside) {
-      const float2 xk = xT[ti + 1][tj + 1];
       const float2 y = coarse_apply_tile(a, xT, ti, tj);
       const float2 d = fmul4(dk, make_float2(bk.x - y.x, bk.y - y.y));
-      L.x[k] = make_float2(xk.x + omega * d.x, xk.y + omega * d.y);
+      L.x[q] = make_float2(xk.x + omega * d.x, xk.y + omega * d.y);
     }
   }
 }
@@ -678,7 +724,9 @@ inline int small_window_cells(const MGLevel *lev, int first, int nlev, int parts
 
 __global__ void __cluster_dims__(SMALL_CLUSTER, 1, 1) __launch_bounds__(CTA_THREADS)
     k_mg_small_cycle(SmallLevels S, float omega, float corr, const KState *st) {
+  pdl_wait();
   if (st && st->done) return;
+  pdl_release();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = cluster.block_rank() * CTA_THREADS + threadIdx.x, nthr = SMALL_CLUSTER * CTA_THREADS;
   // the small levels' operators are evicted from L2 by the fine-level passes between
@@ -872,7 +920,9 @@ __device__ __forceinline__ float2 small_apply(const float4 *__restrict__ A0, int
 
 __global__ void __cluster_dims__(SMALL_CLUSTER, 1, 1) __launch_bounds__(CTA_THREADS)
     k_mg_small_dsmem(SmallDs S, float omega, float corr, KState *st) {
+  pdl_wait();
   if (st && st->done) return;
+  pdl_release();
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(128) unsigned char sm[];
   __shared__ SmallPlan P;
@@ -1246,7 +1296,9 @@ __global__ void __cluster_dims__(WIDE ? SMALL_CLUSTER : 1, 1, 1) __launch_bounds
     }
   }
   if (WIDE) cluster_wait();
+  pdl_wait();
   if (st && st->done) return;   // the same answer in every CTA
+  pdl_release();
   float2 bk[SR_ITEMS], v[SR_ITEMS];
   if (WIDE && !lead) {
     // ---- the first small level, down: x0 = omega D^-1 b on the window, R (b - A x0) to the lead ----
@@ -1662,7 +1714,7 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     const MGLevel &C = H.lev[0];
     const TileM tm = tiles_of(g.Mx, g.My);
     const int nb = blocks_for(Lc, tm.tiles);
-#define MG0R(AX, AY) [&] { k_mg0_restrict<AX, AY, BA><<<nb, NTm, 0, Lc.stream>>>(F, b, omega, C.Mx, C.My, tm, C.b, st); }
+#define MG0R(AX, AY) [&] { launch_pdl(Lc, k_mg0_restrict<AX, AY, BA>, nb, NTm, 0, F, b, omega, C.Mx, C.My, tm, C.b, st); }
     dispatch_ax(H.fine_ax, H.fine_ay, MG0R(2, 2), MG0R(2, 1), MG0R(1, 2), MG0R(1, 1));
 #undef MG0R
     ++launches;
@@ -1676,7 +1728,7 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     const LevelView V = view(L);
     const TileM tm = tiles_of(L.Mx, L.My);
     const int nb = blocks_for(Lc, tm.tiles);
-#define MGCR(AX, AY) [&] { k_mgc_restrict<AX, AY><<<nb, NTm, 0, Lc.stream>>>(V, omega, C.Mx, C.My, tm, C.b, st); }
+#define MGCR(AX, AY) [&] { launch_pdl(Lc, k_mgc_restrict<AX, AY>, nb, NTm, 0, V, omega, C.Mx, C.My, tm, C.b, st); }
     dispatch_ax(L.ax, L.ay, MGCR(2, 2), MGCR(2, 1), MGCR(1, 2), MGCR(1, 1));
 #undef MGCR
     ++launches;
@@ -1689,7 +1741,7 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     S.first = H.small_first;
     S.invT = H.cinv;
     S.n = 2 * H.lev[H.nlev - 1].N;
-    k_mg_small_dsmem<<<SMALL_CLUSTER, CTA_THREADS, H.small_plan.smem, Lc.stream>>>(S, omega, corr, st);
+    launch_pdl(Lc, k_mg_small_dsmem, SMALL_CLUSTER, CTA_THREADS, H.small_plan.smem, S, omega, corr, st);
     ++launches;
   } else if (H.resident && H.small_kernel != 2) {
     // every level set that fits (all but grids with long thin small levels)
@@ -1699,9 +1751,9 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     S.invT = H.cinv;
     S.n = 2 * H.lev[H.nlev - 1].N;
     if (H.res_plan.wide)
-      k_mg_small_resident<true><<<SMALL_CLUSTER, SR_THREADS, H.res_plan.smem, Lc.stream>>>(S, omega, corr, st);
+      launch_pdl(Lc, k_mg_small_resident<true>, SMALL_CLUSTER, SR_THREADS, H.res_plan.smem, S, omega, corr, st);
     else
-      k_mg_small_resident<false><<<1, SR_THREADS, H.res_plan.smem, Lc.stream>>>(S, omega, corr, st);
+      launch_pdl(Lc, k_mg_small_resident<false>, 1, SR_THREADS, H.res_plan.smem, S, omega, corr, st);
     ++launches;
   } else {
     SmallLevels S;
@@ -1710,7 +1762,7 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     S.lev = reinterpret_cast<const LevelView *>(H.views);
     S.invT = H.cinv;
     S.n = 2 * H.lev[H.nlev - 1].N;
-    k_mg_small_cycle<<<SMALL_CLUSTER, CTA_THREADS, H.small_smem, Lc.stream>>>(S, omega, corr, st);
+    launch_pdl(Lc, k_mg_small_cycle, SMALL_CLUSTER, CTA_THREADS, H.small_smem, S, omega, corr, st);
     ++launches;
   }
   // up through the large coarse levels
@@ -1719,7 +1771,7 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     const LevelView V = view(L);
     const TileM tm = tiles_of(L.Mx, L.My);
     const int nb = H.post_blocks > 0 ? std::min(blocks_for(Lc, tm.tiles), H.post_blocks) : blocks_for(Lc, tm.tiles);
-#define MGCP(AX, AY) [&] { k_mgc_post<AX, AY><<<nb, NTm, 0, Lc.stream>>>(V, omega, corr, C.My, C.x, tm, st); }
+#define MGCP(AX, AY) [&] { launch_pdl(Lc, k_mgc_post<AX, AY>, nb, NTm, 0, V, omega, corr, C.My, C.x, tm, st); }
     dispatch_ax(L.ax, L.ay, MGCP(2, 2), MGCP(2, 1), MGCP(1, 2), MGCP(1, 1));
 #undef MGCP
     ++launches;
@@ -1730,12 +1782,12 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
     const TileM tm = tiles_of(g.Mx, g.My);
     const int nb = blocks_for(Lc, tm.tiles);
     if constexpr (std::is_same<EPI, NoEpi>::value) {
-#define MG0P(AX, AY) [&] { k_mg0_post<AX, AY, BA, ZV><<<nb, NTm, 0, Lc.stream>>>(F, b, omega, corr, C.My, C.x, tm, z, st); }
+#define MG0P(AX, AY) [&] { launch_pdl(Lc, k_mg0_post<AX, AY, BA, ZV>, nb, NTm, 0, F, b, omega, corr, C.My, C.x, tm, z, st); }
       dispatch_ax(H.fine_ax, H.fine_ay, MG0P(2, 2), MG0P(2, 1), MG0P(1, 2), MG0P(1, 1));
 #undef MG0P
     } else {
       static_assert(std::is_same<ZV, float2>::value, "the fused pass produces FP32 iterates");
-#define MG0PA(AX, AY) [&] { k_mg0_post_apply<AX, AY, BA, EPI><<<nb, NTm, 0, Lc.stream>>>(F, b, omega, corr, C.My, C.x, tm, z, epi); }
+#define MG0PA(AX, AY) [&] { launch_pdl(Lc, k_mg0_post_apply<AX, AY, BA, EPI>, nb, NTm, 0, F, b, omega, corr, C.My, C.x, tm, z, epi); }
       dispatch_ax(H.fine_ax, H.fine_ay, MG0PA(2, 2), MG0PA(2, 1), MG0PA(1, 2), MG0PA(1, 1));
 #undef MG0PA
     }

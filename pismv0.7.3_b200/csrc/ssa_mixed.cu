@@ -11,6 +11,7 @@
 // reads 32 B per cell (x 8, nu*H 8, beta 4, flags 4, y 8) instead of 60.
 #include "ssa_fine32.cuh"
 #include "ssa_krylov32.cuh"
+#include "ssa_pdl.cuh"
 #include "ssa_tma_tile.cuh"
 
 namespace pism_gpu {
@@ -102,10 +103,15 @@ __global__ void __launch_bounds__(NT32) k32_init(int N, const float2 *__restrict
   }
 }
 
-__global__ void __launch_bounds__(NT32) k32_p(int N, const float2 *__restrict__ r, const float2 *__restrict__ v,
-                                              float2 *__restrict__ p, const KState *st) {
+// p = r + beta (p - omega v)
+__global__ void __launch_bounds__(NT32) k32_p(int N, const float2 *r_, const float2 *v_, float2 *p_, const KState *st_) {
+  pdl_wait();
+  const KState *st = after_wait(st_);
   if (st->done) return;
+  pdl_release();
   const float bta = (float)st->beta, om = (float)st->omega;
+  const float2 *__restrict__ r = after_wait(r_), *__restrict__ v = after_wait(v_);
+  float2 *__restrict__ p = after_wait(p_);
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const float2 rk = r[k], pk = p[k], vk = v[k];
     p[k] = make_float2(rk.x + bta * (pk.x - om * vk.x), rk.y + bta * (pk.y - om * vk.y));
@@ -185,7 +191,9 @@ __device__ __forceinline__ bool tile_loop_staged(const FineF &F, const Tile32 &t
 // STAGED: interior tiles through the bulk-copy stages, else every tile by plain loads
 template <class EPI, bool STAGED>
 __global__ void __launch_bounds__(NT32) k32_apply(FineF F, Tile32 tm, const float2 *__restrict__ x, EPI e) {
+  pdl_wait();   // not launched early: its operands are restrict pointers
   if (e.st->done) return;
+  pdl_release();
   e.begin();
   auto body = [&](int k, const float2 &y) { e.body(k, y); };
   if constexpr (STAGED) {
@@ -204,14 +212,24 @@ __global__ void __launch_bounds__(NT32) k32_apply(FineF F, Tile32 tm, const floa
   e.finish();
 }
 
-// d += alpha phat + omega shat; r = s - omega t with s = r - alpha v formed here
-__global__ void __launch_bounds__(NT32) k32_x(int N, const float2 *__restrict__ phat, const float2 *__restrict__ shat,
-                                              const float2 *__restrict__ v, const float2 *__restrict__ tv,
-                                              const float2 *__restrict__ rhat, float2 *__restrict__ d,
-                                              float2 *__restrict__ r, double *partials, unsigned *ticket,
-                                              KState *st) {
-  if (st->done) return;
+// d += alpha phat + omega shat; r = s - omega t with s = r - alpha v formed here; the
+// convergence test, and the WHILE condition of a graph-resident loop (cond, 0: none)
+__global__ void __launch_bounds__(NT32) k32_x(int N, const float2 *phat_, const float2 *shat_, const float2 *v_,
+                                              const float2 *tv_, const float2 *rhat_, float2 *d_, float2 *r_,
+                                              double *partials, unsigned *ticket, KState *st_,
+                                              cudaGraphConditionalHandle cond) {
+  pdl_wait();
+  KState *st = after_wait(st_);
+  if (st->done) {
+    if (cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
+    return;
+  }
+  pdl_release();
   const float al = (float)st->alpha, om = (float)st->omega;
+  const float2 *__restrict__ phat = after_wait(phat_), *__restrict__ shat = after_wait(shat_);
+  const float2 *__restrict__ v = after_wait(v_), *__restrict__ tv = after_wait(tv_);
+  const float2 *__restrict__ rhat = after_wait(rhat_);
+  float2 *__restrict__ d = after_wait(d_), *__restrict__ r = after_wait(r_);
   double acc[2] = {0.0, 0.0};
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const float2 rk0 = r[k], vk = v[k];
@@ -232,18 +250,22 @@ __global__ void __launch_bounds__(NT32) k32_x(int N, const float2 *__restrict__ 
     st->rnorm2 = tot[1];
     st->iter += 1;
     const double rn = sqrt(tot[1]), tol = st->rtol * sqrt(st->bnorm2);
+    int done = 1;
     if (!isfinite(rn)) {
-      st->done = 1; st->status = KSP_NAN;
+      st->status = KSP_NAN;
     } else if (rn <= tol) {
-      st->done = 1; st->status = 0;
+      st->status = 0;
     } else if (st->iter >= st->maxit) {
-      st->done = 1; st->status = KSP_MAXIT;
+      st->status = KSP_MAXIT;
     } else if (om == 0.0f || rho_new == 0.0) {
-      st->done = 1; st->status = KSP_BREAKDOWN;
+      st->status = KSP_BREAKDOWN;
     } else {
+      done = 0;
       st->beta = (rho_new / st->rho) * ((double)al / (double)om);
       st->rho = rho_new;
     }
+    st->done = done;
+    if (cond) cudaGraphSetConditional(cond, done ? 0u : 1u);
   }
 }
 
@@ -266,14 +288,14 @@ void launch_mixed_init_dev(const Launch &L, int N, const Krylov32 &K, const doub
 }
 
 void launch_mixed_iteration(const Launch &L, const GridDev &g, const Fields &f, const MGHierarchy &H,
-                            const Krylov32 &K) {
+                            const Krylov32 &K, cudaGraphConditionalHandle cond) {
   const int N = g.Mx * g.My;
   const FineF F = fine_view(g, f, H);
   const Tile32 tm = tiles32(g);
   const int bv = blocks_n(L, N), bt = std::min(tm.tiles, L.max_blocks);
   const EpiV ev{K.rhat, K.v, L.partials, L.ticket, K.st, {0.0}};
   const EpiT et{K.r, K.v, K.t, L.partials, L.ticket, K.st, {0.0, 0.0}, 0.0f};
-  k32_p<<<bv, NT32, 0, L.stream>>>(N, K.r, K.v, K.p, K.st);
+  launch_pdl(L, k32_p, bv, NT32, 0, N, K.r, K.v, K.p, K.st);
   if (H.apply_kernel == 2) {   // the V-cycles' fine-level passes apply A to their results
     mg_vcycle_apply(L, g, f, H, K.p, K.phat, ev);
     mg_vcycle_s_apply(L, g, f, H, K.r, K.v, K.shat, et);   // s = r - alpha v is not stored
@@ -287,7 +309,7 @@ void launch_mixed_iteration(const Launch &L, const GridDev &g, const Fields &f, 
     else k32_apply<EpiT, false><<<bt, NT32, 0, L.stream>>>(F, tm, K.shat, et);
     L.tick(2);
   }
-  k32_x<<<bv, NT32, 0, L.stream>>>(N, K.phat, K.shat, K.v, K.t, K.rhat, K.d, K.r, L.partials, L.ticket, K.st);
+  launch_pdl(L, k32_x, bv, NT32, 0, N, K.phat, K.shat, K.v, K.t, K.rhat, K.d, K.r, L.partials, L.ticket, K.st, cond);
   L.tick(2);
 }
 
