@@ -29,32 +29,27 @@ struct FineF {
   GridDev g;
   float rdx2, rdy2, r2, r4, scaling, nu_bedrock;
   const uint32_t *flags;
-  const float2 *nuH;    // FP32 nu*H
-  const float *beta;    // FP32 beta
+  const float2 *nuH;    // FP32 nu*H and beta, for the apply kernels of their own
+  const float *beta;
+  const float4 *op;     // a cell's nu*H (east, north), beta and flag word in 16 bytes
   const float4 *dinv;   // FP32 inverse diagonal blocks
   const double *H;      // thickness, read only where F_NB_* flags are set
 };
 
 
-// rows / apply of a fine cell from staged tiles
-// the two FP32 rows of fine cell (i, j) from a staged tile of FP32 nu*H; false for a
-// diagonal-only row
-__device__ __forceinline__ bool fine_rows_tile(const FineF &F, int i, int j, uint32_t f, float bta,
-                                               const HaloTile<float2> &nT, int ti, int tj, Row2T<float> &e1,
-                                               Row2T<float> &e2) {
-  if (f & F_DIAG_ONLY) return false;
-  const GridDev &g = F.g;
-  float c_w = nT[ti][tj + 1].x, c_e = nT[ti + 1][tj + 1].x, c_s = nT[ti + 1][tj].y, c_n = nT[ti + 1][tj + 1].y;
-  if (f & F_NB_ANY) {   // nu_bedrock_set overrides, SSAFD.cc:561-585
-    const int k = cell(g, i, j);
-    const double Hc = F.H[k], HE = F.H[nbr(g, i, j, 1, 0)];
-    if (f & F_NB_W) c_w = (float)(F.nu_bedrock * 0.5 * (Hc + F.H[nbr(g, i, j, -1, 0)]));
-    if (f & F_NB_E) c_e = (float)(F.nu_bedrock * 0.5 * (Hc + HE));
-    if (f & F_NB_N) c_n = (float)(F.nu_bedrock * 0.5 * (Hc + F.H[nbr(g, i, j, 0, 1)]));
-    if (f & F_NB_S) c_s = (float)(F.nu_bedrock * 0.5 * (Hc + HE));
-  }
-  stencil_rows_t<float>(F.rdx2, F.rdy2, F.r2, F.r4, f, c_w, c_e, c_s, c_n, bta, e1, e2);
-  return true;
+// y = A x of a row whose weights are not all 1 (next to a calving front): the 36 coefficients
+// formed.  Out of line: few cells take it, and the kernels share one copy of it and its rounding.
+static __device__ __noinline__ float2 fine_apply_weighted(float rdx2, float rdy2, float r2, float r4, uint32_t f,
+                                                          float c_w, float c_e, float c_s, float c_n, float bta,
+                                                          float2 xNW, float2 xN, float2 xNE, float2 xW, float2 xC,
+                                                          float2 xE, float2 xSW, float2 xS, float2 xSE) {
+  Row2T<float> e1, e2;
+  stencil_rows_t<float>(rdx2, rdy2, r2, r4, f, c_w, c_e, c_s, c_n, bta, e1, e2);
+  auto xr = [&](int di, int dj) {
+    return di < 0 ? (dj > 0 ? xNW : dj < 0 ? xSW : xW) : di > 0 ? (dj > 0 ? xNE : dj < 0 ? xSE : xE)
+                                                               : (dj > 0 ? xN : dj < 0 ? xS : xC);
+  };
+  return apply_rows_rel<float, float2>(e1, e2, xr);
 }
 
 // y = A x at fine cell (i, j) from its flag word f, beta, the four staggered nu*H
@@ -77,9 +72,8 @@ __device__ __forceinline__ float2 fine_apply_coef(const FineF &F, int i, int j, 
     if (f & F_NB_N) c_n = (float)(F.nu_bedrock * 0.5 * (Hc + F.H[nbr(g, i, j, 0, 1)]));
     if (f & F_NB_S) c_s = (float)(F.nu_bedrock * 0.5 * (Hc + HE));
   }
-  Row2T<float> e1, e2;
-  stencil_rows_t<float>(F.rdx2, F.rdy2, F.r2, F.r4, f, c_w, c_e, c_s, c_n, bta, e1, e2);
-  return apply_rows_rel<float, float2>(e1, e2, xr);
+  return fine_apply_weighted(F.rdx2, F.rdy2, F.r2, F.r4, f, c_w, c_e, c_s, c_n, bta, xr(-1, 1), xr(0, 1), xr(1, 1),
+                             xr(-1, 0), xr(0, 0), xr(1, 0), xr(-1, -1), xr(0, -1), xr(1, -1));
 }
 
 // y = A x at fine cell (i, j) = tile position (ti, tj), x and nu*H from tiles

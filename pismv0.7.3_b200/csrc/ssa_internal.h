@@ -100,7 +100,8 @@ struct MGHierarchy {
   int post_blocks = 0;                           // grid cap of the coarse post-smoothing (0: none)
   double *cinv = nullptr;                        // dense inverse of the coarsest operator (transposed)
   int *singular = nullptr;
-  float2 *nuHf = nullptr;                        // FP32 copies of the fine nu*H, beta, D^-1
+  float4 *opf = nullptr;                         // FP32 nu*H (east, north), beta and the flag word
+  float2 *nuHf = nullptr;                        // FP32 nu*H and beta apart (mixed_apply_kernel 0, 1)
   float *betaf = nullptr;
   float4 *dinvf = nullptr;
   void *views = nullptr;                         // device copy of the level views

@@ -1,12 +1,13 @@
 // ssa_krylov32.cuh — what the FP32 BiCGStab does with each operator apply y = A x: the two
 // epilogues of the inner iteration, shared by the apply kernels of ssa_mixed.cu and by the
-// multigrid fine-level pass fused with them (ssa_mg.cu), so both routes give the same bits.
+// multigrid fine-level pass fused with them (ssa_march.cuh).
 //
 //   EpiV:  v = A phat, alpha = rho / (rhat, v)
 //   EpiT:  t = A shat, omega = (t, s) / (t, t), s = r - alpha v formed where it is read
 //
-// Each thread accumulates its cells' terms in FP64 in tile order; finish() adds the grid's
-// partial sums in block order (ssa_reduce.cuh) and writes the scalar to the Krylov state.
+// Each thread accumulates its cells' terms in FP64 in its own order; finish() adds the grid's
+// partial sums in block order (ssa_reduce.cuh) and writes the scalar to the Krylov state.  The
+// iteration reads the scalars as FP32, which rounds the order of the FP64 sums away.
 #pragma once
 
 #include "ssa_reduce.cuh"
@@ -30,9 +31,10 @@ struct EpiV {
     v[k] = y;
     acc[0] += dotf(rhat[k], y);
   }
+  template <int THREADS = RED_THREADS>
   __device__ __forceinline__ void finish() {
     double tot[1];
-    if (grid_reduce<1>(acc, partials, ticket, tot)) {
+    if (grid_reduce<1, THREADS>(acc, partials, ticket, tot)) {
       if (tot[0] == 0.0 || !isfinite(tot[0])) {
         st->done = 1;
         st->status = isfinite(tot[0]) ? KSP_BREAKDOWN : KSP_NAN;
@@ -62,9 +64,10 @@ struct EpiT {
     acc[0] += dotf(y, make_float2(rk.x - al * vk.x, rk.y - al * vk.y));
     acc[1] += dotf(y, y);
   }
+  template <int THREADS = RED_THREADS>
   __device__ __forceinline__ void finish() {
     double tot[2];
-    if (grid_reduce<2>(acc, partials, ticket, tot)) st->omega = (tot[1] != 0.0) ? tot[0] / tot[1] : 0.0;
+    if (grid_reduce<2, THREADS>(acc, partials, ticket, tot)) st->omega = (tot[1] != 0.0) ? tot[0] / tot[1] : 0.0;
   }
 };
 

@@ -36,6 +36,7 @@
 
 #include "ssa_fine32.cuh"
 #include "ssa_krylov32.cuh"
+#include "ssa_march.cuh"
 #include "ssa_pdl.cuh"
 #include "ssa_small_plan.h"
 
@@ -106,15 +107,21 @@ __device__ __forceinline__ float2 coarse_apply(const LevelView &L, int i, int j,
   return make_float2(y1, y2);
 }
 
-// FP32 copies of nu*H, beta and D^-1 for the fine-level passes (once per Picard iteration)
+// FP32 copies of nu*H, beta and D^-1 for the fine-level passes (once per Picard iteration), nu*H,
+// beta and the flag word packed into 16 bytes a cell; nu*H and beta also apart where nuHf is given
 __global__ void k_mg0_compact(int N, const double2 *__restrict__ nuH, const double *__restrict__ beta,
-                              const double4 *__restrict__ dinv, float2 *__restrict__ nuHf, float *__restrict__ betaf,
+                              const double4 *__restrict__ dinv, const uint32_t *__restrict__ flags,
+                              float4 *__restrict__ opf, float2 *__restrict__ nuHf, float *__restrict__ betaf,
                               float4 *__restrict__ dinvf) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 n = nuH[k];
     const double4 d = dinv[k];
-    nuHf[k] = make_float2((float)n.x, (float)n.y);
-    betaf[k] = (float)beta[k];
+    const float nx = (float)n.x, ny = (float)n.y, bta = (float)beta[k];
+    opf[k] = make_float4(nx, ny, bta, __uint_as_float(flags[k]));
+    if (nuHf) {
+      nuHf[k] = make_float2(nx, ny);
+      betaf[k] = bta;
+    }
     dinvf[k] = make_float4((float)d.x, (float)d.y, (float)d.z, (float)d.w);
   }
 }
@@ -438,143 +445,6 @@ __device__ __forceinline__ void store_aggregates(float2 (&rsh)[TILE_I][TILE_J], 
     const int I = i0 / AX + ci, J = j0 / AY + cj;
     if (I < Mxc && J < Myc) bc[I * Myc + J] = make_float2(ru, rv);
   }
-}
-
-// fine level: b_1 = R (b - A x0), x0 = omega D^-1 b
-template <int AX, int AY, class BA>
-__global__ void __launch_bounds__(NTm) k_mg0_restrict(FineF F, BA b_in, float omega, int Mxc,
-                                                      int Myc, TileM tm, float2 *__restrict__ bc, const KState *st) {
-  pdl_wait();
-  if (st && st->done) return;
-  pdl_release();
-  const auto b = b_in.bind();
-  __shared__ HaloTile<float2> xT, nT;
-  __shared__ float2 rsh[TILE_I][TILE_J];
-  const GridDev &g = F.g;
-  const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
-  for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
-    const int i0 = (t / tm.tiles_j) * TILE_I, j0 = (t % tm.tiles_j) * TILE_J;
-    const int i = i0 + ti, j = j0 + tj;
-    const bool inside = i < g.Mx && j < g.My;
-    const int k = inside ? i * g.My + j : 0;
-    const uint32_t f = F.flags[k];   // issued with the tile loads: one round trip per tile
-    const float bta = F.beta[k];
-    const float2 bk = b(k);
-    __syncthreads();
-    load_halo_tile<float2>(xT, i0, j0, g.Mx, g.My, [&](int ii, int jj) {
-      const int q = ii * g.My + jj;
-      const float2 v = fmul4(F.dinv[q], b(q));
-      return make_float2(omega * v.x, omega * v.y);
-    });
-    load_halo_tile<float2>(nT, i0, j0, g.Mx, g.My, [&](int ii, int jj) { return F.nuH[ii * g.My + jj]; });
-    __syncthreads();
-    float2 r = make_float2(0.0f, 0.0f);
-    if (inside) {
-      const float2 y = fine_apply_tile(F, i, j, f, bta, xT, nT, ti, tj);
-      r = make_float2(bk.x - y.x, bk.y - y.y);
-    }
-    rsh[ti][tj] = r;
-    __syncthreads();
-    store_aggregates<AX, AY>(rsh, i0, j0, Mxc, Myc, bc);
-  }
-}
-
-// fine level: x = omega D^-1 b + s P x_1;  z = x + omega D^-1 (b - A x)
-template <int AX, int AY, class BA, class ZV>
-__global__ void __launch_bounds__(NTm) k_mg0_post(FineF F, BA b_in, float omega, float corr,
-                                                  int Myc, const float2 *xc_, TileM tm,
-                                                  ZV *__restrict__ z, const KState *st) {
-  pdl_wait();
-  if (st && st->done) return;
-  pdl_release();
-  const float2 *__restrict__ xc = after_wait(xc_);
-  const auto b = b_in.bind();
-  __shared__ HaloTile<float2> xT, nT;
-  const GridDev &g = F.g;
-  const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
-  for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
-    const int i0 = (t / tm.tiles_j) * TILE_I, j0 = (t % tm.tiles_j) * TILE_J;
-    const int i = i0 + ti, j = j0 + tj;
-    const bool inside = i < g.Mx && j < g.My;
-    const int k = inside ? i * g.My + j : 0;
-    const uint32_t f = F.flags[k];   // issued with the tile loads: one round trip per tile
-    const float bta = F.beta[k];
-    const float2 bk = b(k);
-    const float4 dk = F.dinv[k];
-    __syncthreads();
-    load_halo_tile<float2>(xT, i0, j0, g.Mx, g.My, [&](int ii, int jj) {
-      const int q = ii * g.My + jj;
-      const float2 v = fmul4(F.dinv[q], b(q));
-      const float2 c = xc[(ii / AX) * Myc + jj / AY];
-      return make_float2(omega * v.x + corr * c.x, omega * v.y + corr * c.y);
-    });
-    load_halo_tile<float2>(nT, i0, j0, g.Mx, g.My, [&](int ii, int jj) { return F.nuH[ii * g.My + jj]; });
-    __syncthreads();
-    if (inside) {
-      const float2 xk = xT[ti + 1][tj + 1];
-      const float2 y = fine_apply_tile(F, i, j, f, bta, xT, nT, ti, tj);
-      const float2 d = fmul4(dk, make_float2(bk.x - y.x, bk.y - y.y));
-      z[k] = from_f2<ZV>(make_float2(xk.x + omega * d.x, xk.y + omega * d.y));
-    }
-  }
-}
-
-// The fine-level pass fused with the FP32 operator apply that follows the V-cycle in
-// BiCGStab.  Per tile: x = omega D^-1 b + corr P x_1 on the tile and a two-cell halo;
-// z = x + omega D^-1 (b - A x) on the tile and a one-cell halo (the halo's z recomputed here
-// rather than read back from the tiles that own it); z stored on the tile; y = A z on the
-// tile handed to the epilogue.  Every value comes from the same arithmetic as k_mg0_post
-// followed by the apply kernel, over the same tiles in the same order per block, so the
-// results and the epilogue's sums are the same bits.
-constexpr int H2I = TIm + 4, H2J = TJm + 4;   // the two-cell-halo region of a tile
-
-template <int AX, int AY, class BA, class EPI>
-__global__ void __launch_bounds__(NTm) k_mg0_post_apply(FineF F, BA b_in, float omega, float corr, int Myc,
-                                                        const float2 *xc_, TileM tm,
-                                                        float2 *__restrict__ z, EPI e) {
-  pdl_wait();
-  if (e.st->done) return;
-  pdl_release();
-  const float2 *__restrict__ xc = after_wait(xc_);
-  e.begin();
-  const auto b = b_in.bind();
-  __shared__ float2 xs[H2I][H2J], ns[H2I][H2J], zs[TIm + 2][TJm + 2];
-  const int Mx = F.g.Mx, My = F.g.My;
-  const int ti = threadIdx.x >> 5, tj = threadIdx.x & 31;
-  for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
-    const int i0 = (t / tm.tiles_j) * TIm, j0 = (t % tm.tiles_j) * TJm;
-    __syncthreads();   // the previous tile's readers are done
-    for (int q = threadIdx.x; q < H2I * H2J; q += NTm) {   // cell (i0 - 2 + a, j0 - 2 + c), wrapped
-      const int a = q / H2J, c = q - a * H2J;
-      const int ii = pmod(i0 - 2 + a, Mx), jj = pmod(j0 - 2 + c, My), kq = ii * My + jj;
-      const float2 v = fmul4(F.dinv[kq], b(kq));
-      const float2 cc = xc[(ii / AX) * Myc + jj / AY];
-      xs[a][c] = make_float2(omega * v.x + corr * cc.x, omega * v.y + corr * cc.y);
-      ns[a][c] = F.nuH[kq];
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < (TIm + 2) * (TJm + 2); q += NTm) {   // cell (i0 - 1 + a, j0 - 1 + c)
-      const int a = q / (TJm + 2), c = q - a * (TJm + 2);
-      const int ii = pmod(i0 - 1 + a, Mx), jj = pmod(j0 - 1 + c, My), kq = ii * My + jj;
-      auto xr = [&](int di, int dj) { return xs[a + 1 + di][c + 1 + dj]; };
-      const float2 y = fine_apply_coef(F, ii, jj, F.flags[kq], F.beta[kq], ns[a][c + 1].x, ns[a + 1][c + 1].x,
-                                       ns[a + 1][c].y, ns[a + 1][c + 1].y, xr);
-      const float2 xk = xs[a + 1][c + 1], bk = b(kq);
-      const float2 d = fmul4(F.dinv[kq], make_float2(bk.x - y.x, bk.y - y.y));
-      zs[a][c] = make_float2(xk.x + omega * d.x, xk.y + omega * d.y);
-    }
-    __syncthreads();
-    const int i = i0 + ti, j = j0 + tj;
-    if (i < Mx && j < My) {
-      const int k = i * My + j;
-      z[k] = zs[ti + 1][tj + 1];
-      auto zr = [&](int di, int dj) { return zs[ti + 1 + di][tj + 1 + dj]; };
-      const float2 y = fine_apply_coef(F, i, j, F.flags[k], F.beta[k], ns[ti + 1][tj + 2].x, ns[ti + 2][tj + 2].x,
-                                       ns[ti + 2][tj + 1].y, ns[ti + 2][tj + 2].y, zr);
-      e.body(k, y);
-    }
-  }
-  e.finish();
 }
 
 // The halo element of a tile that thread (ti, tj) loads beside its own cell (load_halo_tile's
@@ -1173,6 +1043,12 @@ struct SmallResident {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+// 16 bytes from global to this CTA's shared memory, not waited for until copies_done()
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // y = A x from the nine blocks a(b) and the nine neighbour values x(b), in block order
 template <class AB, class XB>
 __device__ __forceinline__ float2 apply_blocks(const AB &a, const XB &x) {
@@ -1274,11 +1150,11 @@ __global__ void __cluster_dims__(WIDE ? SMALL_CLUSTER : 1, 1, 1) __launch_bounds
         const int k = ok ? i * F.My + j : 0;
 #pragma unroll
         for (int b = 0; b < 9; ++b) {
-          A[b * items + tid] = F.A[b * F.N + k];
+          copy16(&A[b * items + tid], &F.A[b * F.N + k]);
           const int ni = wrap(i + (b % 3) - 1, F.Mx), nj = wrap(j + 1 - b / 3, F.My);
           nb[b * items + tid] = ok ? (uint16_t)(ni * F.My + nj) : (uint16_t)0xffffu;
         }
-        A[9 * items + tid] = F.dinv[k];
+        copy16(&A[9 * items + tid], &F.dinv[k]);
       }
     }
     // row r = warp (+ 16) of the coarsest inverse, one column a lane
@@ -1292,11 +1168,12 @@ __global__ void __cluster_dims__(WIDE ? SMALL_CLUSTER : 1, 1, 1) __launch_bounds
       int k = w0 * My + q;
       if (k < 0) k += L.N;
       else if (k >= L.N) k -= L.N;
-      dw[q] = L.dinv[k];
+      copy16(&dw[q], &L.dinv[k]);
     }
   }
   if (WIDE) cluster_wait();
   pdl_wait();
+  copies_done();   // a thread reads back only what it copied itself
   if (st && st->done) return;   // the same answer in every CTA
   pdl_release();
   float2 bk[SR_ITEMS], v[SR_ITEMS];
@@ -1574,6 +1451,7 @@ int mg_allocate(MGHierarchy &H, int fine_cells) {
     if (cudaMalloc(&L.b, sizeof(float2) * L.N) != cudaSuccess) return 1;
     if (cudaMalloc(&L.x, sizeof(float2) * L.N) != cudaSuccess) return 1;
   }
+  if (cudaMalloc(&H.opf, sizeof(float4) * fine_cells) != cudaSuccess) return 1;
   if (cudaMalloc(&H.nuHf, sizeof(float2) * fine_cells) != cudaSuccess) return 1;
   if (cudaMalloc(&H.betaf, sizeof(float) * fine_cells) != cudaSuccess) return 1;
   if (cudaMalloc(&H.dinvf, sizeof(float4) * fine_cells) != cudaSuccess) return 1;
@@ -1613,6 +1491,7 @@ void mg_free(MGHierarchy &H) {
     L.dinv = nullptr;
     L.b = L.x = nullptr;
   }
+  cudaFree(H.opf);
   cudaFree(H.nuHf);
   cudaFree(H.betaf);
   cudaFree(H.dinvf);
@@ -1622,6 +1501,7 @@ void mg_free(MGHierarchy &H) {
   cudaFree(H.small_plan_dev);
   H.small_plan_dev = nullptr;
   H.views = nullptr;
+  H.opf = nullptr;
   H.nuHf = nullptr;
   H.betaf = nullptr;
   H.dinvf = nullptr;
@@ -1646,6 +1526,7 @@ FineF fine_view(const GridDev &g, const Fields &f, const MGHierarchy &H) {
   F.flags = f.flags;
   F.nuH = H.nuHf;
   F.beta = H.betaf;
+  F.op = H.opf;
   F.dinv = H.dinvf;
   F.H = f.H;
   return F;
@@ -1660,8 +1541,9 @@ void mg_setup(const Launch &Lc, const GridDev &g, const Fields &f, const double4
 // operator's): always from the current nu*H
 void mg_setup_fine(const Launch &Lc, const GridDev &g, const Fields &f, const double4 *dinv0, MGHierarchy &H) {
   const int N = g.Mx * g.My;
-  k_mg0_compact<<<std::min((N + NTm - 1) / NTm, Lc.max_blocks), NTm, 0, Lc.stream>>>(N, f.nuH, f.beta, dinv0, H.nuHf,
-                                                                                     H.betaf, H.dinvf);
+  const bool apart = H.apply_kernel != 2;
+  k_mg0_compact<<<std::min((N + NTm - 1) / NTm, Lc.max_blocks), NTm, 0, Lc.stream>>>(
+      N, f.nuH, f.beta, dinv0, f.flags, H.opf, apart ? H.nuHf : nullptr, H.betaf, H.dinvf);
   Lc.tick();
 }
 
@@ -1708,13 +1590,13 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
                    KState *st, const EPI &epi = EPI{}) {
   const FineF F = fine_view(g, f, H);
   const float omega = H.omega, corr = H.correction;
+  const int sms = Lc.max_blocks / 4;
   int launches = 0;
   // down: fine -> level 1
   {
     const MGLevel &C = H.lev[0];
-    const TileM tm = tiles_of(g.Mx, g.My);
-    const int nb = blocks_for(Lc, tm.tiles);
-#define MG0R(AX, AY) [&] { launch_pdl(Lc, k_mg0_restrict<AX, AY, BA>, nb, NTm, 0, F, b, omega, C.Mx, C.My, tm, C.b, st); }
+    const MarchPlan m = march_plan(g.Mx, g.My, 1, 2, H.fine_ax, sms, 8, 1);
+#define MG0R(AX, AY) [&] { launch_pdl(Lc, k_mg0_restrict<AX, AY, BA>, m.blocks, MARCH_THREADS, 0, F, b, omega, C.My, m, C.b, st); }
     dispatch_ax(H.fine_ax, H.fine_ay, MG0R(2, 2), MG0R(2, 1), MG0R(1, 2), MG0R(1, 1));
 #undef MG0R
     ++launches;
@@ -1779,15 +1661,15 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
   // fine level
   {
     const MGLevel &C = H.lev[0];
-    const TileM tm = tiles_of(g.Mx, g.My);
-    const int nb = blocks_for(Lc, tm.tiles);
     if constexpr (std::is_same<EPI, NoEpi>::value) {
-#define MG0P(AX, AY) [&] { launch_pdl(Lc, k_mg0_post<AX, AY, BA, ZV>, nb, NTm, 0, F, b, omega, corr, C.My, C.x, tm, z, st); }
+      const MarchPlan m = march_plan(g.Mx, g.My, 1, 2, 1, sms, 10, 1);
+#define MG0P(AX, AY) [&] { launch_pdl(Lc, k_mg0_post<AX, AY, BA, ZV>, m.blocks, MARCH_THREADS, 0, F, b, omega, corr, C.My, C.x, m, z, st); }
       dispatch_ax(H.fine_ax, H.fine_ay, MG0P(2, 2), MG0P(2, 1), MG0P(1, 2), MG0P(1, 1));
 #undef MG0P
     } else {
       static_assert(std::is_same<ZV, float2>::value, "the fused pass produces FP32 iterates");
-#define MG0PA(AX, AY) [&] { launch_pdl(Lc, k_mg0_post_apply<AX, AY, BA, EPI>, nb, NTm, 0, F, b, omega, corr, C.My, C.x, tm, z, epi); }
+      const MarchPlan m = march_plan(g.Mx, g.My, 2, 4, 1, sms, 16, 1);
+#define MG0PA(AX, AY) [&] { launch_pdl(Lc, k_mg0_post_apply<AX, AY, BA, EPI>, m.blocks, MARCH_THREADS, 0, F, b, omega, corr, C.My, C.x, m, z, epi); }
       dispatch_ax(H.fine_ax, H.fine_ay, MG0PA(2, 2), MG0PA(2, 1), MG0PA(1, 2), MG0PA(1, 1));
 #undef MG0PA
     }

@@ -7,7 +7,7 @@
 
 namespace pism_gpu {
 
-constexpr int RED_THREADS = 256;   // every reducing kernel runs 256-thread blocks
+constexpr int RED_THREADS = 256;   // the block size of a reducing kernel unless it says otherwise
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -17,10 +17,10 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // Reduce NV values over the grid.  Returns true in thread 0 of the last block,
 // with the grid totals in tot[].
-template <int NV>
+template <int NV, int THREADS = RED_THREADS>
 __device__ __forceinline__ bool grid_reduce(double (&val)[NV], double *partials, unsigned *ticket,
                                             double (&tot)[NV]) {
-  __shared__ double sh[NV][RED_THREADS / 32];
+  __shared__ double sh[NV][THREADS / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -33,7 +33,7 @@ __device__ __forceinline__ bool grid_reduce(double (&val)[NV], double *partials,
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       double s = 0.0;
-      for (int w = 0; w < RED_THREADS / 32; ++w) s += sh[v][w];
+      for (int w = 0; w < THREADS / 32; ++w) s += sh[v][w];
       partials[blockIdx.x * NV + v] = s;
     }
     __threadfence();
@@ -47,7 +47,7 @@ __device__ __forceinline__ bool grid_reduce(double (&val)[NV], double *partials,
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     double s = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += RED_THREADS) s += __ldcg(&partials[b * NV + v]);
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += THREADS) s += __ldcg(&partials[b * NV + v]);
     s = warp_sum(s);
     if (lane == 0) sh[v][warp] = s;
   }
@@ -56,7 +56,7 @@ __device__ __forceinline__ bool grid_reduce(double (&val)[NV], double *partials,
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     double s = 0.0;
-    for (int w = 0; w < RED_THREADS / 32; ++w) s += sh[v][w];
+    for (int w = 0; w < THREADS / 32; ++w) s += sh[v][w];
     tot[v] = s;
   }
   *ticket = 0u;
