@@ -1557,10 +1557,16 @@ int pism_gpu_ssafem_solve(pism_gpu_ssa *h, const pism_gpu_ssafem_options *o, pis
       rc = fail(h, PISM_GPU_SSA_EZERODIAG, "SSAFEM: singular diagonal block at node %d", zp - 1);
       break;
     }
-    // conjugate gradients in batches of FEM_CG_BATCH iterations, each skipped on the device once
-    // done; the batch is captured into a CUDA graph on first use (its buffers never move) and
-    // replayed, with direct launches if the capture fails
-    if (!S.cg_batch && !S.cg_batch_failed && h->cfg.graphs >= 1) {
+    // conjugate gradients: the whole solve in one kernel where the grid fits the device, else in
+    // batches of FEM_CG_BATCH iterations, each skipped on the device once done; the batch is
+    // captured into a CUDA graph on first use (its buffers never move) and replayed, with
+    // direct launches if the capture fails
+    const bool resident = launch_fem_cg_resident(L, P, S);
+    if (resident) {
+      CK(h, cudaGetLastError());
+      RET(copy_out(h, &cg, S.cg, sizeof(cg), PISM_MEM_HOST));
+    }
+    if (!resident && !S.cg_batch && !S.cg_batch_failed && h->cfg.graphs >= 1) {
       cudaGraph_t graph = nullptr;
       const long long before = h->stats.kernel_launches;
       bool ok = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
@@ -1577,7 +1583,7 @@ int pism_gpu_ssafem_solve(pism_gpu_ssa *h, const pism_gpu_ssafem_options *o, pis
       }
       h->stats.kernel_launches = before;   // nothing ran during the capture
     }
-    for (;;) {
+    while (!resident) {
       if (S.cg_batch) {
         CK(h, cudaGraphLaunch(S.cg_batch, h->stream));
         L.tick(3 * FEM_CG_BATCH);
@@ -1591,7 +1597,10 @@ int pism_gpu_ssafem_solve(pism_gpu_ssa *h, const pism_gpu_ssafem_options *o, pis
     st.ksp_iterations += cg.its;
     if (cg.done != 1) {
       rc = fail(h, PISM_GPU_SSA_EKSP, "SSAFEM: the linear solve %s after %d iterations",
-                cg.done == 2 ? "broke down (J not positive definite)" : "reached ksp_max_it", cg.its);
+                cg.done == 2   ? "broke down (J not positive definite)"
+                : cg.done == 4 ? "gave up waiting for its blocks"
+                               : "reached ksp_max_it",
+                cg.its);
       break;
     }
     // backtracking line search on ||F||

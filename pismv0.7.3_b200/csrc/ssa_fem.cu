@@ -15,6 +15,7 @@
 // structure-of-arrays ([36][N]), which the CG apply reads coalesced.
 #include <algorithm>
 
+#include "ssa_exchange.cuh"
 #include "ssa_fem.h"
 #include "ssa_reduce.cuh"
 
@@ -362,6 +363,174 @@ __global__ void __launch_bounds__(NTF) k_cg_direction(int N, const double2 *z, d
   }
 }
 
+// The whole CG solve in one cooperative kernel, one thread a node: the node's 36 Jacobian
+// coefficients and the p its block reads in shared memory, its x, r and z in registers.  An
+// iteration costs two exchanges (ssa_exchange.cuh): (p, q), then (r, z) and (r, r); then the z
+// around the block are read from words of their own, and the block updates its copies of the
+// neighbours' p as their owners do.
+//
+// A block owns NTF nodes in a row of the linear order, from s0 on.  The p its stencils read lie in
+// three runs of NTF + 2 nodes, from s0 - My - 1, s0 - 1 and s0 + My - 1 (modulo N: the grid's rows
+// wrap), but for a neighbour of a node at a row's end, or two of the last node's, which that
+// thread keeps by itself.
+//
+// Bound: the two exchanges' and the halo's trips through L2; the Jacobian's 288 B a node come from
+// shared memory.  One B200, three kernels an iteration / this kernel: 5 x 481 nodes 12.5 / 4.5 us
+// an iteration, 241 x 241 15.3 / 7.4 us.  The same operations per node and the same order of the
+// sums as those kernels, which remain for the grids that do not fit (more than two blocks an SM,
+// 75 776 nodes on 148).
+constexpr int CG_RUN = NTF + 2;
+constexpr int CG_SMEM = 36 * NTF * (int)sizeof(double) + 3 * CG_RUN * (int)sizeof(double2);
+
+__global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double *__restrict__ J,
+                                                        const double4 *__restrict__ dinv,
+                                                        const double2 *__restrict__ r0, const double2 *__restrict__ z0,
+                                                        double2 *__restrict__ x_out, ExNodes zex, FemCG *cg,
+                                                        ExSlots slots_q, ExSlots slots_r) {
+  extern __shared__ __align__(16) double Js[];   // [36][NTF], then the three runs of p
+  double2 *const P = reinterpret_cast<double2 *>(Js + 36 * NTF);
+  const int N = G.Mx * G.My, tid = threadIdx.x, s0 = blockIdx.x * NTF, n = s0 + tid;
+  const bool mine = n < N;
+  const int i = mine ? n / G.My : 0, j = mine ? n - i * G.My : 0;
+  auto modN = [&](int k) { return (k % N + N) % N; };
+  const int base[3] = {s0 - G.My - 1, s0 - 1, s0 + G.My - 1};
+  // each neighbour's place in the runs; -1, -2: the node apart[0], apart[1], kept by this thread
+  short at[9];
+  int apart[2] = {-1, -1};
+  bool lone = false;
+#pragma unroll
+  for (int b = 0; b < 9; ++b) {
+    const int m = mine ? fem_node(G, i + b / 3 - 1, j + b % 3 - 1) : 0;
+    int place = -1;
+#pragma unroll
+    for (int q = 2; q >= 0; --q) {
+      const int k = modN(m - base[q]);
+      // the middle run is the block's own nodes and one on either side
+      if (k < CG_RUN && (q != 1 || k == 0 || k == CG_RUN - 1 || s0 + k - 1 < N)) place = q * CG_RUN + k;
+    }
+    if (mine && place < 0) {
+      if (apart[0] < 0 || apart[0] == m) {
+        apart[0] = m;
+      } else {
+        lone = lone || (apart[1] >= 0 && apart[1] != m);
+        apart[1] = m;
+        place = -2;
+      }
+    }
+    at[b] = (short)place;
+  }
+  // what this thread reads into the runs: above and below its node; six threads a run's end each
+  const int above = modN(base[0] + tid), below = modN(base[2] + tid), e = tid - (NTF - 6);
+  const int end_run = e >> 1, end_k = e < 0 ? -1 : (end_run == 1 ? (e & 1) * (NTF + 1) : NTF + (e & 1));
+  const int end = e < 0 ? -1 : modN(base[end_run] + end_k), end_at = end_run * CG_RUN + end_k;
+  const bool more = __any_sync(0xffffffffu, apart[0] >= 0 || end >= 0);
+  double2 x = make_double2(0.0, 0.0), r = x, z = x;   // p starts as z
+  double2 pa = apart[0] >= 0 ? z0[apart[0]] : x, pa2 = apart[1] >= 0 ? z0[apart[1]] : x;
+  double4 d = make_double4(0.0, 0.0, 0.0, 0.0);
+  P[tid] = z0[above];
+  P[2 * CG_RUN + tid] = z0[below];
+  if (end >= 0) P[end_at] = z0[end];
+  if (mine) {
+    P[CG_RUN + 1 + tid] = z0[n];
+    r = r0[n];
+    d = dinv[n];
+#pragma unroll 12
+    for (int q = 0; q < 36; ++q) Js[q * NTF + tid] = J[(size_t)q * N + n];
+  }
+  double rz = cg->rz, pq = 0.0, alpha = 0.0, beta = 0.0, rr = cg->rr;
+  const double tol = cg->rtol * cg->rtol * cg->bb;
+  const int maxit = cg->maxit;
+  int its = 0, done = cg->done;
+  // a node with three neighbours outside the runs (no grid has one): the solve gives up at once
+  if (__syncthreads_or(lone)) done = 4;
+  while (!done) {
+    const unsigned round = (unsigned)its + 1u;
+    double2 y = make_double2(0.0, 0.0), pn = y;
+    double acc[1] = {0.0};
+    if (mine) {
+      pn = P[CG_RUN + 1 + tid];
+#pragma unroll
+      for (int b = 0; b < 9; ++b) {
+        const double2 pb = b == 4 ? pn : (at[b] >= 0 ? P[at[b]] : at[b] == -1 ? pa : pa2);
+        y.x += Js[(b * 4 + 0) * NTF + tid] * pb.x + Js[(b * 4 + 1) * NTF + tid] * pb.y;
+        y.y += Js[(b * 4 + 2) * NTF + tid] * pb.x + Js[(b * 4 + 3) * NTF + tid] * pb.y;
+      }
+      acc[0] += pn.x * y.x + pn.y * y.y;
+    }
+    double tq[1];
+    if (!exchange_sum<1>(acc, slots_q, round, tq)) {
+      done = 4;
+      break;
+    }
+    pq = tq[0];
+    if (!(pq > 0.0)) {   // J not positive definite along p
+      done = 2;
+      break;
+    }
+    alpha = rz / pq;
+    double acc2[2] = {0.0, 0.0};
+    if (mine) {
+      x.x += alpha * pn.x;
+      x.y += alpha * pn.y;
+      r.x -= alpha * y.x;
+      r.y -= alpha * y.y;
+      z = bmul(d, r);
+      asm volatile("" : "+d"(z.x), "+d"(z.y));   // rounded here, as the other blocks' copies are
+      // every owner has posted its (p, q) of this round, so none still reads the last round's z
+      zex.put(n, z, round);
+      acc2[0] += r.x * z.x + r.y * z.y;
+      acc2[1] += r.x * r.x + r.y * r.y;
+    }
+    double tr[2];
+    if (!exchange_sum<2>(acc2, slots_r, round, tr)) {
+      done = 4;
+      break;
+    }
+    beta = tr[0] / rz;
+    rz = tr[0];
+    rr = tr[1];
+    its += 1;
+    if (rr <= tol) done = 1;
+    else if (its >= maxit) done = 3;
+    if (done) break;
+    // read after the sums, when the words are there: reads before them, repeated by every thread
+    // until the owners have written, hold the sums up
+    auto direction = [&](const double2 &zn, const double2 &p) {
+      return make_double2(zn.x + beta * p.x, zn.y + beta * p.y);
+    };
+    bool ok;
+    if (more) {   // warps that also read rows' ends or runs' ends
+      const int nodes[5] = {above, below, apart[0] >= 0 ? apart[0] : above, apart[1] >= 0 ? apart[1] : above,
+                            end >= 0 ? end : above};
+      double2 v[5];
+      ok = zex.get<5>(nodes, round, v);
+      P[tid] = direction(v[0], P[tid]);
+      P[2 * CG_RUN + tid] = direction(v[1], P[2 * CG_RUN + tid]);
+      pa = direction(v[2], pa);
+      pa2 = direction(v[3], pa2);
+      if (end >= 0) P[end_at] = direction(v[4], P[end_at]);
+    } else {
+      const int nodes[2] = {above, below};
+      double2 v[2];
+      ok = zex.get<2>(nodes, round, v);
+      P[tid] = direction(v[0], P[tid]);
+      P[2 * CG_RUN + tid] = direction(v[1], P[2 * CG_RUN + tid]);
+    }
+    if (mine) P[CG_RUN + 1 + tid] = direction(z, pn);
+    if (__syncthreads_or(!ok)) done = 4;   // its next sum is never posted: the other blocks give up too
+  }
+  if (mine) x_out[n] = x;
+  if (blockIdx.x == 0 && tid == 0) {
+    cg->rz = rz;
+    cg->pq = pq;
+    cg->rr = rr;
+    cg->alpha = alpha;
+    cg->beta = beta;
+    cg->its = its;
+    cg->done = done;
+  }
+}
+
 // trial = vel + lambda du, with ||lambda du||^2 and ||trial||^2
 __global__ void __launch_bounds__(NTF) k_fem_trial(int N, const double2 *vel, const double2 *du, double lambda,
                                                    double2 *trial, FemScalars *sc, double *partials,
@@ -445,7 +614,7 @@ int fem_allocate(FemState &S, int Mx, int My, int periodicity) {
 
 void fem_free(FemState &S) {
   void *ptrs[] = {S.C.H, S.C.tauc, S.C.tdu, S.C.tdv, S.C.B, S.C.mask, S.J, S.dinv, S.F, S.Ft,
-                  S.du, S.trial, S.vel0, S.r, S.z, S.p, S.q, S.cg, S.sc, S.zero_pivot};
+                  S.du, S.trial, S.vel0, S.r, S.z, S.p, S.q, S.cg, S.sc, S.zero_pivot, S.ex};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (S.cg_batch) cudaGraphExecDestroy(S.cg_batch);
@@ -489,6 +658,36 @@ void launch_fem_cg_iterations(const Launch &L, const FemProblem &P, const FemSta
     k_cg_update<<<b, NTF, 0, L.stream>>>(S.N, S.dinv, S.p, S.q, S.du, S.r, S.z, S.cg, L.partials, L.ticket);
     k_cg_direction<<<b, NTF, 0, L.stream>>>(S.N, S.z, S.p, S.cg);
   }
+}
+
+bool launch_fem_cg_resident(const Launch &L, const FemProblem &P, FemState &S) {
+  const int nb = (S.N + NTF - 1) / NTF;
+  if (!S.cg_resident_blocks) {   // once per grid: what the device holds at once
+    cudaFuncSetAttribute((const void *)k_cg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM);
+    S.cg_resident_blocks = std::max(1, resident_blocks((const void *)k_cg_resident, NTF, CG_SMEM));
+  }
+  // one thread a node: the order of the sums is that of the kernels below L.max_blocks blocks
+  if (nb > S.cg_resident_blocks || nb > L.max_blocks) return false;
+  const size_t ws = ex_slot_words(nb), words = 2 * ws + ex_node_words(S.N);   // the slots, then z by node
+  if (!S.ex && alloc(&S.ex, words) != 0) {
+    cudaGetLastError();
+    return false;
+  }
+  if (cudaMemsetAsync(S.ex, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
+  FemGrid G = fem_grid(P);
+  ExSlots sq{S.ex}, sr{S.ex + ws};
+  ExNodes zex{S.ex + 2 * ws, S.N};
+  const double *J = S.J;
+  const double4 *dinv = S.dinv;
+  const double2 *r = S.r, *z = S.z;
+  void *args[] = {&G, &J, &dinv, &r, &z, &S.du, &zex, &S.cg, &sq, &sr};
+  if (cudaLaunchCooperativeKernel((const void *)k_cg_resident, dim3(nb), dim3(NTF), args, CG_SMEM, L.stream) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  L.tick();
+  return true;
 }
 
 void launch_fem_trial(const Launch &L, const FemState &S, const double2 *vel, double lambda) {

@@ -25,7 +25,7 @@ struct FemCoef {
 // the state of the conjugate-gradient solve of one Newton step
 struct FemCG {
   double rz, pq, rr, bb, alpha, beta, rtol;
-  int its, maxit, done;   // done: 1 converged, 2 breakdown (p.Ap <= 0), 3 iteration limit
+  int its, maxit, done;   // done: 1 converged, 2 breakdown (p.Ap <= 0), 3 iteration limit, 4 a wait gave up
 };
 
 // the scalars of a Newton step: ||F||^2, then ||lambda du||^2 and ||u + lambda du||^2
@@ -46,6 +46,8 @@ struct FemState {
   int *zero_pivot = nullptr;
   cudaGraphExec_t cg_batch = nullptr;  // FEM_CG_BATCH CG iterations captured once (all buffers fixed)
   bool cg_batch_failed = false;
+  unsigned long long *ex = nullptr;    // the resident solve's exchange words
+  int cg_resident_blocks = 0;          // blocks of it that the device holds at once
 };
 constexpr int FEM_CG_BATCH = 16;
 
@@ -68,6 +70,8 @@ void launch_fem_residual(const Launch &L, const FemProblem &P, const FemState &S
 // CG on J du = -F: init, then `n` iterations (each skipped once cg->done)
 void launch_fem_cg_init(const Launch &L, const FemProblem &P, const FemState &S, double rtol, int maxit);
 void launch_fem_cg_iterations(const Launch &L, const FemProblem &P, const FemState &S, int n);
+// the same solve in one cooperative kernel where the grid fits; false: nothing was launched
+bool launch_fem_cg_resident(const Launch &L, const FemProblem &P, FemState &S);
 // trial = vel + lambda du with ||lambda du||^2 and ||trial||^2 into sc
 void launch_fem_trial(const Launch &L, const FemState &S, const double2 *vel, double lambda);
 
