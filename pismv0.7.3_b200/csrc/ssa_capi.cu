@@ -77,6 +77,7 @@ struct pism_gpu_ssa {
   PState *pstate_host = nullptr;
   double *res_dev = nullptr;   // {||r||^2, ||b||^2} of the refinement
   double *res_host = nullptr;
+  KrylovExchange kex;
   MGHierarchy mg{};
   double *partials = nullptr;
   unsigned *ticket = nullptr;
@@ -704,6 +705,12 @@ int linear_solve(pism_gpu_ssa *h, double2 *x, double rtol, int *its_out, int *st
   const MGHierarchy *mg = active_mg(h);
   const LinePC *line = active_line(h);
   const int kind = mg ? GRAPH_BICG_MG : line ? GRAPH_BICG_LINE : GRAPH_BICG_JACOBI;
+  // block Jacobi on a grid that fits the device at once: the loop is one kernel
+  if (kind == GRAPH_BICG_JACOBI && h->cfg.graphs >= 2 && launch_bicg_resident(h->L, g, f, h->K, x, h->kex)) {
+    CK(h, cudaGetLastError());
+    CK(h, cudaMemcpyAsync(h->st_host, h->K.st, sizeof(KState), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaStreamSynchronize(h->stream));
+  } else
   // long FP64 solves: four iterations per pass of the loop body
   RET(run_until_done(h, kind, x, h->K.st, std::max(8, (int)(0.8 * h->last_ksp_its)), 4,
                      [&](cudaGraphConditionalHandle cond) { launch_bicg_iteration(h->L, g, f, h->K, x, mg, line, cond); }));
@@ -1139,7 +1146,7 @@ int pism_gpu_ssa_destroy(pism_gpu_ssa *h) {
                  h->K32.shat, h->K32.d, h->K32.st, h->res_dev, h->lfeat, h->lout, h->G.V, h->G.Z,
                  h->G.partials, h->G.gs, h->G.st, h->line.P, h->line.F, h->line.G, h->lpc.img, h->lpc.out,
                  h->lpc.r, h->lpc.d, h->lpc.ad, h->lpc.part, h->lpc.rho, h->lpc.gamma, h->sb3d, h->mc,
-                 h->ec, h->ec_mask};
+                 h->ec, h->ec_mask, h->kex.w};
   for (void *p : dev)
     if (p) cudaFree(p);
   fem_free(h->fem);

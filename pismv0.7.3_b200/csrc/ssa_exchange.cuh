@@ -105,11 +105,11 @@ struct ExNodes {
 };
 inline size_t ex_node_words(int nodes) { return 4 * (size_t)nodes; }
 
-// Sum NV values over the grid; every thread gets the totals.  False (in every thread of the block)
-// when a wait gave up; the other blocks then give up too.
+// Sum NV values over the first nb blocks of the grid; every thread of the grid gets the totals.
+// False (in every thread of the block) when a wait gave up; the other blocks then give up too.
 template <int NV>
 __device__ __forceinline__ bool exchange_sum(double (&val)[NV], const ExSlots &slots, unsigned round,
-                                             double (&tot)[NV]) {
+                                             double (&tot)[NV], int nb = gridDim.x) {
   static_assert(2 * NV <= EX_WORDS, "a slot holds two values");
   constexpr int WARPS = RED_THREADS / 32;
   __shared__ double part[NV][WARPS], total[NV];
@@ -121,12 +121,11 @@ __device__ __forceinline__ bool exchange_sum(double (&val)[NV], const ExSlots &s
   }
   __syncthreads();
   bool ok = true;
-  if (threadIdx.x < NV) {
+  if (threadIdx.x < NV && (int)blockIdx.x < nb) {
     double s = 0.0;
     for (int q = 0; q < WARPS; ++q) s += part[threadIdx.x][q];
     ex_put(slots.block(blockIdx.x) + 2 * threadIdx.x, s, round);
   }
-  const int nb = gridDim.x;
   // the sum of slots 32 g + lane (and those RED_THREADS further), as warp g of ssa_reduce.cuh adds it
   auto gather = [&](int g, double (&acc)[NV]) {
 #pragma unroll

@@ -133,6 +133,14 @@ void launch_bicg_init(const Launch &L, const GridDev &g, const Fields &f, const 
 // (cond: the WHILE condition of a graph-resident loop, set by the iteration's last kernel; 0: none)
 void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
                            const MGHierarchy *mg, const LinePC *line, cudaGraphConditionalHandle cond = 0);
+// the whole block-Jacobi solve after launch_bicg_init in one cooperative kernel where the grid
+// fits; false: nothing was launched
+struct KrylovExchange {
+  unsigned long long *w = nullptr;   // the exchange words, allocated on first use
+  int capacity = 0;                  // blocks of the kernel that the device holds at once
+};
+bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+                          KrylovExchange &E);
 // FGMRES: r0 = b - A x into V0 (init) / after a restart; one Arnoldi step j; the end of a cycle
 void launch_gmres_residual(const Launch &L, const GridDev &g, const Fields &f, const Gmres &G, const double2 *b,
                            const double2 *x, int init);

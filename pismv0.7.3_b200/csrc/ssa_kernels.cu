@@ -9,8 +9,10 @@
 // writes its partial sums, and the last block to finish (atomic ticket) adds them
 // in block order — deterministic — and updates the solver scalars on the device,
 // so no kernel boundary or host round trip is spent on a dot product.
+#include <algorithm>
 #include <cstdio>
 
+#include "ssa_exchange.cuh"
 #include "ssa_internal.h"
 #include "ssa_pdl.cuh"
 #include "ssa_stencil.cuh"
@@ -720,6 +722,214 @@ __global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *phat_, cons
   }
 }
 
+// ---------------------------------------------------------------------------
+// The whole block-Jacobi BiCGStab solve in one cooperative kernel, one block a tile, one thread a
+// cell: the cell's vectors in registers, nu*H in shared memory, and beside it each thread keeps one
+// cell of the tile's halo, whose r, p and v it updates as their owner does from the owner's v
+// and t (ssa_exchange.cuh).  Three sums and two halo reads an iteration.  The terms of the last
+// sum go through memory once more, because k_bicg_x adds them in linear cell order and the other
+// two kernels in tile order: the same operations and the same sums as those five kernels, bit
+// for bit.
+//
+// Bound: the exchanges' trips through L2 (about 1 us each).  Test I on 5 x 201 (1486 iterations in
+// 22 Picard steps), one B200: 27.2 ms with the five kernels, 10.2 ms with this one.  Grids of
+// more tiles than SMs (37 888 cells at most) keep the five kernels.
+// ---------------------------------------------------------------------------
+struct BicgResident {
+  ExSlots a, b, c;      // the slots of (rhat, v); (t, s), (t, t); (rhat, r), (r, r)
+  ExNodes v, t, terms;  // v and t of the tiles' border cells; the last sum's terms by cell
+};
+
+__global__ void __launch_bounds__(NT, 1) k_bicg_resident(GridDev g, TileMap tm, StencilConst sc,
+                                                         const uint32_t *__restrict__ flags,
+                                                         const double2 *__restrict__ nuH,
+                                                         const double *__restrict__ beta_,
+                                                         const double4 *__restrict__ dinv,
+                                                         const double2 *__restrict__ r0, double2 *x_, BicgResident ex,
+                                                         KState *st) {
+  __shared__ HaloTile<double2> xT, nT;
+  const int N = g.Mx * g.My, tid = threadIdx.x, ti = tid >> 5, tj = tid & 31;
+  const int i0 = (blockIdx.x / tm.tiles_j) * TI, j0 = (blockIdx.x % tm.tiles_j) * TJ, i = i0 + ti, j = j0 + tj;
+  const bool inside = i < g.Mx && j < g.My;
+  // a thread outside the grid keeps the wrapped cell, as the tile's halo does
+  const int k = pmod(i, g.Mx) * g.My + pmod(j, g.My);
+  int ha = -1, hb = 0;   // the halo cell this thread keeps (load_halo_tile's assignment)
+  if (ti < 2) {
+    ha = ti == 0 ? 0 : TI + 1;
+    hb = tj;
+  } else if (ti < 4 && tj < 2) {
+    ha = ti == 2 ? 0 : TI + 1;
+    hb = TJ + tj;
+  } else if (ti < 6 && tj < TI) {
+    ha = tj + 1;
+    hb = ti == 4 ? 0 : TJ + 1;
+  }
+  const int h = ha >= 0 ? pmod(i0 - 1 + ha, g.Mx) * g.My + pmod(j0 - 1 + hb, g.My) : k;
+  const bool border = inside && (ti == 0 || ti == TI - 1 || tj == 0 || tj == TJ - 1 || i == 0 || j == 0 ||
+                                 i == g.Mx - 1 || j == g.My - 1);
+  // whether an inside cell's stencil reads the copies: cells one past the grid's edge at most (they
+  // wrap to border cells; what lies further is never posted)
+  const bool need_k = !inside && i <= g.Mx && j <= g.My;
+  const bool need_h = ha >= 0 && i0 - 1 + ha <= g.Mx && j0 - 1 + hb <= g.My;
+  nT[ti + 1][tj + 1] = nuH[k];
+  if (ha >= 0) nT[ha][hb] = nuH[h];
+  const uint32_t f = flags[k];
+  const double bta = beta_[k];
+  const double4 dk = dinv[k], dh = dinv[h];
+  double2 r = r0[k], p = make_double2(0.0, 0.0), v = p, s = p, t = p, ph = p, sh = p;
+  double2 rh = r0[h], pH = p, vH = p, sH = p, tH = p;   // the kept halo cell's
+  const double2 rhat = r;
+  double2 x = inside ? x_[k] : p;
+  double rho = st->rho, alpha = st->alpha, omega = st->omega, beta = st->beta, rnorm2 = st->rnorm2;
+  const double tol = st->rtol * sqrt(st->bnorm2);
+  const int maxit = st->maxit, nlin = (N + NT - 1) / NT;
+  int its = st->iter, done = st->done, status = st->status;
+  // the owners' values of the cells this thread keeps: past the edge (own), in the halo (halo)
+  auto copies = [&](const ExNodes &e, unsigned round, double2 &own, double2 &halo) {
+    bool ok = true;
+    double2 w[1];
+    if (need_k) {
+      const int q[1] = {k};
+      ok = e.get<1>(q, round, w);
+      own = w[0];
+    }
+    if (need_h) {
+      const int q[1] = {h};
+      ok = e.get<1>(q, round, w) && ok;
+      halo = w[0];
+    }
+    return ok;
+  };
+  auto keep = [](double2 &q) { asm volatile("" : "+d"(q.x), "+d"(q.y)); };   // rounded here
+  for (unsigned round = 1; !done; ++round) {
+    // p = r + beta (p - omega v);  phat = D^-1 p
+    auto dir = [&](const double2 &rk, const double2 &pk, const double2 &vk) {
+      return make_double2(rk.x + beta * (pk.x - omega * vk.x), rk.y + beta * (pk.y - omega * vk.y));
+    };
+    p = dir(r, p, v);
+    pH = dir(rh, pH, vH);
+    keep(p);
+    keep(pH);
+    ph = dmul(dk, p);
+    keep(ph);
+    xT[ti + 1][tj + 1] = ph;
+    if (ha >= 0) xT[ha][hb] = dmul(dh, pH);
+    __syncthreads();
+    // v = A phat;  alpha = rho / (rhat, v)
+    double acc[1] = {0.0}, tot[1];
+    if (inside) {
+      v = apply_cell_tile(g, sc, i, j, f, xT, nT, bta, ti, tj);
+      keep(v);
+      acc[0] += dot2(rhat, v);
+      if (border) ex.v.put(k, v, round);
+    }
+    if (!exchange_sum<1>(acc, ex.a, round, tot)) {
+      done = 1;
+      status = KSP_STALLED;
+      break;
+    }
+    if (tot[0] == 0.0 || !isfinite(tot[0])) {
+      done = 1;
+      status = isfinite(tot[0]) ? KSP_BREAKDOWN : KSP_NAN;
+      break;
+    }
+    alpha = rho / tot[0];
+    bool ok = copies(ex.v, round, v, vH);
+    // s = r - alpha v;  shat = D^-1 s
+    auto half = [&](const double2 &rk, const double2 &vk) {
+      return make_double2(rk.x - alpha * vk.x, rk.y - alpha * vk.y);
+    };
+    s = half(r, v);
+    sH = half(rh, vH);
+    keep(s);
+    keep(sH);
+    sh = dmul(dk, s);
+    keep(sh);
+    xT[ti + 1][tj + 1] = sh;
+    if (ha >= 0) xT[ha][hb] = dmul(dh, sH);
+    if (__syncthreads_or(!ok)) {
+      done = 1;
+      status = KSP_STALLED;
+      break;
+    }
+    // t = A shat;  omega = (t, s) / (t, t)
+    double acc2[2] = {0.0, 0.0}, tot2[2];
+    if (inside) {
+      t = apply_cell_tile(g, sc, i, j, f, xT, nT, bta, ti, tj);
+      keep(t);
+      acc2[0] += dot2(t, s);
+      acc2[1] += dot2(t, t);
+      if (border) ex.t.put(k, t, round);
+    }
+    if (!exchange_sum<2>(acc2, ex.b, round, tot2)) {
+      done = 1;
+      status = KSP_STALLED;
+      break;
+    }
+    omega = (tot2[1] != 0.0) ? tot2[0] / tot2[1] : 0.0;
+    // x += alpha phat + omega shat;  r = s - omega t
+    auto rest = [&](const double2 &sk, const double2 &tk) {
+      return make_double2(sk.x - omega * tk.x, sk.y - omega * tk.y);
+    };
+    if (inside) {
+      x.x += alpha * ph.x + omega * sh.x;
+      x.y += alpha * ph.y + omega * sh.y;
+      r = rest(s, t);
+      keep(r);
+      double a0 = 0.0, a1 = 0.0;
+      a0 += dot2(rhat, r);
+      a1 += dot2(r, r);
+      ex.terms.put(k, make_double2(a0, a1), round);
+    }
+    ok = copies(ex.t, round, t, tH);
+    if (!inside) {
+      r = rest(s, t);
+      keep(r);
+    }
+    rh = rest(sH, tH);
+    keep(rh);
+    // (rhat, r) and (r, r) in linear cell order: block b adds cells NT b .. NT b + NT - 1
+    acc2[0] = acc2[1] = 0.0;
+    const int kl = blockIdx.x * NT + tid;
+    if (kl < N) {
+      const int q[1] = {kl};
+      double2 w[1];
+      ok = ex.terms.get<1>(q, round, w) && ok;
+      acc2[0] = w[0].x;
+      acc2[1] = w[0].y;
+    }
+    if (__syncthreads_or(!ok) || !exchange_sum<2>(acc2, ex.c, round, tot2, nlin)) {
+      done = 1;
+      status = KSP_STALLED;
+      break;
+    }
+    const double rho_new = tot2[0], rn = sqrt(tot2[1]);
+    rnorm2 = tot2[1];
+    its += 1;
+    done = 1;
+    if (!isfinite(rn)) status = KSP_NAN;
+    else if (rn <= tol) status = 0;
+    else if (its >= maxit) status = KSP_MAXIT;
+    else if (omega == 0.0 || rho_new == 0.0) status = KSP_BREAKDOWN;
+    else {
+      done = 0;
+      beta = (rho_new / rho) * (alpha / omega);
+      rho = rho_new;
+    }
+  }
+  if (inside) x_[k] = x;
+  if (blockIdx.x == 0 && tid == 0) {
+    st->rho = rho;
+    st->alpha = alpha;
+    st->omega = omega;
+    st->beta = beta;
+    st->rnorm2 = rnorm2;
+    st->iter = its;
+    st->status = status;
+    st->done = done;
+  }
+}
+
 // the outer residual of the mixed-precision refinement: r = b - A x in FP64, handed to the
 // inner FP32 solve; the two norms feed the FP64 convergence test
 __global__ void __launch_bounds__(NT, 4) k_residual32(GridDev g, TileMap tm, StencilConst s,
@@ -872,6 +1082,44 @@ void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, c
   else if (line) line_apply(L, g, *line, K.s, K.shat, K.st);
   launch_pdl(L, k_bicg_t, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.shat, K.s, K.t, L.partials, L.ticket, K.st);
   launch_pdl(L, k_bicg_x, bv, NT, 0, N, K.phat, K.shat, K.s, K.t, K.rhat, x, K.r, L.partials, L.ticket, K.st, cond);
+}
+
+bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+                          KrylovExchange &E) {
+  const int N = g.Mx * g.My;
+  TileMap tm = make_tiles(g);
+  if (!E.capacity) E.capacity = std::max(1, resident_blocks((const void *)k_bicg_resident, NT, 0));
+  // one cell a thread in both orders: below L.max_blocks blocks the five kernels add alike
+  if (tm.tiles > E.capacity || tm.tiles > L.max_blocks) return false;
+  const size_t slots = ex_slot_words(tm.tiles), nodes = ex_node_words(N), words = 3 * slots + 3 * nodes;
+  if (!E.w && cudaMalloc((void **)&E.w, sizeof(unsigned long long) * words) != cudaSuccess) {
+    E.w = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  if (cudaMemsetAsync(E.w, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
+  BicgResident ex;
+  ex.a.w = E.w;
+  ex.b.w = E.w + slots;
+  ex.c.w = E.w + 2 * slots;
+  ex.v = ExNodes{E.w + 3 * slots, N};
+  ex.t = ExNodes{E.w + 3 * slots + nodes, N};
+  ex.terms = ExNodes{E.w + 3 * slots + 2 * nodes, N};
+  GridDev gd = g;
+  StencilConst s = stencil_const(g, f);
+  const uint32_t *flags = f.flags;
+  const double2 *nuH = f.nuH, *r = K.r;
+  const double *beta = f.beta;
+  const double4 *dinv = K.dinv;
+  KState *st = K.st;
+  void *args[] = {&gd, &tm, &s, &flags, &nuH, &beta, &dinv, &r, &x, &ex, &st};
+  if (cudaLaunchCooperativeKernel((const void *)k_bicg_resident, dim3(tm.tiles), dim3(NT), args, 0, L.stream) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  L.tick();
+  return true;
 }
 
 void launch_residual32(const Launch &L, const GridDev &g, const Fields &f, const double2 *b, const double2 *x,

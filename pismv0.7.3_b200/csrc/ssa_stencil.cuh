@@ -126,33 +126,27 @@ __device__ __forceinline__ V apply_regular(T rdx2, T rdy2, T r2, T r4, T c_w, T 
   const V xNW = xr(-1, 1), xN = xr(0, 1), xNE = xr(1, 1);
   const V xW = xr(-1, 0), xC = xr(0, 0), xE = xr(1, 0);
   const V xSW = xr(-1, -1), xS = xr(0, -1), xSE = xr(1, -1);
+  // which product of each sum is rounded by itself is written out, so that every kernel that
+  // applies it gives the same bits: p a + q b with q b rounded first
+  auto fma_ = [](T p, T a, T c) {
+    if constexpr (std::is_same<T, float>::value) return __fmaf_rn(p, a, c);
+    else return __fma_rn(p, a, c);
+  };
+  auto two = [&](T p, T a, T q, T b) {
+    if constexpr (std::is_same<T, float>::value) return __fmaf_rn(p, a, __fmul_rn(q, b));
+    else return __fma_rn(p, a, __dmul_rn(q, b));
+  };
+  // d/dy (c du/dy), d/dx (c du/dx) and the mixed terms of the first equation
+  const T uy = two(c_n, xC.x - xN.x, c_s, xC.x - xS.x), ux = two(c_w, xC.x - xW.x, c_e, xC.x - xE.x);
+  const T vA = two(c_w, xNW.y + xN.y - xSW.y - xS.y, c_e, xSE.y + xS.y - xNE.y - xN.y);
+  const T vB = two(c_n, xNW.y - xNE.y + xW.y - xE.y, c_s, xSE.y - xSW.y - xW.y + xE.y);
+  // and of the second equation
+  const T vy = two(c_n, xC.y - xN.y, c_s, xC.y - xS.y), vx = two(c_w, xC.y - xW.y, c_e, xC.y - xE.y);
+  const T uA = two(c_w, xNW.x + xN.x - xSW.x - xS.x, c_e, xSE.x + xS.x - xNE.x - xN.x);
+  const T uB = two(c_n, xNW.x - xNE.x + xW.x - xE.x, c_s, xSE.x - xSW.x - xW.x + xE.x);
   V y;
-  if constexpr (std::is_same<T, float>::value) {
-    // FP32 (the multigrid smoother, the mixed-precision inner solve): which product of each sum
-    // is rounded by itself is written out, so every kernel that applies it gives the same bits
-    auto two = [](float p, float a, float q, float b) { return __fmaf_rn(p, a, __fmul_rn(q, b)); };
-    const float uy = two(c_n, xC.x - xN.x, c_s, xC.x - xS.x), ux = two(c_w, xC.x - xW.x, c_e, xC.x - xE.x);
-    const float vA = two(c_w, xNW.y + xN.y - xSW.y - xS.y, c_e, xSE.y + xS.y - xNE.y - xN.y);
-    const float vB = two(c_n, xNW.y - xNE.y + xW.y - xE.y, c_s, xSE.y - xSW.y - xW.y + xE.y);
-    const float vy = two(c_n, xC.y - xN.y, c_s, xC.y - xS.y), vx = two(c_w, xC.y - xW.y, c_e, xC.y - xE.y);
-    const float uA = two(c_w, xNW.x + xN.x - xSW.x - xS.x, c_e, xSE.x + xS.x - xNE.x - xN.x);
-    const float uB = two(c_n, xNW.x - xNE.x + xW.x - xE.x, c_s, xSE.x - xSW.x - xW.x + xE.x);
-    y.x = __fmaf_rn(bta, xC.x, __fmaf_rn(r4, vB, __fmaf_rn(r2, vA, two(4 * rdx2, ux, rdy2, uy))));
-    y.y = __fmaf_rn(bta, xC.y, __fmaf_rn(r2, uB, __fmaf_rn(r4, uA, two(rdx2, vx, 4 * rdy2, vy))));
-  } else {
-    // d/dy (c du/dy), d/dx (4 c du/dx) and the mixed terms of the first equation
-    const T uy = c_n * (xC.x - xN.x) + c_s * (xC.x - xS.x);
-    const T ux = c_e * (xC.x - xE.x) + c_w * (xC.x - xW.x);
-    const T vA = c_w * (xNW.y + xN.y - xSW.y - xS.y) + c_e * (xSE.y + xS.y - xNE.y - xN.y);
-    const T vB = c_n * (xNW.y - xNE.y + xW.y - xE.y) + c_s * (xSE.y - xSW.y - xW.y + xE.y);
-    // and of the second equation
-    const T vy = c_n * (xC.y - xN.y) + c_s * (xC.y - xS.y);
-    const T vx = c_e * (xC.y - xE.y) + c_w * (xC.y - xW.y);
-    const T uA = c_w * (xNW.x + xN.x - xSW.x - xS.x) + c_e * (xSE.x + xS.x - xNE.x - xN.x);
-    const T uB = c_n * (xNW.x - xNE.x + xW.x - xE.x) + c_s * (xSE.x - xSW.x - xW.x + xE.x);
-    y.x = rdy2 * uy + 4 * rdx2 * ux + r2 * vA + r4 * vB + bta * xC.x;
-    y.y = 4 * rdy2 * vy + rdx2 * vx + r4 * uA + r2 * uB + bta * xC.y;
-  }
+  y.x = fma_(bta, xC.x, fma_(r4, vB, fma_(r2, vA, two(4 * rdx2, ux, rdy2, uy))));
+  y.y = fma_(bta, xC.y, fma_(r2, uB, fma_(r4, uA, two(rdx2, vx, 4 * rdy2, vy))));
   return y;
 }
 
