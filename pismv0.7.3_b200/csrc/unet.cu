@@ -2,12 +2,13 @@
 // BF16 with FP32 accumulation on the tensor cores (mma.sync m16n8k16, operands staged in
 // shared memory and fed by ldmatrix), its backward pass and an Adam step.
 //
-// The convolutions are implicit GEMMs over an 8 x 16 pixel output tile: the CTA stages the
-// 10 x 18 input patch of one 16- or 32-channel slice and the 3 x 3 x 32 weights of its 32
-// output channels, each warp owns one output row (M = 16 pixels) and all 32 channels
-// (4 n-blocks of 8), K runs over taps x channels.  The backward data pass is the same kernel
-// on flipped, transposed weights with the ReLU mask applied while staging; the weight
-// gradient is a GEMM over pixels (one warp per tap) reduced deterministically across CTAs.
+// The convolutions are implicit GEMMs over a tile of 8 or 16 x 16 output pixels and 32 output
+// channels: the patch of one 16- or 32-channel slice and its 3 x 3 weights are copied
+// asynchronously one step ahead, each warp owns one or two output rows (16 pixels a row) and all
+// 32 channels, K runs over taps x channels.  The backward data pass is the same kernel on
+// flipped, transposed weights; every gradient is masked by its layer's ReLU by the kernel that
+// makes it.  The weight gradient is a GEMM over pixels (one warp per tap) reduced
+// deterministically across CTAs, on a second stream beside the data gradients.
 // Every reduction (weight / bias gradients, loss) is written as per-CTA partial sums and
 // summed in a fixed order, so training runs are bit-reproducible.
 #include <cuda_bf16.h>
@@ -28,10 +29,9 @@ using bf16 = __nv_bfloat16;
 
 namespace pism_unet {
 
-constexpr int TH = 8, TW = 16;            // output tile
+constexpr int TH = 8, TW = 16;            // pixel tile of the weight gradient; the convolution's is 8 or 16 x 16
 constexpr int PH = TH + 2, PW = TW + 2;   // input patch with the 3 x 3 halo
-constexpr int NT = 32;                    // output channels per CTA
-constexpr int THREADS = 256;              // 8 warps = 8 tile rows
+constexpr int THREADS = 256;              // 8 warps, one or two tile rows each
 constexpr int WG_THREADS = 288;           // weight gradient: 9 warps = 9 taps
 constexpr int WG_MAX_CTAS = 64;           // pixel-range partial sums per weight gradient
 
@@ -106,164 +106,248 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
   return v;
 }
 
-// Stage the (TH+2) x (TW+2) patch of channels [c0, c0 + CS) around the tile at (i0, j0) of
-// image b; zero outside the image; masked by (mask > 0) when mask is given.
-template <int CS, int NTHR>
-__device__ __forceinline__ void stage_patch(bf16 *patch, const bf16 *__restrict__ x, const bf16 *__restrict__ mask,
-                                            int C, int c0, int b, int i0, int j0, int H, int W) {
+// 16 bytes to shared memory, zeros where `from` is outside the image; not waited for
+__device__ __forceinline__ void copy16(void *to, const void *from, bool inside) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from),
+               "r"(inside ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all groups but the latest N are complete
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Copy the ROWS x (TW+2) patch of channels [c0, c0 + CS) around the tile at (i0, j0) of image b;
+// zero outside the image.
+template <int CS, int NTHR, int ROWS>
+__device__ __forceinline__ void copy_patch(bf16 *patch, const bf16 *__restrict__ x, int C, int c0, int b, int i0, int j0,
+                                           int H, int W) {
   constexpr int CP = CS + 8, CH = CS / 8;
-  for (int q = threadIdx.x; q < PH * PW * CH; q += NTHR) {
+  for (int q = threadIdx.x; q < ROWS * PW * CH; q += NTHR) {
     const int pix = q / CH, ch = q - pix * CH;
     const int pi = pix / PW, pj = pix - pi * PW;
     const int ii = i0 - 1 + pi, jj = j0 - 1 + pj;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (ii >= 0 && ii < H && jj >= 0 && jj < W) {
-      const size_t off = (((size_t)b * H + ii) * W + jj) * C + c0 + ch * 8;
-      v = *reinterpret_cast<const uint4 *>(x + off);
-      if (mask) v = relu_mask8(v, *reinterpret_cast<const uint4 *>(mask + off));
-    }
-    *reinterpret_cast<uint4 *>(patch + pix * CP + ch * 8) = v;
+    const bool inside = ii >= 0 && ii < H && jj >= 0 && jj < W;
+    copy16(patch + pix * CP + ch * 8, inside ? x + (((size_t)b * H + ii) * W + jj) * C + c0 + ch * 8 : x, inside);
   }
 }
 
 // ---- 3x3 convolution (forward, and backward data on flipped weights) ----
-// y[b, i, j, co] = act(bias[co] + sum_{tap, ci} w[tap, co, ci] * xm[b, i + ky - 1, j + kx - 1, ci])
-// xm = x * (mask > 0) when mask is given.  grid = (B * tiles, Cout / 32).
-template <int CS>
-__global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x, const bf16 *__restrict__ xmask,
-                                                     int Cin, const bf16 *__restrict__ w,
-                                                     const float *__restrict__ bias, int relu, bf16 *__restrict__ y,
-                                                     int Cout, int H, int W) {
-  constexpr int CP = CS + 8, CH = CS / 8;
-  __shared__ __align__(16) bf16 patch[PH * PW * CP];
-  __shared__ __align__(16) bf16 wsm[9 * NT * CP];
-  const int tiles_w = (W + TW - 1) / TW, tiles_h = (H + TH - 1) / TH;
-  int t = blockIdx.x;
-  const int b = t / (tiles_h * tiles_w);
-  t -= b * tiles_h * tiles_w;
-  const int i0 = (t / tiles_w) * TH, j0 = (t % tiles_w) * TW;
-  const int co0 = blockIdx.y * NT;
+// y[b, i, j, co] = act(bias[co] + sum_{tap, ci} w[tap, co, ci] * x[b, i + ky - 1, j + kx - 1, ci]),
+// zero where omask[b, i, j, co] <= 0 (backward data: the ReLU of the layer that made the input).
+//
+// A CTA walks pixel tiles of 8 MR x 16 pixels for NB output channels; each warp has MR rows (16
+// pixels a row) by all NB channels.  A step is one channel slice of a tile: its patch (and its
+// weights, unless the layer has one slice: then they stay) is copied asynchronously while the
+// step before multiplies.
+//
+// Bound: the legacy tensor pipe and the loads that feed it.  Unpipelined, at 8 x 16 pixels by 32
+// channels, the warps waited on global loads (9 of 17 stalled warps an issue, the tensor pipe
+// 28 - 36 % active).  Every output adds the same products in the same order (slices, taps, halves
+// of a slice) whatever the tile, so the tile may follow the shape.  Forward of 1 x 408 x 408 (34
+// GFLOP): 314 us then, 269 us now.
+template <int CS, int NB, int MR, bool RESIDENT>
+constexpr int conv_smem() {
+  return (2 * (8 * MR + 2) * PW + (RESIDENT ? 1 : 2) * 9 * NB) * (CS + 8) * (int)sizeof(bf16);
+}
+
+template <int CS, int NB, int MR, bool RESIDENT>
+__global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x, int Cin, const bf16 *__restrict__ w,
+                                                     const float *__restrict__ bias, int relu,
+                                                     const bf16 *__restrict__ omask, bf16 *__restrict__ y, int Cout,
+                                                     int B, int H, int W) {
+  constexpr int CP = CS + 8, CH = CS / 8, ROWS = 8 * MR + 2, PATCH = ROWS * PW * CP, WSM = 9 * NB * CP;
+  extern __shared__ __align__(16) bf16 conv_sm[];
+  bf16 *const patches = conv_sm, *const weights = conv_sm + 2 * PATCH;
+  const int tiles_w = (W + TW - 1) / TW, tiles_h = (H + 8 * MR - 1) / (8 * MR), tiles = B * tiles_h * tiles_w;
+  const int co0 = blockIdx.y * NB, nslice = Cin / CS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int steps = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * nslice;
   // ldmatrix row addresses: A (pixels x channels, row-major), B (channels x couts, stored [cout][cin])
   const int am = (lane & 7) + 8 * ((lane >> 3) & 1), ak = 8 * (lane >> 4);
   const int bn = (lane & 7) + 8 * (lane >> 4), bk = 8 * ((lane >> 3) & 1);
-  float acc[NT / 8][4];
-#pragma unroll
-  for (int n = 0; n < NT / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
-  for (int c0 = 0; c0 < Cin; c0 += CS) {
-    stage_patch<CS, THREADS>(patch, x, xmask, Cin, c0, b, i0, j0, H, W);
-    for (int q = threadIdx.x; q < 9 * NT * CH; q += THREADS) {
-      const int row = q / CH, ch = q - row * CH;   // row = tap * NT + n
-      const int tap = row / NT, n = row - tap * NT;
-      *reinterpret_cast<uint4 *>(wsm + row * CP + ch * 8) =
-          *reinterpret_cast<const uint4 *>(w + ((size_t)tap * Cout + co0 + n) * Cin + c0 + ch * 8);
+  auto tile_at = [&](int step, int &b, int &i0, int &j0) {
+    int t = blockIdx.x + step / nslice * gridDim.x;
+    b = t / (tiles_h * tiles_w);
+    t -= b * tiles_h * tiles_w;
+    i0 = t / tiles_w * 8 * MR;
+    j0 = t % tiles_w * TW;
+  };
+  // Channel n of a group of 32 goes to row 8 ((n mod 8) / 2) + 2 (n / 8) + n mod 2 of the staged
+  // weights: a lane's columns of the four n-blocks are then eight neighbouring channels, 16 bytes
+  // of a pixel.
+  auto copy_weights = [&](bf16 *to, int c0) {
+    for (int q = threadIdx.x; q < 9 * NB * CH; q += THREADS) {
+      const int row = q / CH, ch = q - row * CH;   // row = tap * NB + n
+      const int tap = row / NB, n = row - tap * NB;
+      const int at = (n & ~31) + 8 * ((n & 7) >> 1) + 2 * ((n & 31) >> 3) + (n & 1);
+      copy16(to + (tap * NB + at) * CP + ch * 8, w + ((size_t)tap * Cout + co0 + n) * Cin + c0 + ch * 8, true);
     }
+  };
+  auto copy_step = [&](int step) {
+    int b, i0, j0;
+    tile_at(step, b, i0, j0);
+    const int c0 = step % nslice * CS;
+    copy_patch<CS, THREADS, ROWS>(patches + (step & 1) * PATCH, x, Cin, c0, b, i0, j0, H, W);
+    if (!RESIDENT) copy_weights(weights + (step & 1) * WSM, c0);
+  };
+  if (RESIDENT) copy_weights(weights, 0);
+  copy_step(0);
+  copy_commit();
+  float acc[MR][NB / 8][4];
+#pragma unroll
+  for (int m = 0; m < MR; ++m)
+#pragma unroll
+    for (int n = 0; n < NB / 8; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
+  for (int step = 0; step < steps; ++step) {
+    if (step + 1 < steps) copy_step(step + 1);
+    copy_commit();
+    copy_wait<1>();
     __syncthreads();
+    const bf16 *const patch = patches + (step & 1) * PATCH;
+    const bf16 *const wsm = RESIDENT ? weights : weights + (step & 1) * WSM;
 #pragma unroll
     for (int tap = 0; tap < 9; ++tap) {
       const int ky = tap / 3, kx = tap - 3 * (tap / 3);
 #pragma unroll
       for (int kk = 0; kk < CS; kk += 16) {
-        uint32_t a[4];
-        ldsm_x4(a, patch + ((warp + ky) * PW + am + kx) * CP + kk + ak);
+        uint32_t a[MR][4];
 #pragma unroll
-        for (int nb2 = 0; nb2 < NT / 16; ++nb2) {
+        for (int m = 0; m < MR; ++m) ldsm_x4(a[m], patch + ((MR * warp + m + ky) * PW + am + kx) * CP + kk + ak);
+#pragma unroll
+        for (int nb2 = 0; nb2 < NB / 16; ++nb2) {
           uint32_t bb[4];
-          ldsm_x4(bb, wsm + (tap * NT + nb2 * 16 + bn) * CP + kk + bk);
-          mma_bf16(acc[2 * nb2], a, bb[0], bb[1]);
-          mma_bf16(acc[2 * nb2 + 1], a, bb[2], bb[3]);
+          ldsm_x4(bb, wsm + (tap * NB + nb2 * 16 + bn) * CP + kk + bk);
+#pragma unroll
+          for (int m = 0; m < MR; ++m) {
+            mma_bf16(acc[m][2 * nb2], a[m], bb[0], bb[1]);
+            mma_bf16(acc[m][2 * nb2 + 1], a[m], bb[2], bb[3]);
+          }
         }
       }
     }
-    __syncthreads();
-  }
-  const int g = lane >> 2, tq = lane & 3, i = i0 + warp;
-  if (i >= H) return;
+    __syncthreads();   // this step's buffers are free for the step after next
+    if ((step + 1) % nslice != 0) continue;
+    int b, i0, j0;
+    tile_at(step, b, i0, j0);
+    const int g = lane >> 2, tq = lane & 3;
 #pragma unroll
-  for (int nb = 0; nb < NT / 8; ++nb) {
-    const int co = co0 + nb * 8 + 2 * tq;
-    const float b0 = bias ? bias[co] : 0.0f, b1 = bias ? bias[co + 1] : 0.0f;
+    for (int m = 0; m < MR; ++m) {
+      const int i = i0 + MR * warp + m;
 #pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-      const int j = j0 + g + 8 * hh;
-      if (j >= W) continue;
-      float v0 = acc[nb][2 * hh] + b0, v1 = acc[nb][2 * hh + 1] + b1;
-      if (relu) {
-        v0 = fmaxf(v0, 0.0f);
-        v1 = fmaxf(v1, 0.0f);
+      for (int q = 0; q < NB / 32; ++q) {
+        const int co = co0 + 32 * q + 8 * tq;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const int j = j0 + g + 8 * hh;
+          float v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            v[u] = acc[m][4 * q + u / 2][2 * hh + (u & 1)] + (bias ? bias[co + u] : 0.0f);
+            acc[m][4 * q + u / 2][2 * hh + (u & 1)] = 0.0f;   // the next tile's
+            if (relu) v[u] = fmaxf(v[u], 0.0f);
+          }
+          if (i >= H || j >= W) continue;
+          const size_t off = (((size_t)b * H + i) * W + j) * Cout + co;
+          uint4 out = pack8(v);
+          if (omask) out = relu_mask8(out, *reinterpret_cast<const uint4 *>(omask + off));
+          *reinterpret_cast<uint4 *>(y + off) = out;
+        }
       }
-      *reinterpret_cast<__nv_bfloat162 *>(y + (((size_t)b * H + i) * W + j) * Cout + co) =
-          __floats2bfloat162_rn(v0, v1);
     }
   }
 }
 
 // ---- weight gradient ----
-// part[cta][tap][co][ci] = sum over the CTA's pixel tiles of dym[p, co] * x[p + tap offset, ci],
-// dym = dy * (ymask > 0).  grid = (ctas over pixel tiles, (Cout / 32) * (Cin / CS)).
-template <int CS>
+// part[cta][tap][co][ci] = sum over the CTA's pixel tiles of dy[p, co] * x[p + tap offset, ci] (dy
+// masked by its ReLU where it was made).  grid = (ctas over pixel tiles, (Cout / CO) * (Cin / CI)).
+// A tile's operands are copied two tiles ahead of their use.  A CTA's pixel ranges and the order
+// of their sums do not depend on CO and CI, which follow from how many CTAs they leave.
+//
+// Bound: the chain of a CTA's tiles (its sum's order is fixed).  Waiting for each tile's loads
+// took 4.3 us a tile.  Forward, backward and Adam of 16 x 128 x 128: 1.87 ms then, 1.13 ms now, of
+// which the gradients on a stream of their own, one launch for all flipped weights and the masks
+// made by their producers are a part.
+constexpr int WG_STAGES = 3;
+template <int CI, int CO>
+constexpr int wgrad_smem() {
+  return WG_STAGES * (PH * PW * (CI + 8) + TH * TW * (CO + 8)) * (int)sizeof(bf16);
+}
+
+template <int CI, int CO>
 __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(const bf16 *__restrict__ x, int Cin,
-                                                              const bf16 *__restrict__ dy,
-                                                              const bf16 *__restrict__ ymask, int Cout, int B, int H,
+                                                              const bf16 *__restrict__ dy, int Cout, int B, int H,
                                                               int W, float *__restrict__ part) {
-  constexpr int CP = CS + 8, DP = NT + 8;
-  __shared__ __align__(16) bf16 patch[PH * PW * CP];
-  __shared__ __align__(16) bf16 dys[TH * TW * DP];
-  const int nci = Cin / CS;
-  const int co0 = (blockIdx.y / nci) * NT, ci0 = (blockIdx.y % nci) * CS;
+  constexpr int CP = CI + 8, DP = CO + 8, PATCH = PH * PW * CP, DYS = TH * TW * DP;
+  extern __shared__ __align__(16) bf16 wg_sm[];
+  const int nci = Cin / CI;
+  const int co0 = (blockIdx.y / nci) * CO, ci0 = (blockIdx.y % nci) * CI;
   const int tiles_w = (W + TW - 1) / TW, tiles_h = (H + TH - 1) / TH, tiles = B * tiles_h * tiles_w;
   const int tap = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ky = tap / 3, kx = tap - 3 * (tap / 3);
   // A = dy^T (couts x pixels) from [pixel][cout]; B = x (pixels x cins) from [pixel][cin]
   const int apx = (lane & 7) + 8 * (lane >> 4), amo = 8 * ((lane >> 3) & 1);
   const int bpx = (lane & 7) + 8 * ((lane >> 3) & 1), bno = 8 * (lane >> 4);
-  float acc[2][CS / 8][4];
+  float acc[CO / 16][CI / 8][4];
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int m = 0; m < CO / 16; ++m)
 #pragma unroll
-    for (int n = 0; n < CS / 8; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
-  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    for (int n = 0; n < CI / 8; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
+  auto copy_tile = [&](int t, int stage) {
+    bf16 *const patch = wg_sm + stage * (PATCH + DYS), *const dys = patch + PATCH;
     int r = t;
     const int b = r / (tiles_h * tiles_w);
     r -= b * tiles_h * tiles_w;
     const int i0 = (r / tiles_w) * TH, j0 = (r % tiles_w) * TW;
-    stage_patch<CS, WG_THREADS>(patch, x, nullptr, Cin, ci0, b, i0, j0, H, W);
-    for (int q = threadIdx.x; q < TH * TW * (NT / 8); q += WG_THREADS) {
-      const int pix = q / (NT / 8), ch = q - pix * (NT / 8);
+    copy_patch<CI, WG_THREADS, PH>(patch, x, Cin, ci0, b, i0, j0, H, W);
+    for (int q = threadIdx.x; q < TH * TW * (CO / 8); q += WG_THREADS) {
+      const int pix = q / (CO / 8), ch = q - pix * (CO / 8);
       const int ii = i0 + pix / TW, jj = j0 + pix % TW;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (ii < H && jj < W) {
-        const size_t off = (((size_t)b * H + ii) * W + jj) * Cout + co0 + ch * 8;
-        v = *reinterpret_cast<const uint4 *>(dy + off);
-        if (ymask) v = relu_mask8(v, *reinterpret_cast<const uint4 *>(ymask + off));
-      }
-      *reinterpret_cast<uint4 *>(dys + pix * DP + ch * 8) = v;
+      const bool inside = ii < H && jj < W;
+      copy16(dys + pix * DP + ch * 8, inside ? dy + (((size_t)b * H + ii) * W + jj) * Cout + co0 + ch * 8 : dy, inside);
     }
-    __syncthreads();
+  };
+  int next = blockIdx.x, fill = 0;
+#pragma unroll
+  for (int q = 0; q < WG_STAGES - 1; ++q, next += gridDim.x) {
+    if (next < tiles) copy_tile(next, fill);
+    copy_commit();
+    ++fill;
+  }
+  int use = 0;
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x, next += gridDim.x) {
+    copy_wait<WG_STAGES - 2>();
+    __syncthreads();   // this tile is there for all, and the stage filled next is free
+    if (next < tiles) copy_tile(next, fill);
+    copy_commit();
+    if (++fill == WG_STAGES) fill = 0;
+    const bf16 *const patch = wg_sm + use * (PATCH + DYS), *const dys = patch + PATCH;
+    if (++use == WG_STAGES) use = 0;
 #pragma unroll 2
     for (int row = 0; row < TH; ++row) {
-      uint32_t a[2][4];
+      uint32_t a[CO / 16][4];
 #pragma unroll
-      for (int mb = 0; mb < 2; ++mb) ldsm_x4_t(a[mb], dys + (row * TW + apx) * DP + mb * 16 + amo);
+      for (int mb = 0; mb < CO / 16; ++mb) ldsm_x4_t(a[mb], dys + (row * TW + apx) * DP + mb * 16 + amo);
 #pragma unroll
-      for (int nb2 = 0; nb2 < CS / 16; ++nb2) {
+      for (int nb2 = 0; nb2 < CI / 16; ++nb2) {
         uint32_t bb[4];
         ldsm_x4_t(bb, patch + ((row + ky) * PW + bpx + kx) * CP + nb2 * 16 + bno);
 #pragma unroll
-        for (int mb = 0; mb < 2; ++mb) {
+        for (int mb = 0; mb < CO / 16; ++mb) {
           mma_bf16(acc[mb][2 * nb2], a[mb], bb[0], bb[1]);
           mma_bf16(acc[mb][2 * nb2 + 1], a[mb], bb[2], bb[3]);
         }
       }
     }
-    __syncthreads();
   }
   const int g = lane >> 2, tq = lane & 3;
   float *dst = part + ((size_t)blockIdx.x * 9 + tap) * Cout * Cin;
 #pragma unroll
-  for (int mb = 0; mb < 2; ++mb)
+  for (int mb = 0; mb < CO / 16; ++mb)
 #pragma unroll
-    for (int nb = 0; nb < CS / 8; ++nb)
+    for (int nb = 0; nb < CI / 8; ++nb)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         const int co = co0 + mb * 16 + g + 8 * hh, ci = ci0 + nb * 8 + 2 * tq;
@@ -275,24 +359,58 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(const bf16 *__rest
 __global__ void k_reduce_parts(const float *__restrict__ part, int nparts, int n, float *__restrict__ out) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     float s = 0.0f;
-    for (int q = 0; q < nparts; ++q) s += part[(size_t)q * n + k];
+    int q = 0;
+    for (; q + 16 <= nparts; q += 16) {   // sixteen loads in flight
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = part[(size_t)(q + u) * n + k];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) s += v[u];
+    }
+    for (; q < nparts; ++q) s += part[(size_t)q * n + k];
     out[k] = s;
   }
 }
 
-// part[cta][c] = sum over the CTA's pixels of dy[p, c] * (ymask[p, c] > 0)
-__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dy, const bf16 *__restrict__ ymask, int C,
-                                                   long long P, float *__restrict__ part) {
+// the same for few outputs (n <= 128): one block brings the parts to shared memory in rows of
+// 64, then a thread adds an output's in order
+constexpr int RS_ROWS = 64, RS_MAX = 128;
+__global__ void __launch_bounds__(256) k_reduce_few(const float *__restrict__ part, int nparts, int n,
+                                                    float *__restrict__ out) {
+  __shared__ float rows[RS_ROWS * RS_MAX];
+  float s = 0.0f;
+  for (int q0 = 0; q0 < nparts; q0 += RS_ROWS) {
+    const int nq = min(RS_ROWS, nparts - q0);
+    __syncthreads();
+#pragma unroll 8
+    for (int e = threadIdx.x; e < nq * n; e += 256) rows[e] = part[(size_t)q0 * n + e];
+    __syncthreads();
+    if ((int)threadIdx.x < n) {
+#pragma unroll 16
+      for (int q = 0; q < nq; ++q) s += rows[q * n + threadIdx.x];
+    }
+  }
+  if ((int)threadIdx.x < n) out[threadIdx.x] = s;
+}
+
+// part[cta][c] = sum over the CTA's pixels of dy[p, c]
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dy, int C, long long P,
+                                                   float *__restrict__ part) {
   __shared__ float red[256];
   const int lanes = 256 / C;   // pixels in flight per CTA
   const int c = threadIdx.x % C, l = threadIdx.x / C;
   float s = 0.0f;
   if (l < lanes) {
-    for (long long p = (long long)blockIdx.x * lanes + l; p < P; p += (long long)gridDim.x * lanes) {
-      const bf16 v = dy[p * C + c];
-      const bf16 m = ymask[p * C + c];
-      if (__bfloat162float(m) > 0.0f) s += __bfloat162float(v);
+    const long long stride = (long long)gridDim.x * lanes;
+    long long p = (long long)blockIdx.x * lanes + l;
+    for (; p + 15 * stride < P; p += 16 * stride) {   // sixteen loads in flight
+      bf16 v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = dy[(p + u * stride) * C + c];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) s += __bfloat162float(v[u]);
     }
+    for (; p < P; p += stride) s += __bfloat162float(dy[p * C + c]);
   }
   red[threadIdx.x] = s;
   __syncthreads();
@@ -303,9 +421,16 @@ __global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ dy, 
   }
 }
 
-// wt[8 - tap][ci][co] = w[tap][co][ci]: the backward-data weights
-__global__ void k_flip_weights(const bf16 *__restrict__ w, int Cout, int Cin, bf16 *__restrict__ wt) {
-  const int n = 9 * Cout * Cin;
+// wt[8 - tap][ci][co] = w[tap][co][ci]: the backward-data weights of layers 1 .. NLAYERS - 1
+// (blockIdx.y), at their offsets in the parameter and the flipped arrays
+struct FlipLayers {
+  long long w[NLAYERS], wt[NLAYERS];
+  int cin[NLAYERS], cout[NLAYERS];
+};
+__global__ void k_flip_weights(const bf16 *__restrict__ p16, FlipLayers F, bf16 *__restrict__ flip) {
+  const int l = blockIdx.y + 1, Cin = F.cin[l], Cout = F.cout[l], n = 9 * Cout * Cin;
+  const bf16 *__restrict__ w = p16 + F.w[l];
+  bf16 *__restrict__ wt = flip + F.wt[l];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const int tap = k / (Cout * Cin), r = k - tap * Cout * Cin, co = r / Cin, ci = r - co * Cin;
     wt[((size_t)(8 - tap) * Cin + ci) * Cout + co] = w[k];
@@ -338,8 +463,9 @@ __global__ void k_pool(const bf16 *__restrict__ x, int C, int B, int H, int W, b
   }
 }
 
-// dx[b, i, j, :] += dy[b, i/2, j/2, :] / 4
-__global__ void k_pool_back_add(const bf16 *__restrict__ dy, int C, int B, int H, int W, bf16 *__restrict__ dx) {
+// dx[b, i, j, :] += dy[b, i/2, j/2, :] / 4, then zero where ymask <= 0 (dx's own ReLU)
+__global__ void k_pool_back_add(const bf16 *__restrict__ dy, int C, int B, int H, int W,
+                                const bf16 *__restrict__ ymask, bf16 *__restrict__ dx) {
   const int h = H / 2, w = W / 2, CH = C / 8;
   const long long n = (long long)B * H * W * CH;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -355,7 +481,7 @@ __global__ void k_pool_back_add(const bf16 *__restrict__ dy, int C, int B, int H
     unpack8(*reinterpret_cast<const uint4 *>(dy + (((size_t)b * h + i / 2) * w + j / 2) * C + ch * 8), d);
 #pragma unroll
     for (int q = 0; q < 8; ++q) a[q] += 0.25f * d[q];
-    *reinterpret_cast<uint4 *>(dst) = pack8(a);
+    *reinterpret_cast<uint4 *>(dst) = relu_mask8(pack8(a), *reinterpret_cast<const uint4 *>(ymask + (dst - dx)));
   }
 }
 
@@ -378,9 +504,10 @@ __global__ void k_upcat(const bf16 *__restrict__ u, int Cu, const bf16 *__restri
   }
 }
 
-// du[b, I, J, :] = sum of dc[b, 2I + di, 2J + dj, 0:Cu];  ds[b, i, j, :] = dc[b, i, j, Cu:]
-__global__ void k_upcat_back(const bf16 *__restrict__ dc, int Cu, int Cs, int B, int H, int W, bf16 *__restrict__ du,
-                             bf16 *__restrict__ ds) {
+// du[b, I, J, :] = sum of dc[b, 2I + di, 2J + dj, 0:Cu], zero where umask <= 0 (du's ReLU);
+// ds[b, i, j, :] = dc[b, i, j, Cu:]
+__global__ void k_upcat_back(const bf16 *__restrict__ dc, int Cu, int Cs, int B, int H, int W,
+                             const bf16 *__restrict__ umask, bf16 *__restrict__ du, bf16 *__restrict__ ds) {
   const int C = Cu + Cs, h = H / 2, w = W / 2;
   const long long nu = (long long)B * h * w * (Cu / 8), ns = (long long)B * H * W * (Cs / 8);
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nu + ns;
@@ -400,7 +527,8 @@ __global__ void k_upcat_back(const bf16 *__restrict__ dc, int Cu, int Cs, int B,
 #pragma unroll
         for (int q = 0; q < 8; ++q) s[q] += f[q];
       }
-      *reinterpret_cast<uint4 *>(du + (((size_t)b * h + I) * w + J) * Cu + ch * 8) = pack8(s);
+      const size_t off = (((size_t)b * h + I) * w + J) * Cu + ch * 8;
+      *reinterpret_cast<uint4 *>(du + off) = relu_mask8(pack8(s), *reinterpret_cast<const uint4 *>(umask + off));
     } else {
       const long long kk = k - nu;
       const int CH = Cs / 8, ch = (int)(kk % CH);
@@ -472,12 +600,17 @@ __global__ void __launch_bounds__(256) k_loss_parts(const float *__restrict__ y,
 }
 
 // sums = {ordered sum of the loss parts, sum of weights, loss = sums[0] / (2 sums[1])}
-__global__ void k_loss_finish(const float *__restrict__ part, int nparts, float *__restrict__ sums) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
+__global__ void __launch_bounds__(256) k_loss_finish(const float *__restrict__ part, int nparts,
+                                                     float *__restrict__ sums) {
+  __shared__ float p[2 * 256];   // nparts <= 256
+  for (int q = threadIdx.x; q < 2 * nparts; q += 256) p[q] = part[q];
+  __syncthreads();
+  if (threadIdx.x == 0) {
     float a = 0.0f, b = 0.0f;
+#pragma unroll 16
     for (int q = 0; q < nparts; ++q) {
-      a += part[2 * q];
-      b += part[2 * q + 1];
+      a += p[2 * q];
+      b += p[2 * q + 1];
     }
     sums[0] = a;
     sums[1] = b;
@@ -485,7 +618,7 @@ __global__ void k_loss_finish(const float *__restrict__ part, int nparts, float 
   }
 }
 
-// dy = w (y - t) / sum w;  dd1[p, c] = sum_o dy[p, o] Wh[o, c];
+// dy = w (y - t) / sum w;  dd1[p, c] = sum_o dy[p, o] Wh[o, c], zero where d1 <= 0 (its ReLU);
 // part[cta] = {dWh[2][32], dbh[2]} partial sums
 __global__ void __launch_bounds__(256) k_head_back(const bf16 *__restrict__ d1, const float *__restrict__ y,
                                                    const float *__restrict__ t, const float *__restrict__ wgt,
@@ -512,7 +645,8 @@ __global__ void __launch_bounds__(256) k_head_back(const bf16 *__restrict__ d1, 
         g[c] = fmaf(e0, f[q], g[c]);
         g[HEAD_CIN + c] = fmaf(e1, f[q], g[HEAD_CIN + c]);
       }
-      reinterpret_cast<uint4 *>(dd1 + p * HEAD_CIN)[ch] = pack8(o);
+      reinterpret_cast<uint4 *>(dd1 + p * HEAD_CIN)[ch] =
+          relu_mask8(pack8(o), reinterpret_cast<const uint4 *>(d1 + p * HEAD_CIN)[ch]);
     }
     g[2 * HEAD_CIN] += e0;
     g[2 * HEAD_CIN + 1] += e1;
@@ -720,7 +854,10 @@ struct pism_gpu_unet {
   long long flip_n = 0;
   float *wg_part = nullptr;   // weight-gradient partial sums
   size_t wg_part_n = 0;
-  float *small_part = nullptr;   // bias / head / loss partial sums
+  float *small_part = nullptr;   // head / loss partial sums
+  float *bias_part = nullptr;    // bias partial sums
+  cudaStream_t side = nullptr;   // the weight gradients, beside the data gradients
+  cudaEvent_t ready[NLAYERS] = {}, side_done = nullptr;
   float *sums = nullptr;
   float *sums_host = nullptr;
   // activations (bf16) and their gradients
@@ -780,42 +917,101 @@ cudaError_t ualloc(T **p, size_t count) {
 // level-l pixel count of a B x H x W image
 inline long long pixels(int B, int H, int W, int l) { return (long long)B * (H >> l) * (W >> l); }
 
-void conv_fwd(pism_gpu_unet *h, const bf16 *x, const bf16 *xmask, int Cin, const bf16 *w, const float *bias, int relu,
-              bf16 *y, int Cout, int B, int H, int W) {
-  const int tiles = B * ((H + TH - 1) / TH) * ((W + TW - 1) / TW);
-  dim3 grid(tiles, Cout / NT);
-  if (Cin % 32 == 0)
-    k_conv3x3<32><<<grid, THREADS, 0, h->stream>>>(x, xmask, Cin, w, bias, relu, y, Cout, H, W);
-  else
-    k_conv3x3<16><<<grid, THREADS, 0, h->stream>>>(x, xmask, Cin, w, bias, relu, y, Cout, H, W);
+constexpr int UNET_SMS = 148;
+
+// one kernel form: its dynamic shared memory (granted when a handle is created) and its launch
+template <int CS, int NB, int MR, bool RESIDENT>
+struct Conv {
+  static constexpr int smem = conv_smem<CS, NB, MR, RESIDENT>();
+  static bool allow() {
+    return cudaFuncSetAttribute((const void *)k_conv3x3<CS, NB, MR, RESIDENT>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+  }
+  static void launch(cudaStream_t s, const bf16 *x, int Cin, const bf16 *w, const float *bias, int relu,
+                     const bf16 *omask, bf16 *y, int Cout, int B, int H, int W) {
+    const int tiles = B * ((H + 8 * MR - 1) / (8 * MR)) * ((W + TW - 1) / TW), ny = Cout / NB;
+    // Where the weights stay, as many CTAs as are resident at once, each with the same number of
+    // tiles (a first tile cannot overlap its loads).  Several slices pipeline within a tile and
+    // fetch their weights for each: a tile a CTA, whose start and end then overlap its
+    // neighbours' (forward of 1 x 408 x 408: 269 us; equal shares 289, pairs of tiles 310).
+    const int most = std::max(1, UNET_SMS * std::min(3, (220 * 1024) / smem) / ny);
+    const int per = RESIDENT ? (tiles + most - 1) / most : 1, ctas = (tiles + per - 1) / per;
+    k_conv3x3<CS, NB, MR, RESIDENT><<<dim3(ctas, ny), THREADS, smem, s>>>(x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+  }
+};
+template <int CI, int CO>
+struct Wgrad {
+  static constexpr int smem = wgrad_smem<CI, CO>();
+  static bool allow() {
+    return cudaFuncSetAttribute((const void *)k_conv3x3_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                smem) == cudaSuccess;
+  }
+  static void launch(cudaStream_t s, const bf16 *x, int Cin, const bf16 *dy, int Cout, int B, int H, int W, int ctas,
+                     float *part) {
+    k_conv3x3_wgrad<CI, CO><<<dim3(ctas, (Cout / CO) * (Cin / CI)), WG_THREADS, smem, s>>>(x, Cin, dy, Cout, B, H, W,
+                                                                                          part);
+  }
+};
+bool allow_kernels() {
+  return Conv<32, 32, 2, true>::allow() && Conv<32, 32, 2, false>::allow() && Conv<32, 32, 1, true>::allow() &&
+         Conv<32, 32, 1, false>::allow() && Conv<16, 32, 2, true>::allow() && Conv<16, 32, 1, true>::allow() &&
+         Wgrad<32, 32>::allow() && Wgrad<32, 16>::allow() && Wgrad<16, 16>::allow();
 }
 
-void conv_wgrad(pism_gpu_unet *h, const bf16 *x, int Cin, const bf16 *dy, const bf16 *ymask, int Cout, int B, int H,
-                int W, float *dW) {
+// 16 x 16 pixels where that leaves every SM a CTA, else 8 x 16; the weights stay in shared memory
+// where the layer is one slice
+void conv(cudaStream_t s, const bf16 *x, int Cin, const bf16 *w, const float *bias, int relu, const bf16 *omask,
+          bf16 *y, int Cout, int B, int H, int W) {
+  const bool tall = (long long)B * ((H + 15) / 16) * ((W + TW - 1) / TW) * (Cout / 32) >= UNET_SMS;
+  if (Cin == 16) {
+    if (tall) Conv<16, 32, 2, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    else Conv<16, 32, 1, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+  } else if (Cin == 32) {
+    if (tall) Conv<32, 32, 2, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    else Conv<32, 32, 1, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+  } else {
+    if (tall) Conv<32, 32, 2, false>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    else Conv<32, 32, 1, false>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+  }
+}
+
+// dW: the channel blocks are halved while that still leaves SMs without a CTA
+void conv_wgrad(pism_gpu_unet *h, cudaStream_t s, const bf16 *x, int Cin, const bf16 *dy, int Cout, int B, int H, int W,
+                float *dW) {
   const int tiles = B * ((H + TH - 1) / TH) * ((W + TW - 1) / TW);
   const int ctas = std::min(tiles, WG_MAX_CTAS);
-  const int CS = (Cin % 32 == 0) ? 32 : 16;
-  dim3 grid(ctas, (Cout / NT) * (Cin / CS));
-  if (CS == 32)
-    k_conv3x3_wgrad<32><<<grid, WG_THREADS, 0, h->stream>>>(x, Cin, dy, ymask, Cout, B, H, W, h->wg_part);
-  else
-    k_conv3x3_wgrad<16><<<grid, WG_THREADS, 0, h->stream>>>(x, Cin, dy, ymask, Cout, B, H, W, h->wg_part);
+  const int blocks = ctas * (Cout / 32) * std::max(1, Cin / 32);   // with blocks of 32 x 32
+  const bool half = blocks < 2 * UNET_SMS, quarter = blocks < UNET_SMS;
+  if (Cin % 32 != 0 || quarter) {   // 16 input channels: the first layer only, one block of 32 x 32
+    Wgrad<16, 16>::launch(s, x, Cin, dy, Cout, B, H, W, ctas, h->wg_part);
+  } else if (half) {
+    Wgrad<32, 16>::launch(s, x, Cin, dy, Cout, B, H, W, ctas, h->wg_part);
+  } else {
+    Wgrad<32, 32>::launch(s, x, Cin, dy, Cout, B, H, W, ctas, h->wg_part);
+  }
   const int n = 9 * Cout * Cin;
-  k_reduce_parts<<<grid_for(n), 256, 0, h->stream>>>(h->wg_part, ctas, n, dW);
+  k_reduce_parts<<<grid_for(n), 256, 0, s>>>(h->wg_part, ctas, n, dW);
 }
 
-void bias_grad(pism_gpu_unet *h, const bf16 *dy, const bf16 *ymask, int C, long long P, float *db) {
+void bias_grad(pism_gpu_unet *h, cudaStream_t s, const bf16 *dy, int C, long long P, float *db) {
   const int ctas = (int)std::min<long long>(256, std::max(1LL, P / 64));
-  k_bias_grad<<<ctas, 256, 0, h->stream>>>(dy, ymask, C, P, h->small_part);
-  k_reduce_parts<<<1, 128, 0, h->stream>>>(h->small_part, ctas, C, db);
+  k_bias_grad<<<ctas, 256, 0, s>>>(dy, C, P, h->bias_part);
+  k_reduce_few<<<1, 256, 0, s>>>(h->bias_part, ctas, C, db);
 }
 
-// layer l backward: X input, Y output (post-ReLU), dY given; writes dW, db and (if dX) dX
-void layer_back(pism_gpu_unet *h, int l, const bf16 *X, const bf16 *Y, const bf16 *dY, bf16 *dX, int B, int H, int W) {
+// Layer l backward: X input, dY given, masked by the layer's ReLU; dX (masked by xmask, its own
+// layer's output, where given) on the handle's stream, dW and db beside it on the second one: the
+// data gradients are the only chain.
+cudaError_t layer_back(pism_gpu_unet *h, int l, const bf16 *X, const bf16 *dY, bf16 *dX, const bf16 *xmask, int B, int H,
+                       int W) {
   const LayerDef &L = LAYERS[l];
-  conv_wgrad(h, X, L.cin, dY, Y, L.cout, B, H, W, h->grad + h->w_off[l]);
-  bias_grad(h, dY, Y, L.cout, (long long)B * H * W, h->grad + h->b_off[l]);
-  if (dX) conv_fwd(h, dY, Y, L.cout, h->flip + h->flip_off[l], nullptr, 0, dX, L.cin, B, H, W);
+  cudaError_t e = cudaEventRecord(h->ready[l], h->stream);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ready[l], 0);
+  if (e != cudaSuccess) return e;
+  if (dX) conv(h->stream, dY, L.cout, h->flip + h->flip_off[l], nullptr, 0, xmask, dX, L.cin, B, H, W);
+  conv_wgrad(h, h->side, X, L.cin, dY, L.cout, B, H, W, h->grad + h->w_off[l]);
+  bias_grad(h, h->side, dY, L.cout, (long long)B * H * W, h->grad + h->b_off[l]);
+  return cudaSuccess;
 }
 
 int check_shape(pism_gpu_unet *h, int B, int H, int W) {
@@ -909,6 +1105,7 @@ int pism_gpu_unet_create(int device, int max_batch, int max_h, int max_w, pism_g
   A(&h->flip, h->flip_n);
   AF(&h->wg_part, h->wg_part_n);
   AF(&h->small_part, 256 * 130);
+  AF(&h->bias_part, 256 * 130);
   AF(&h->sums, 4);
   if (rc == PISM_GPU_SSA_OK && cudaMallocHost((void **)&h->sums_host, 4 * sizeof(float)) != cudaSuccess)
     rc = PISM_GPU_SSA_ENOMEM;
@@ -937,6 +1134,12 @@ int pism_gpu_unet_create(int device, int max_batch, int max_h, int max_w, pism_g
   A(&h->de2a, P(1) * 64);
   A(&h->dp1, P(1) * 32);
   A(&h->de1a, P(0) * 32);
+  if (rc == PISM_GPU_SSA_OK) {
+    bool ok = allow_kernels() && cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaEventCreateWithFlags(&h->side_done, cudaEventDisableTiming) == cudaSuccess;
+    for (cudaEvent_t &e : h->ready) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) rc = PISM_GPU_SSA_ECUDA;
+  }
   if (rc != PISM_GPU_SSA_OK) {
     pism_gpu_unet_destroy(h);
     return rc;
@@ -958,7 +1161,12 @@ int pism_gpu_unet_destroy(pism_gpu_unet *h) {
   if (!h) return PISM_GPU_SSA_OK;
   UDevice dg(h->device);
   cudaStreamSynchronize(h->stream);
-  for (float *p : {h->p32, h->grad, h->m, h->v, h->wg_part, h->small_part, h->sums, h->y}) cudaFree(p);
+  if (h->side) cudaStreamSynchronize(h->side);
+  if (h->side) cudaStreamDestroy(h->side);
+  if (h->side_done) cudaEventDestroy(h->side_done);
+  for (cudaEvent_t e : h->ready)
+    if (e) cudaEventDestroy(e);
+  for (float *p : {h->p32, h->grad, h->m, h->v, h->wg_part, h->small_part, h->bias_part, h->sums, h->y}) cudaFree(p);
   for (bf16 *p : {h->p16, h->flip, h->in16, h->p1, h->p2, h->p3, h->c3, h->c2, h->c1, h->dd1, h->dc1, h->dd2, h->de1,
                   h->dc2, h->dd3, h->de2, h->dc3, h->dbt, h->de3, h->dp3, h->de3a, h->dp2, h->de2a, h->dp1, h->de1a})
     cudaFree(p);
@@ -1008,7 +1216,7 @@ int pism_gpu_unet_forward(pism_gpu_unet *h, const float *input, int B, int H, in
   const bf16 *w = h->p16;
   const float *p = h->p32;
   auto L = [&](int l, const bf16 *x, int Hl, int Wl) {
-    conv_fwd(h, x, nullptr, LAYERS[l].cin, w + h->w_off[l], p + h->b_off[l], 1, h->act[l], LAYERS[l].cout, B, Hl, Wl);
+    conv(h->stream, x, LAYERS[l].cin, w + h->w_off[l], p + h->b_off[l], 1, nullptr, h->act[l], LAYERS[l].cout, B, Hl, Wl);
   };
   k_pack_input<<<grid_for(P0), 256, 0, h->stream>>>(input, P0, h->in16);
   L(0, h->in16, H, W);
@@ -1046,38 +1254,47 @@ int pism_gpu_unet_backward(pism_gpu_unet *h, const float *target, const float *w
   const int B = h->B, H = h->H, W = h->W;
   const long long P0 = (long long)B * H * W;
   // weights of the backward-data convolutions
+  FlipLayers fl{};
   for (int l = 1; l < NLAYERS; ++l) {
-    const int n = 9 * LAYERS[l].cout * LAYERS[l].cin;
-    k_flip_weights<<<grid_for(n), 256, 0, h->stream>>>(h->p16 + h->w_off[l], LAYERS[l].cout, LAYERS[l].cin,
-                                                       h->flip + h->flip_off[l]);
+    fl.w[l] = h->w_off[l];
+    fl.wt[l] = h->flip_off[l];
+    fl.cin[l] = LAYERS[l].cin;
+    fl.cout[l] = LAYERS[l].cout;
   }
+  k_flip_weights<<<dim3(128, NLAYERS - 1), 256, 0, h->stream>>>(h->p16, fl, h->flip);
   // loss and the head
   const int lctas = (int)std::min<long long>(256, std::max(1LL, P0 / 256));
   k_loss_parts<<<lctas, 256, 0, h->stream>>>(h->y, target, weight, P0, h->small_part);
-  k_loss_finish<<<1, 32, 0, h->stream>>>(h->small_part, lctas, h->sums);
+  k_loss_finish<<<1, 256, 0, h->stream>>>(h->small_part, lctas, h->sums);
   const int hctas = (int)std::min<long long>(256, std::max(1LL, P0 / 256));
   constexpr int NG = HEAD_COUT * HEAD_CIN + HEAD_COUT;
   k_head_back<<<hctas, 256, 0, h->stream>>>(h->act[9], h->y, target, weight, h->sums, h->p32 + h->head_off, P0, h->dd1,
                                             h->small_part);
-  k_reduce_parts<<<1, 128, 0, h->stream>>>(h->small_part, hctas, NG, h->grad + h->head_off);
-  // decoder
-  layer_back(h, 9, h->c1, h->act[9], h->dd1, h->dc1, B, H, W);
-  k_upcat_back<<<grid_for(P0 * 12), 256, 0, h->stream>>>(h->dc1, 64, 32, B, H, W, h->dd2, h->de1);
-  layer_back(h, 8, h->c2, h->act[8], h->dd2, h->dc2, B, H / 2, W / 2);
-  k_upcat_back<<<grid_for(pixels(B, H, W, 1) * 20), 256, 0, h->stream>>>(h->dc2, 96, 64, B, H / 2, W / 2, h->dd3, h->de2);
-  layer_back(h, 7, h->c3, h->act[7], h->dd3, h->dc3, B, H / 4, W / 4);
-  k_upcat_back<<<grid_for(pixels(B, H, W, 2) * 28), 256, 0, h->stream>>>(h->dc3, 128, 96, B, H / 4, W / 4, h->dbt, h->de3);
+  k_reduce_few<<<1, 256, 0, h->stream>>>(h->small_part, hctas, NG, h->grad + h->head_off);
+  // decoder (every gradient masked by its layer's ReLU where it is made)
+  UCK(h, layer_back(h, 9, h->c1, h->dd1, h->dc1, nullptr, B, H, W));
+  k_upcat_back<<<grid_for(P0 * 12), 256, 0, h->stream>>>(h->dc1, 64, 32, B, H, W, h->act[8], h->dd2, h->de1);
+  UCK(h, layer_back(h, 8, h->c2, h->dd2, h->dc2, nullptr, B, H / 2, W / 2));
+  k_upcat_back<<<grid_for(pixels(B, H, W, 1) * 20), 256, 0, h->stream>>>(h->dc2, 96, 64, B, H / 2, W / 2, h->act[7],
+                                                                       h->dd3, h->de2);
+  UCK(h, layer_back(h, 7, h->c3, h->dd3, h->dc3, nullptr, B, H / 4, W / 4));
+  k_upcat_back<<<grid_for(pixels(B, H, W, 2) * 28), 256, 0, h->stream>>>(h->dc3, 128, 96, B, H / 4, W / 4, h->act[6],
+                                                                       h->dbt, h->de3);
   // bottleneck and encoder
-  layer_back(h, 6, h->p3, h->act[6], h->dbt, h->dp3, B, H / 8, W / 8);
-  k_pool_back_add<<<grid_for(pixels(B, H, W, 2) * 12), 256, 0, h->stream>>>(h->dp3, 96, B, H / 4, W / 4, h->de3);
-  layer_back(h, 5, h->act[4], h->act[5], h->de3, h->de3a, B, H / 4, W / 4);
-  layer_back(h, 4, h->p2, h->act[4], h->de3a, h->dp2, B, H / 4, W / 4);
-  k_pool_back_add<<<grid_for(pixels(B, H, W, 1) * 8), 256, 0, h->stream>>>(h->dp2, 64, B, H / 2, W / 2, h->de2);
-  layer_back(h, 3, h->act[2], h->act[3], h->de2, h->de2a, B, H / 2, W / 2);
-  layer_back(h, 2, h->p1, h->act[2], h->de2a, h->dp1, B, H / 2, W / 2);
-  k_pool_back_add<<<grid_for(P0 * 4), 256, 0, h->stream>>>(h->dp1, 32, B, H, W, h->de1);
-  layer_back(h, 1, h->act[0], h->act[1], h->de1, h->de1a, B, H, W);
-  layer_back(h, 0, h->in16, h->act[0], h->de1a, nullptr, B, H, W);
+  UCK(h, layer_back(h, 6, h->p3, h->dbt, h->dp3, nullptr, B, H / 8, W / 8));
+  k_pool_back_add<<<grid_for(pixels(B, H, W, 2) * 12), 256, 0, h->stream>>>(h->dp3, 96, B, H / 4, W / 4, h->act[5],
+                                                                          h->de3);
+  UCK(h, layer_back(h, 5, h->act[4], h->de3, h->de3a, h->act[4], B, H / 4, W / 4));
+  UCK(h, layer_back(h, 4, h->p2, h->de3a, h->dp2, nullptr, B, H / 4, W / 4));
+  k_pool_back_add<<<grid_for(pixels(B, H, W, 1) * 8), 256, 0, h->stream>>>(h->dp2, 64, B, H / 2, W / 2, h->act[3],
+                                                                         h->de2);
+  UCK(h, layer_back(h, 3, h->act[2], h->de2, h->de2a, h->act[2], B, H / 2, W / 2));
+  UCK(h, layer_back(h, 2, h->p1, h->de2a, h->dp1, nullptr, B, H / 2, W / 2));
+  k_pool_back_add<<<grid_for(P0 * 4), 256, 0, h->stream>>>(h->dp1, 32, B, H, W, h->act[1], h->de1);
+  UCK(h, layer_back(h, 1, h->act[0], h->de1, h->de1a, h->act[0], B, H, W));
+  UCK(h, layer_back(h, 0, h->in16, h->de1a, nullptr, nullptr, B, H, W));
+  UCK(h, cudaEventRecord(h->side_done, h->side));
+  UCK(h, cudaStreamWaitEvent(h->stream, h->side_done, 0));
   UCK(h, cudaGetLastError());
   if (grad_out)
     UCK(h, cudaMemcpyAsync(grad_out, h->grad, h->nparam * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
