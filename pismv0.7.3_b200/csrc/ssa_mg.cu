@@ -19,8 +19,8 @@
 //   x_l <- x_l + s P x_{l+1};  x_l <- x_l + omega D_l^-1 (b_l - A_l x_l)   (post kernel)
 // so each level costs two stencil passes.  Levels of <= MG_CTA_CELLS cells are cycled by
 // one thread-block cluster in one launch (their kernels would be launch- and
-// latency-bound), and their Galerkin operators and the coarsest inverse are built by one
-// cluster launch per Picard iteration.
+// latency-bound).  The Galerkin operators of the levels of at most MG_TAIL_CELLS cells and the
+// coarsest inverse are built by one block.
 // The defaults omega = 0.9 and s = 1.2 (mg_omega, mg_correction; s > 1 over-corrects to
 // compensate the piecewise-constant interpolation) come from a sweep of whole 801^2
 // synthetic solves: 7115 BiCGStab iterations against 9558 at (0.7, 1.5) and 8042 at
@@ -233,180 +233,231 @@ __global__ void __launch_bounds__(NTm) k_mg_build1(GridDev g, StencilConst s, co
   }
 }
 
-// Galerkin operator and D^-1 of coarse cell (I, J) of the level below F, summed in FP64 in
-// registers, fine cell by fine cell of the aggregate and block by block (no stores between
-// the loads, so the compiler may issue them all at once)
-__device__ __forceinline__ void galerkin_cell(const LevelView &F, int Mxc, int Myc, int I, int J, float4 *Ac,
-                                              float4 *dinvc) {
-  const int ax = F.ax, ay = F.ay;
-  double acc[36];
+// The Galerkin operators below level 1: four neighbouring lanes sum a coarse cell's nine blocks,
+// one of the blocks' four entries each (nine FP64 sums a thread), fine cell by fine cell of the
+// aggregate and block by block.  One thread a cell held 36 sums and nine float4 loads: 128
+// registers and 256 threads an SM, latency-bound (201 x 201 cells 9 us; now 3.4 us).
+__device__ __forceinline__ void acc_entry(double (&acc)[9], int cb, double x) {
 #pragma unroll
-  for (int q = 0; q < 36; ++q) acc[q] = 0.0;
-  const bool fast = static_blocks(ax, ay, Mxc, Myc);
+  for (int c = 0; c < 9; ++c)
+    if (cb == c) acc[c] += x;
+}
+
+// The operator above a coarse level: block b of cell k at A[b * N + k]
+struct GalerkinView {
+  int Mx, My, N, ax, ay;
+  const float4 *A;
+};
+
+// entry e (0 .. 3) of the blocks of coarse cell kc, from F; all four lanes of the cell call it.
+// Stored to Ac (and to the copy, where given) with D^-1.
+__device__ __forceinline__ void galerkin_entry(const GalerkinView &F, int Mxc, int Myc, int kc, int e, float4 *Ac,
+                                               float4 *dinvc, float4 *copy) {
+  const int Nc = Mxc * Myc, I = kc / Myc, J = kc - I * Myc;
+  double acc[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) acc[q] = 0.0;
+  const float *const A = reinterpret_cast<const float *>(F.A) + e;
+  const bool fast = static_blocks(F.ax, F.ay, Mxc, Myc);
   const bool ex = (F.Mx & 1) && I == Mxc - 1, ey = (F.My & 1) && J == Myc - 1;
-  auto fine = [&](auto PI, auto PJ) {
-    constexpr int pi = decltype(PI)::value, pj = decltype(PJ)::value;
-    const int i = I * ax + pi, j = J * ay + pj;
-    if (pi >= ax || pj >= ay || i >= F.Mx || j >= F.My) return;
-    const int k = i * F.My + j;
-    auto v = [&](int b) {
-      const float4 a = F.A[b * F.N + k];
-      return make_double4(a.x, a.y, a.z, a.w);
-    };
-    if (fast) {
-      acc_fine_static<pi, pj>(acc, ex, ey, v);
-    } else {
+  // all loads first: the aggregate's fine cells that exist
+  float a[4][9];
+  bool has[4];
 #pragma unroll
-      for (int b = 0; b < 9; ++b) {
-        const int di = (b % 3) - 1, dj = 1 - (b / 3);
+  for (int p = 0; p < 4; ++p) {
+    const int i = I * F.ax + p / 2, j = J * F.ay + p % 2;
+    has[p] = p / 2 < F.ax && p % 2 < F.ay && i < F.Mx && j < F.My;
+    const float *const at = A + 4 * (size_t)(has[p] ? i * F.My + j : 0);
+#pragma unroll
+    for (int b = 0; b < 9; ++b) a[p][b] = has[p] ? at[4 * (size_t)(b * F.N)] : 0.0f;
+  }
+  auto fine = [&](auto P) {
+    constexpr int p = decltype(P)::value, pi = p / 2, pj = p % 2;
+    if (!has[p]) return;
+    const int i = I * F.ax + pi, j = J * F.ay + pj;
+#pragma unroll
+    for (int b = 0; b < 9; ++b) {
+      const int di = (b % 3) - 1, dj = 1 - (b / 3);
+      if (fast) {
+        const int ci = (pi + di + 2) / 2 - 1, cj = (pj + dj + 2) / 2 - 1;   // floor((p + d) / 2)
+        const bool wx = pi == 0 && di == 1, wy = pj == 0 && dj == 1;       // may cross the odd edge
+        if (wx || wy) acc_entry(acc, blk_of(ci + (wx && ex ? 1 : 0), cj + (wy && ey ? 1 : 0)), a[p][b]);
+        else acc[blk_of(ci, cj)] += a[p][b];
+      } else {
         const int ni = wrap(i + di, F.Mx), nj = wrap(j + dj, F.My);
-        const double4 x = v(b);
-        acc_block(acc, blk_of(wdiff(ni / ax, I, Mxc), wdiff(nj / ay, J, Myc)), x.x, x.y, x.z, x.w);
+        acc_entry(acc, blk_of(wdiff(ni / F.ax, I, Mxc), wdiff(nj / F.ay, J, Myc)), a[p][b]);
       }
     }
   };
-  fine(std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{});
-  fine(std::integral_constant<int, 0>{}, std::integral_constant<int, 1>{});
-  fine(std::integral_constant<int, 1>{}, std::integral_constant<int, 0>{});
-  fine(std::integral_constant<int, 1>{}, std::integral_constant<int, 1>{});
-  store_coarse(acc, Mxc * Myc, I * Myc + J, Ac, dinvc);
+  fine(std::integral_constant<int, 0>{});
+  fine(std::integral_constant<int, 1>{});
+  fine(std::integral_constant<int, 2>{});
+  fine(std::integral_constant<int, 3>{});
+#pragma unroll
+  for (int b = 0; b < 9; ++b) {
+    const float v = (float)acc[b];
+    reinterpret_cast<float *>(Ac)[4 * (size_t)(b * Nc + kc) + e] = v;
+    if (copy) reinterpret_cast<float *>(copy)[4 * (b * Nc + kc) + e] = v;
+  }
+  const unsigned quad = 0xfu << (threadIdx.x & 28);
+  const float c = (float)acc[4];
+  const float c0 = __shfl_sync(quad, c, 0, 4), c1 = __shfl_sync(quad, c, 1, 4), c2 = __shfl_sync(quad, c, 2, 4),
+              c3 = __shfl_sync(quad, c, 3, 4);
+  if (e == 0) dinvc[kc] = inv2x2(c0, c1, c2, c3);
 }
 
 // level l+1 from the stored operator of level l
-__global__ void __launch_bounds__(NTm, 2) k_mg_build(LevelView F, int Mxc, int Myc, TileM tm, float4 *Ac, float4 *dinvc) {
-  for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
-    int I, J;
-    if (!tile_cell(tm, Mxc, Myc, t, I, J)) continue;
-    galerkin_cell(F, Mxc, Myc, I, J, Ac, dinvc);
-  }
+__global__ void __launch_bounds__(NTm) k_mg_build(GalerkinView F, int Mxc, int Myc, float4 *Ac, float4 *dinvc) {
+  pdl_wait();
+  pdl_release();
+  F.A = after_wait(F.A);
+  const int n = 4 * Mxc * Myc;
+  for (int q = blockIdx.x * NTm + threadIdx.x; q < n; q += gridDim.x * NTm)
+    galerkin_entry(F, Mxc, Myc, q >> 2, q & 3, Ac, dinvc, nullptr);
 }
 
 // Dense inverse of the coarsest operator (n = 2 N <= 32 unknowns) by Gauss-Jordan elimination
-// with partial pivoting, in place in shared memory, by one thread block (rows padded to 33
-// entries, so a column's entries of consecutive rows sit in different banks).  Warp 0 finds
-// each pivot, swaps and scales the pivot row (two block barriers per step in all); the
-// elimination spreads the n x n element updates of a step over the block,
-// reading the step's multipliers from a copy of the pivot column, so each element is updated
-// with the same operands in the same order whatever thread does it.  Written transposed, so
-// that the per-cycle product reads it coalesced.
-constexpr int CI_PAD = 2 * MG_MAX_COARSE_CELLS + 1;
-static_assert(2 * MG_MAX_COARSE_CELLS <= 32, "one lane per row of the coarsest operator");
-
+// with partial pivoting: thread (w, lane) of four warps has entries 8 w .. 8 w + 7 of row `lane` in
+// registers.  Rows are not interchanged; `pos` is where a row would be.  A step's column is its
+// warp's to search: the pivot is the largest |entry| at positions >= col, the first on ties; a
+// magnitude's bits order as integers, so warp-wide integer reductions find it while every lane
+// takes its own reciprocal.  The multipliers, the pivot's lane and reciprocal go to the other warps
+// through shared memory (two copies, so that one barrier a step is enough).
+//
+// Bound: the chain of n steps.  A block of 1024 threads, an element each, with two barriers a
+// step took 29 us for 16 cells, one warp with whole rows 14 us, four warps
+// 10 us: a step is two dependent chains of FP64 latencies, the reciprocal and the update.
 struct CoarseInvertSmem {
-  double a[2 * MG_MAX_COARSE_CELLS][CI_PAD];
-  double fcol[2 * MG_MAX_COARSE_CELLS];
-  int perm[2 * MG_MAX_COARSE_CELLS];
+  double a[2 * MG_MAX_COARSE_CELLS][2 * MG_MAX_COARSE_CELLS + 1];
+  double2 prow[4][4];
+  struct Step {
+    double f[2 * MG_MAX_COARSE_CELLS], pinv;
+    int lane, pos;
+  } step[2];
+  int own[2 * MG_MAX_COARSE_CELLS];
 };
+static_assert(2 * MG_MAX_COARSE_CELLS == 32, "one lane per row of the coarsest operator");
+constexpr int CI_THREADS = 128;
 
-__device__ void coarse_invert_block(const LevelView &L, CoarseInvertSmem &S, double *invT_out, int *singular) {
-  const int tid = threadIdx.x, nth = blockDim.x, n = 2 * L.N;
-  for (int q = tid; q < n * CI_PAD; q += nth) (&S.a[0][0])[q] = 0.0;
-  __syncthreads();
-  if (tid < L.N) {   // each cell's two rows are written by one thread
-    const int k = tid, i = k / L.My, j = k % L.My;
-    for (int b = 0; b < 9; ++b) {
-      const int di = (b % 3) - 1, dj = 1 - (b / 3);
-      const int kn = wrap(i + di, L.Mx) * L.My + wrap(j + dj, L.My);
-      const float4 v = L.A[b * L.N + k];
-      S.a[2 * k + 0][2 * kn + 0] += (double)v.x;
-      S.a[2 * k + 0][2 * kn + 1] += (double)v.y;
-      S.a[2 * k + 1][2 * kn + 0] += (double)v.z;
-      S.a[2 * k + 1][2 * kn + 1] += (double)v.w;
+__device__ __forceinline__ void coarse_invert_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+// threads 0 .. CI_THREADS - 1 of a block
+__device__ __noinline__ void coarse_invert(int Mx, int My, const float4 *A, CoarseInvertSmem &S, double *invT_out,
+                                           int *singular) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = Mx * My, n = 2 * N;
+  if (warp == 0) {
+    for (int c = 0; c < 33; ++c) S.a[lane][c] = 0.0;
+    if (lane < n) {
+      const int k = lane >> 1, i = k / My, j = k - i * My;
+      float2 v[9];
+      int kn[9];
+#pragma unroll
+      for (int b = 0; b < 9; ++b) {
+        const float4 t = A[b * N + k];
+        v[b] = (lane & 1) ? make_float2(t.z, t.w) : make_float2(t.x, t.y);
+        kn[b] = wrap(i + (b % 3) - 1, Mx) * My + wrap(j + 1 - (b / 3), My);
+      }
+      for (int b = 0; b < 9; ++b) {
+        S.a[lane][2 * kn[b] + 0] += (double)v[b].x;
+        S.a[lane][2 * kn[b] + 1] += (double)v[b].y;
+      }
     }
   }
-  __syncthreads();
-  for (int col = 0; col < n; ++col) {
-    // warp 0: the pivot (the largest |a[r][col]|, r >= col, lowest row on ties), the row
-    // interchange, the scaled pivot row and the copy of the multipliers, ordered by __syncwarp
-    if (tid < 32) {
-      const int t = tid;
-      double best = -1.0;
-      int bi = col;
-      if (col + t < n) {
-        best = fabs(S.a[col + t][col]);
-        bi = col + t;
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
+  coarse_invert_sync();
+  double row[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) row[q] = S.a[lane][8 * warp + q];
+  int pos = lane;
+#pragma unroll 1
+  for (int col0 = 0; col0 < n; col0 += 8) {
+#pragma unroll
+    for (int cc = 0; cc < 8; ++cc) {
+      const int col = col0 + cc;
+      if (col >= n) break;
+      const bool mine = 8 * warp == col0;
+      CoarseInvertSmem::Step &T = S.step[cc & 1];
+      if (mine) {
+        const double pv = row[cc], pinv = pv != 0.0 ? 1.0 / pv : 0.0;
+        const bool open = pos >= col && pos < n;
+        const unsigned long long key = (unsigned long long)__double_as_longlong(fabs(pv));
+        const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+        const unsigned top = __reduce_max_sync(ALL, open ? hi : 0u);
+        bool best = open && hi == top;
+        if (__popc(__ballot_sync(ALL, best)) != 1) {   // the same exponent and leading 20 bits
+          const unsigned low = __reduce_max_sync(ALL, best ? lo : 0u);
+          best = best && lo == low;
+          best = best && pos == (int)__reduce_min_sync(ALL, best ? (unsigned)pos : 64u);
+        }
+        T.f[lane] = pv;
+        if (best) {
+          T.pinv = pinv;
+          T.lane = lane;
+          T.pos = pos;
+          if (!(fabs(pv) > 0.0)) *singular = 1;
         }
       }
-      if (t == 0) {
-        S.perm[col] = bi;
-        if (!(best > 0.0)) *singular = 1;
-      }
-      const int p = bi;
-      if (p != col && t < n) {   // lane t swaps column t of the two rows
-        const double tmp = S.a[col][t];
-        S.a[col][t] = S.a[p][t];
-        S.a[p][t] = tmp;
+      coarse_invert_sync();
+      const double f = T.f[lane], pinv = T.pinv;
+      const bool pivot = lane == T.lane;
+      const int p = T.pos;
+      if (pivot) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) row[q] *= pinv;
+        if (mine) row[cc] = pinv;   // 1 * pinv
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S.prow[warp][q] = make_double2(row[2 * q], row[2 * q + 1]);
       }
       __syncwarp();
-      const double pv = S.a[col][col];
-      const double pinv = pv != 0.0 ? 1.0 / pv : 0.0;
-      __syncwarp();
-      // pivot row: a[col][col] <- 1, then scaled by 1 / pivot (so it holds 1 / pivot); the
-      // multipliers of the other rows are copied before any of them changes
-      if (t < n) {
-        S.a[col][t] = (t == col ? 1.0 : S.a[col][t]) * pinv;
-        S.fcol[t] = S.a[t][col];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double2 x = S.prow[warp][q];
+        const double a = 2 * q == cc && mine ? -f * x.x : fma(-f, x.x, row[2 * q]);
+        const double b = 2 * q + 1 == cc && mine ? -f * x.y : fma(-f, x.y, row[2 * q + 1]);
+        if (!pivot) {
+          row[2 * q] = a;
+          row[2 * q + 1] = b;
+        }
       }
+      pos = pivot ? col : (pos == col ? p : pos);
+      __syncwarp();   // the pivot row has been read by the warp
     }
-    __syncthreads();
-    // other rows: a[r][q] -= a[r][col] a[col][q]; a[r][col] <- -a[r][col] / pivot (element e
-    // is (r, q) = (e / 32, e % 32), those outside n x n idle)
-    for (int e = tid; e < 32 * 32; e += nth) {
-      const int r = e >> 5, q = e & 31;
-      if (r == col || r >= n || q >= n) continue;
-      const double f = S.fcol[r];
-      if (q != col) S.a[r][q] -= f * S.a[col][q];
-      else S.a[r][col] = -f * S.a[col][col];
-    }
-    __syncthreads();
   }
-  // undo the row interchanges as column interchanges, in reverse order
-  for (int col = n - 1; col >= 0; --col) {
-    const int p = S.perm[col];
-    if (p != col && tid < n) {
-      const double tmp = S.a[tid][col];
-      S.a[tid][col] = S.a[tid][p];
-      S.a[tid][p] = tmp;
-    }
-    __syncthreads();
-  }
-  for (int q = tid; q < n * n; q += nth) {
-    const int c = q / n, r = q - c * n;
-    invT_out[q] = S.a[r][c];   // invT[c][r] = inverse[r][c]
+  // the interchanges undone: column pos of the elimination is column lane of the inverse
+  if (warp == 0) S.own[pos] = lane;
+  coarse_invert_sync();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int c = 8 * warp + q;
+    if (c < n && pos < n) invT_out[S.own[c] * n + pos] = row[q];   // invT[c][r] = inverse[r][c]
   }
 }
 
-// the coarsest inverse, after the last level build (CI_THREADS threads: one element of the
-// 32 x 32 elimination each)
-constexpr int CI_THREADS = 1024;
-__global__ void __launch_bounds__(CI_THREADS) k_mg_coarse_invert(LevelView L, double *invT_out, int *singular) {
-  __shared__ CoarseInvertSmem S;
-  coarse_invert_block(L, S, invT_out, singular);
-}
-
-// The small levels' Galerkin operators (levels first .. nlev - 1, each from the level above it,
-// all of <= MG_CTA_CELLS cells) and the coarsest inverse in one launch on one thread-block
-// cluster: one cluster barrier (release / acquire at cluster scope) between levels; the
-// coarsest inverse follows as its own launch.  The arithmetic of every cell is k_mg_build's.
-__global__ void __cluster_dims__(SMALL_CLUSTER, 1, 1) __launch_bounds__(NTm)
-    k_mg_build_small(const LevelView *__restrict__ lev, int first, int nlev) {
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = cluster.block_rank() * NTm + threadIdx.x, nthr = SMALL_CLUSTER * NTm;
+// The levels of at most MG_TAIL_CELLS cells and the coarsest inverse, by one block: a level's
+// operator goes to global memory for the cycle and to shared memory for the level below it.
+// Levels first .. nlev - 1; from 51 x 51 cells down, a cluster of eight blocks with a barrier a
+// level took 17 us and the inverse 29 us after it; now 18 us together.
+constexpr int MG_TAIL_CELLS = 128, TAIL_THREADS = 4 * MG_TAIL_CELLS;
+constexpr int TAIL_SMEM = 2 * 9 * MG_TAIL_CELLS * (int)sizeof(float4) + (int)sizeof(CoarseInvertSmem);
+__global__ void __launch_bounds__(TAIL_THREADS) k_mg_build_tail(const LevelView *lev, int first, int nlev,
+                                                                double *invT_out, int *singular) {
+  extern __shared__ __align__(16) char tail_sm[];
+  float4 *const ops = reinterpret_cast<float4 *>(tail_sm);
+  CoarseInvertSmem &S = *reinterpret_cast<CoarseInvertSmem *>(ops + 2 * 9 * MG_TAIL_CELLS);
+  const LevelView above = lev[first - 1];
+  GalerkinView F{above.Mx, above.My, above.N, above.ax, above.ay, above.A};
+  pdl_wait();
+  pdl_release();
+  F.A = after_wait(F.A);
   for (int c = first; c < nlev; ++c) {
-    const LevelView F = lev[c - 1], C = lev[c];
-    for (int kc = rank; kc < C.N; kc += nthr) {
-      const int I = kc / C.My, J = kc - I * C.My;
-      galerkin_cell(F, C.Mx, C.My, I, J, const_cast<float4 *>(C.A), const_cast<float4 *>(C.dinv));
-    }
-    cluster.sync();
+    const LevelView C = lev[c];
+    float4 *const copy = ops + ((c - first) & 1) * 9 * MG_TAIL_CELLS;
+    for (int q = threadIdx.x; q < 4 * C.N; q += TAIL_THREADS)
+      galerkin_entry(F, C.Mx, C.My, q >> 2, q & 3, const_cast<float4 *>(C.A), const_cast<float4 *>(C.dinv), copy);
+    __syncthreads();
+    F = GalerkinView{C.Mx, C.My, C.N, C.ax, C.ay, copy};
   }
+  if (threadIdx.x < CI_THREADS) coarse_invert(F.Mx, F.My, F.A, S, invT_out, singular);
 }
 
 // ---------------------------------------------------------------------------
@@ -1466,6 +1517,7 @@ int mg_allocate(MGHierarchy &H, int fine_cells) {
     if (cudaMalloc(&H.views, sizeof(LevelView) * MG_MAX_LEVELS) != cudaSuccess) return 1;
     if (cudaMemcpy(H.views, v, sizeof(LevelView) * H.nlev, cudaMemcpyHostToDevice) != cudaSuccess) return 1;
   }
+  if (raise_dynamic_smem((const void *)k_mg_build_tail, TAIL_SMEM) != 0) return 1;
   if (raise_dynamic_smem((const void *)k_mg_small_cycle, H.small_smem) != 0) return 1;
   if (H.resident && raise_dynamic_smem(H.res_plan.wide ? (const void *)k_mg_small_resident<true>
                                                        : (const void *)k_mg_small_resident<false>,
@@ -1556,21 +1608,17 @@ void mg_setup_coarse(const Launch &Lc, const GridDev &g, const Fields &f, MGHier
     k_mg_build1<<<blocks_for(Lc, tm.tiles), NTm, 0, Lc.stream>>>(g, s, f.flags, f.nuH, f.beta, H.fine_ax,
                                                                      H.fine_ay, C.Mx, C.My, tm, C.A, C.dinv);
   }
-  // levels 1 .. cfirst - 1 by tiled passes; cfirst .. nlev - 1 (the cluster-cycled small
-  // levels) by one cluster launch; then the coarsest inverse
-  const int cfirst = H.nlev > 1 ? std::max(1, H.small_first) : H.nlev;
-  for (int l = 0; l + 1 < cfirst; ++l) {
-    const MGLevel &F = H.lev[l], &C = H.lev[l + 1];
-    const TileM tm = tiles_of(C.Mx, C.My);
-    k_mg_build<<<blocks_for(Lc, tm.tiles), NTm, 0, Lc.stream>>>(view(F), C.Mx, C.My, tm, C.A, C.dinv);
+  // levels of more than MG_TAIL_CELLS cells by a launch each, the rest and the coarsest inverse by
+  // one block
+  int l = 1;
+  for (; l < H.nlev && H.lev[l].N > MG_TAIL_CELLS; ++l) {
+    const MGLevel &F = H.lev[l - 1], &C = H.lev[l];
+    launch_pdl(Lc, k_mg_build, std::min((4 * C.N + NTm - 1) / NTm, 8 * Lc.max_blocks), NTm, 0,
+               GalerkinView{F.Mx, F.My, F.N, F.ax, F.ay, F.A}, C.Mx, C.My, C.A, C.dinv);
   }
-  if (cfirst < H.nlev) {
-    k_mg_build_small<<<SMALL_CLUSTER, NTm, 0, Lc.stream>>>(reinterpret_cast<const LevelView *>(H.views), cfirst,
-                                                             H.nlev);
-    Lc.tick();
-  }
-  k_mg_coarse_invert<<<1, CI_THREADS, 0, Lc.stream>>>(view(H.lev[H.nlev - 1]), H.cinv, H.singular);
-  Lc.tick(cfirst + 1);
+  launch_pdl(Lc, k_mg_build_tail, 1, TAIL_THREADS, TAIL_SMEM, reinterpret_cast<const LevelView *>(H.views), l, H.nlev,
+             H.cinv, H.singular);
+  Lc.tick(l + 1);
 }
 
 template <class F22, class F21, class F12, class F11>
