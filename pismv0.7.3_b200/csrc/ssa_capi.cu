@@ -70,7 +70,7 @@ struct pism_gpu_ssa {
     double reg = 0.0, underrelax = 0.0;
     Fields key{};
     bool mixed = false;
-    long long pre = 0, per_picard = 0, per_refine = 0, per_inner = 0, per_go = 0, per_test = 0, per_rebuild = 0;
+    long long pre = 0, per_picard = 0, per_refine = 0, per_inner = 0, per_rebuild = 0;
     bool failed = false;
   } sgraph;
   PState *pstate = nullptr;
@@ -392,27 +392,32 @@ int run_until_done(pism_gpu_ssa *h, int kind, const void *x, KState *st, int chu
   return PISM_GPU_SSA_OK;
 }
 
-// Inside an active capture on h->L.stream: add a conditional node (WHILE or IF) after the
-// capture's current dependencies.  `set(cond)` launches the kernel that gives the node its
-// value, once before the node and, for a WHILE node, again at the end of each pass of the
-// body (unless body_sets: the body's last kernel does); `body(cond)` launches the body on
-// h->L.stream (itself capturing into the node's body graph, so bodies nest).  *body_kernels gets the kernels of one pass, nested bodies
-// included.  The capture continues after the node.
-template <class SET, class BODY>
-bool add_conditional(pism_gpu_ssa *h, cudaGraphConditionalNodeType type, const SET &set, const BODY &body,
-                     long long *body_kernels, bool body_sets = false) {
+// Inside an active capture on h->L.stream: the handle of a conditional node added later to the
+// graph being captured, for the kernels before the node that give it its value.
+bool new_condition(pism_gpu_ssa *h, cudaGraphConditionalHandle *cond) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaGraph_t cg = nullptr;
+  const cudaGraphNode_t *deps = nullptr;
+  size_t nd = 0;
+  return cudaStreamGetCaptureInfo(h->L.stream, &cs, nullptr, &cg, &deps, &nd) == cudaSuccess &&
+         cs == cudaStreamCaptureStatusActive && cudaGraphConditionalHandleCreate(cond, cg, 0, 0) == cudaSuccess;
+}
+
+// Add the conditional node (WHILE or IF) after the capture's current dependencies; `body()`
+// launches its body on h->L.stream (itself capturing into the node's body graph, so bodies nest),
+// for a WHILE node with the kernel that sets the handle again.  *body_kernels gets the kernels of
+// one pass, nested bodies included.  The capture continues after the node.
+template <class BODY>
+bool add_conditional(pism_gpu_ssa *h, cudaGraphConditionalNodeType type, cudaGraphConditionalHandle cond,
+                     const BODY &body, long long *body_kernels) {
   const cudaStream_t s = h->L.stream;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaGraph_t cg = nullptr;
   const cudaGraphNode_t *deps = nullptr;
   size_t nd = 0;
+  if (cudaGetLastError() != cudaSuccess) return false;
   if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &cg, &deps, &nd) != cudaSuccess || cs != cudaStreamCaptureStatusActive)
     return false;
-  cudaGraphConditionalHandle cond{};
-  if (cudaGraphConditionalHandleCreate(&cond, cg, 0, 0) != cudaSuccess) return false;
-  set(cond);
-  if (cudaGetLastError() != cudaSuccess) return false;
-  if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &cg, &deps, &nd) != cudaSuccess) return false;
   cudaGraphNodeParams p{};
   p.type = cudaGraphNodeTypeConditional;
   p.conditional.handle = cond;
@@ -427,8 +432,7 @@ bool add_conditional(pism_gpu_ssa *h, cudaGraphConditionalNodeType type, const S
   if (ok) {
     const long long b0 = h->stats.kernel_launches;
     h->L.stream = bs;
-    ok = body(cond);
-    if (type == cudaGraphCondTypeWhile && !body_sets) set(cond);
+    ok = body();
     h->L.stream = s;
     *body_kernels = h->stats.kernel_launches - b0;
     ok = cudaGetLastError() == cudaSuccess && ok;
@@ -442,9 +446,12 @@ bool add_conditional(pism_gpu_ssa *h, cudaGraphConditionalNodeType type, const S
 // SSAFD::picard_manager with its linear solves, nu*H updates and stopping test in one graph
 // launch and one read-back: a WHILE node over Picard iterations (its decisions taken on the
 // device by ssa_control.cu), inside it the linear solve — FP64 BiCGStab as a WHILE node of
-// four iterations per pass, or the mixed-precision refinement as a WHILE node over
-// refinement steps around the inner FP32 BiCGStab's WHILE node and an IF node for the
-// correction — and an IF node for the nu*H update and Picard test after a successful solve.
+// four iterations per pass or one cooperative kernel, or the mixed-precision refinement as a
+// WHILE node over refinement steps around the inner FP32 BiCGStab's WHILE node.  A node costs
+// about 5 us to enter and as much again after its body, a kernel that does nothing 1.5 us: so the
+// correction and the nu*H update are kernels that return at once where they do not apply, a
+// node's value is set by the kernel that takes the decision, and a refinement ends without a
+// pass that finds nothing to do.
 // Used for BiCGStab without a fallback preconditioner and verbosity <= 2; everything else
 // (and a stream that cannot be captured) takes the host loop.
 bool solve_graph_eligible(const pism_gpu_ssa *h) {
@@ -479,7 +486,8 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
                  c.ksp_rtol_adaptive ? 1 : 0, c.max_iterations_ssafd, c.mg_rebuild_rtol};
   PState *P = h->pstate;
   const long long t0 = h->stats.kernel_launches;
-  long long inc_picard = 0, inc_refine = 0, inc_inner = 0, inc_go = 0, inc_test = 0, inc_rebuild = 0, pre = 0;
+  long long inc_picard = 0, inc_refine = 0, inc_inner = 0, inc_rebuild = 0, pre = 0;
+  const bool resident = !mg && !line && bicg_resident_fits(h->L, g, h->kex);
   const bool lagged = mg && c.mg_rebuild_rtol > 0.0;
   // a second capture stream for the per-Picard set-up that the coarse-level builds do not read
   struct SideBranch {
@@ -504,22 +512,23 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
     return PISM_GPU_SSA_OK;
   }
   launch_nuH(h->L, g, c, f, reg, 1.0, false, h->norm_dev);
-  launch_picard_start(h->L, P);
-  auto not_done = [&](const int *flag) {
-    return [&h, flag](cudaGraphConditionalHandle cond) { launch_flag_condition(h->L, cond, flag, true); };
-  };
+  cudaGraphConditionalHandle picard_loop{};
+  bool ok = new_condition(h, &picard_loop);
+  launch_picard_start(h->L, P, picard_loop);
   const long long before_loop = h->stats.kernel_launches;
-  bool ok = add_conditional(h, cudaGraphCondTypeWhile, not_done(&P->done), [&](cudaGraphConditionalHandle) {
+  ok = ok && add_conditional(h, cudaGraphCondTypeWhile, picard_loop, [&] {
     bool inner_ok = true, rebuild_ok = true;
-    launch_picard_begin(h->L, P, pc, h->zd_dev);
+    cudaGraphConditionalHandle refine_loop{};
+    if (mixed && !new_condition(h, &refine_loop)) return false;
+    launch_picard_begin(h->L, P, pc, h->zd_dev, refine_loop, mixed ? nullptr : h->K.st, c.ksp_max_it);
     bool residual_queued = false;
     if (split) {
       // The set-up in two branches of the graph. On the loop's stream: the coarse-level
       // Galerkin builds and the coarsest inverse, which read nu*H, beta and the masks only.
       // Beside them: the FP64 diagonal blocks, the FP32 fine-level copies and the first
-      // refinement residual. The small levels' builds run on one cluster and the inverse on
-      // one block, so most SMs are free for the second branch. Same kernels, same inputs:
-      // the results are those of the serial order.
+      // refinement residual. The small levels' builds and the inverse run on one block, so
+      // most SMs are free for the second branch. Same kernels, same inputs: the results are
+      // those of the serial order.
       cudaEventRecord(side.fork, h->L.stream);
       cudaStreamWaitEvent(side.stream, side.fork, 0);
       Launch Ls = h->L;
@@ -534,14 +543,13 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
     } else if (lagged) {
       launch_diag_setup(h->L, g, f, h->K.dinv, h->zd_dev);
       mg_setup_fine(h->L, g, f, h->K.dinv, h->mg);
-      rebuild_ok = add_conditional(
-          h, cudaGraphCondTypeIf,
-          [&](cudaGraphConditionalHandle cond) { launch_flag_condition(h->L, cond, &P->rebuild, false); },
-          [&](cudaGraphConditionalHandle) {
-            mg_setup_coarse(h->L, g, f, h->mg);
-            return true;
-          },
-          &inc_rebuild);
+      cudaGraphConditionalHandle rebuild{};
+      if (!new_condition(h, &rebuild)) return false;
+      launch_flag_condition(h->L, rebuild, &P->rebuild);
+      rebuild_ok = add_conditional(h, cudaGraphCondTypeIf, rebuild, [&] {
+        mg_setup_coarse(h->L, g, f, h->mg);
+        return true;
+      }, &inc_rebuild);
     } else {
       launch_diag_setup(h->L, g, f, h->K.dinv, h->zd_dev);
       if (mg) mg_setup(h->L, g, f, h->K.dinv, h->mg);
@@ -549,50 +557,39 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
     if (line) line_setup(h->L, g, f, h->K.dinv, h->line);
     if (mixed) {
       if (!residual_queued) launch_residual32(h->L, g, f, h->rhs, h->vel, h->K32.rhs, h->res_dev);
-      inner_ok = add_conditional(h, cudaGraphCondTypeWhile, not_done(&P->refine_done), [&](cudaGraphConditionalHandle) {
-        launch_mixed_init_dev(h->L, N, h->K32, h->res_dev, &P->rtol, c.mixed_inner_rtol, c.ksp_max_it);
-        bool ok2 = add_conditional(
-            h, cudaGraphCondTypeWhile,
-            [&](cudaGraphConditionalHandle cond) { launch_loop_condition(h->L, cond, h->K32.st); },
-            [&](cudaGraphConditionalHandle cond) {
-              launch_mixed_iteration(h->L, g, f, *mg, h->K32, cond);
-              return true;
-            },
-            &inc_inner, true);
+      // a refinement step; its last kernel ends the loop where the next inner solve would have
+      // nothing to do
+      inner_ok = add_conditional(h, cudaGraphCondTypeWhile, refine_loop, [&] {
+        cudaGraphConditionalHandle inner_loop{};
+        if (!new_condition(h, &inner_loop)) return false;
+        launch_mixed_init_dev(h->L, N, h->K32, h->res_dev, &P->rtol, c.mixed_inner_rtol, c.ksp_max_it, inner_loop);
+        const bool ok2 = add_conditional(h, cudaGraphCondTypeWhile, inner_loop, [&] {
+          launch_mixed_iteration(h->L, g, f, *mg, h->K32, inner_loop);
+          return true;
+        }, &inc_inner);
         launch_refine_end(h->L, P, h->K32.st, 60);
-        ok2 = ok2 && add_conditional(
-                         h, cudaGraphCondTypeIf,
-                         [&](cudaGraphConditionalHandle cond) { launch_flag_condition(h->L, cond, &P->go, false); },
-                         [&](cudaGraphConditionalHandle) {
-                           launch_axpy32(h->L, N, h->K32.d, h->vel);
-                           launch_residual32(h->L, g, f, h->rhs, h->vel, h->K32.rhs, h->res_dev);
-                           return true;
-                         },
-                         &inc_go);
+        launch_axpy32(h->L, N, h->K32.d, h->vel, P);
+        launch_residual32(h->L, g, f, h->rhs, h->vel, h->K32.rhs, h->res_dev, RefineStep{P, 60, refine_loop});
         return ok2;
       }, &inc_refine);
     } else {
-      launch_ksp_begin(h->L, h->K.st, P, c.ksp_max_it);
-      launch_bicg_init(h->L, g, f, h->K, h->rhs, h->vel);
-      inner_ok = add_conditional(
-          h, cudaGraphCondTypeWhile,
-          [&](cudaGraphConditionalHandle cond) { launch_loop_condition(h->L, cond, h->K.st); },
-          [&](cudaGraphConditionalHandle cond) {
-            for (int q = 0; q < 4; ++q) launch_bicg_iteration(h->L, g, f, h->K, h->vel, mg, line, cond);
-            return true;
-          },
-          &inc_inner, true);
-      launch_ksp_end(h->L, P, h->K.st, 4);
+      cudaGraphConditionalHandle inner_loop{};
+      if (!resident && !new_condition(h, &inner_loop)) return false;
+      launch_bicg_init(h->L, g, f, h->K, h->rhs, h->vel, inner_loop);
+      if (resident)
+        inner_ok = launch_bicg_resident(h->L, g, f, h->K, h->vel, h->kex);
+      else
+        inner_ok = add_conditional(h, cudaGraphCondTypeWhile, inner_loop, [&] {
+          for (int q = 0; q < 4; ++q) launch_bicg_iteration(h->L, g, f, h->K, h->vel, mg, line, inner_loop);
+          return true;
+        }, &inc_inner);
     }
-    launch_picard_after_solve(h->L, P, h->zd_dev);
-    inner_ok = inner_ok && add_conditional(h, cudaGraphCondTypeIf, not_done(&P->done), [&](cudaGraphConditionalHandle) {
-      launch_nuH(h->L, g, c, f, reg, underrelax, true, h->norm_dev);
-      launch_picard_test(h->L, P, h->norm_dev, pc);
-      return true;
-    }, &inc_test);
+    launch_picard_after_solve(h->L, P, h->zd_dev, mixed ? nullptr : h->K.st, 4);
+    launch_nuH(h->L, g, c, f, reg, underrelax, true, h->norm_dev, P);
+    launch_picard_test(h->L, P, h->norm_dev, pc, picard_loop);
     return inner_ok && rebuild_ok;
   }, &inc_picard);
-  pre = before_loop - t0 + 1;   // + the WHILE node's first condition kernel
+  pre = before_loop - t0;
   cudaGraph_t out = nullptr;
   const bool ended = cudaStreamEndCapture(h->stream, &out) == cudaSuccess;
   ok = ok && ended && out != nullptr;
@@ -611,11 +608,9 @@ int build_solve_graph(pism_gpu_ssa *h, double reg, double underrelax, bool *buil
   S.mixed = mixed;
   S.pre = pre;
   S.per_inner = inc_inner;
-  S.per_go = inc_go;
-  S.per_test = inc_test;
   S.per_rebuild = inc_rebuild;
-  S.per_refine = mixed ? inc_refine - inc_inner - inc_go : 0;
-  S.per_picard = inc_picard - (mixed ? inc_refine : inc_inner) - inc_test - inc_rebuild;
+  S.per_refine = mixed ? inc_refine - inc_inner : 0;
+  S.per_picard = inc_picard - (mixed ? inc_refine : inc_inner) - inc_rebuild;
   *built = true;
   return PISM_GPU_SSA_OK;
 }
@@ -650,8 +645,7 @@ int solve_graph_collect(pism_gpu_ssa *h, double reg) {
   const auto &S = h->sgraph;
   const PState &P = *h->pstate_host;
   h->stats.kernel_launches += S.pre + P.passes * S.per_picard + P.refine_passes * S.per_refine +
-                              P.inner_passes * S.per_inner + P.go_count * S.per_go + P.k * S.per_test +
-                              P.rebuilds * S.per_rebuild;
+                              P.inner_passes * S.per_inner + P.rebuilds * S.per_rebuild;
   if (active_mg(h)) h->stats.mg_rebuilds += P.rebuilds;
   h->stats.ksp_iterations += P.ksp_total;
   h->stats.refinement_steps += P.refine_steps;

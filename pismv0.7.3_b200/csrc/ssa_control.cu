@@ -10,70 +10,80 @@
 // apply them to the state in device memory.
 #include <climits>
 
-#include "ssa_internal.h"
+#include "ssa_pdl.cuh"
 
 namespace pism_gpu {
 namespace {
 
-__global__ void k_picard_start(PState *P) { picard_start(*P); }
-
-__global__ void k_picard_begin(PState *P, PicardConst c, int *zero_diag_cell) {
-  *zero_diag_cell = INT_MAX;
-  picard_begin(*P, c);
+// picard_loop: the WHILE node over Picard passes, entered
+__global__ void k_picard_start(PState *P, cudaGraphConditionalHandle picard_loop) {
+  picard_start(*P);
+  cudaGraphSetConditional(picard_loop, 1u);
 }
 
-__global__ void k_ksp_begin(KState *st, const PState *P, int maxit) { ksp_begin(*st, *P, maxit); }
+// mixed precision: refine_loop (the WHILE node over refinement steps) is entered; FP64: st is
+// made ready for the solve
+__global__ void k_picard_begin(PState *P, PicardConst c, int *zero_diag_cell, cudaGraphConditionalHandle refine_loop,
+                               KState *st, int maxit) {
+  *zero_diag_cell = INT_MAX;
+  picard_begin(*P, c);
+  if (st) ksp_begin(*st, *P, maxit);
+  else cudaGraphSetConditional(refine_loop, 1u);
+}
 
-__global__ void k_ksp_end(PState *P, const KState *st, int body_iters) { ksp_end(*P, *st, body_iters); }
+__global__ void k_refine_end(PState *P, const KState *st, int max_refine) {
+  pdl_release();
+  refine_end(*P, *st, max_refine);
+}
 
-__global__ void k_refine_end(PState *P, const KState *st, int max_refine) { refine_end(*P, *st, max_refine); }
-
-__global__ void k_picard_after_solve(PState *P, const int *zero_diag_cell) {
+// st: the FP64 solve's state (body_iters iterations a pass of its loop), else null
+__global__ void k_picard_after_solve(PState *P, const int *zero_diag_cell, const KState *st, int body_iters) {
+  pdl_release();
+  if (st) ksp_end(*P, *st, body_iters);
   picard_after_solve(*P, *zero_diag_cell);
 }
 
-__global__ void k_picard_test(PState *P, const double *norm2, PicardConst c) {
-  picard_test(*P, norm2[0], norm2[1], c);
+// after the nu*H update (neither does anything once the solve failed); picard_loop goes on or ends
+__global__ void k_picard_test(PState *P_, const double *norm2_, PicardConst c, cudaGraphConditionalHandle picard_loop) {
+  pdl_wait();
+  PState *P = after_wait(P_);
+  const double *norm2 = after_wait(norm2_);
+  if (!P->done) picard_test(*P, norm2[0], norm2[1], c);
+  cudaGraphSetConditional(picard_loop, P->done ? 0u : 1u);
 }
 
-__global__ void k_flag_condition(cudaGraphConditionalHandle cond, const int *flag, int negate) {
-  const bool on = (*flag != 0) != (negate != 0);
-  cudaGraphSetConditional(cond, on ? 1u : 0u);
+__global__ void k_flag_condition(cudaGraphConditionalHandle cond, const int *flag) {
+  cudaGraphSetConditional(cond, *flag != 0 ? 1u : 0u);
 }
 
 }  // namespace
 
-void launch_picard_start(const Launch &L, PState *P) {
+void launch_picard_start(const Launch &L, PState *P, cudaGraphConditionalHandle picard_loop) {
   L.tick();
-  k_picard_start<<<1, 1, 0, L.stream>>>(P);
+  k_picard_start<<<1, 1, 0, L.stream>>>(P, picard_loop);
 }
-void launch_picard_begin(const Launch &L, PState *P, const PicardConst &c, int *zero_diag_cell) {
+void launch_picard_begin(const Launch &L, PState *P, const PicardConst &c, int *zero_diag_cell,
+                         cudaGraphConditionalHandle refine_loop, KState *st, int maxit) {
   L.tick();
-  k_picard_begin<<<1, 1, 0, L.stream>>>(P, c, zero_diag_cell);
-}
-void launch_ksp_begin(const Launch &L, KState *st, const PState *P, int maxit) {
-  L.tick();
-  k_ksp_begin<<<1, 1, 0, L.stream>>>(st, P, maxit);
-}
-void launch_ksp_end(const Launch &L, PState *P, const KState *st, int body_iters) {
-  L.tick();
-  k_ksp_end<<<1, 1, 0, L.stream>>>(P, st, body_iters);
+  k_picard_begin<<<1, 1, 0, L.stream>>>(P, c, zero_diag_cell, refine_loop, st, maxit);
 }
 void launch_refine_end(const Launch &L, PState *P, const KState *st, int max_refine) {
   L.tick();
   k_refine_end<<<1, 1, 0, L.stream>>>(P, st, max_refine);
 }
-void launch_picard_after_solve(const Launch &L, PState *P, const int *zero_diag_cell) {
+void launch_picard_after_solve(const Launch &L, PState *P, const int *zero_diag_cell, const KState *st,
+                               int body_iters) {
   L.tick();
-  k_picard_after_solve<<<1, 1, 0, L.stream>>>(P, zero_diag_cell);
+  k_picard_after_solve<<<1, 1, 0, L.stream>>>(P, zero_diag_cell, st, body_iters);
 }
-void launch_picard_test(const Launch &L, PState *P, const double *norm2, const PicardConst &c) {
+void launch_picard_test(const Launch &L, PState *P, const double *norm2, const PicardConst &c,
+                        cudaGraphConditionalHandle picard_loop) {
   L.tick();
-  k_picard_test<<<1, 1, 0, L.stream>>>(P, norm2, c);
+  launch_pdl(L, k_picard_test, 1, 1, 0, P, norm2, c, picard_loop);
 }
-void launch_flag_condition(const Launch &L, cudaGraphConditionalHandle cond, const int *flag, bool negate) {
+void launch_flag_condition(const Launch &L, cudaGraphConditionalHandle cond, const int *flag) {
   L.tick();
-  k_flag_condition<<<1, 1, 0, L.stream>>>(cond, flag, negate ? 1 : 0);
+  k_flag_condition<<<1, 1, 0, L.stream>>>(cond, flag);
 }
 
 }  // namespace pism_gpu

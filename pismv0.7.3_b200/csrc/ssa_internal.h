@@ -124,21 +124,24 @@ void launch_prepare(const Launch &L, const GridDev &g, const pism_gpu_ssa_config
                     const Fields &f);
 void launch_hardness(const Launch &L, const GridDev &g, const pism_gpu_ssa_config &c, const Fields &f, int Mz,
                      const double *z);
+// (P: inside the whole-solve graph, nothing once P->done)
 void launch_nuH(const Launch &L, const GridDev &g, const pism_gpu_ssa_config &c, const Fields &f, double reg,
-                double underrelax, bool with_norm, double *norm_out);
+                double underrelax, bool with_norm, double *norm_out, const PState *P = nullptr);
 void launch_apply(const Launch &L, const GridDev &g, const Fields &f, const double2 *x, double2 *y);
 void launch_diag_setup(const Launch &L, const GridDev &g, const Fields &f, double4 *dinv, int *zero_diag_cell);
+// (cond: the WHILE condition of a graph-resident loop, set by the solve's start and by an iteration's
+// last kernel; 0: none)
 void launch_bicg_init(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, const double2 *b,
-                      const double2 *x);
-// (cond: the WHILE condition of a graph-resident loop, set by the iteration's last kernel; 0: none)
+                      const double2 *x, cudaGraphConditionalHandle cond = 0);
 void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
                            const MGHierarchy *mg, const LinePC *line, cudaGraphConditionalHandle cond = 0);
 // the whole block-Jacobi solve after launch_bicg_init in one cooperative kernel where the grid
-// fits; false: nothing was launched
+// fits (bicg_resident_fits, which allocates the exchange words); false: nothing was launched
 struct KrylovExchange {
   unsigned long long *w = nullptr;   // the exchange words, allocated on first use
   int capacity = 0;                  // blocks of the kernel that the device holds at once
 };
+bool bicg_resident_fits(const Launch &L, const GridDev &g, KrylovExchange &E);
 bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
                           KrylovExchange &E);
 // FGMRES: r0 = b - A x into V0 (init) / after a restart; one Arnoldi step j; the end of a cycle
@@ -205,21 +208,25 @@ void launch_pc_apply(const Launch &L, const GridDev &g, const Fields &f, const d
 
 // ---- device-side control of the Picard loop (ssa_control.cu; state and decisions in
 // ssa_state.h) ----
-void launch_picard_start(const Launch &L, PState *P);
-// a Picard pass begins: zero-diagonal marker reset, the pass's KSP tolerance
-void launch_picard_begin(const Launch &L, PState *P, const PicardConst &c, int *zero_diag_cell);
-// FP64 BiCGStab inside the graph: its state from the pass's tolerance; its outcome
-void launch_ksp_begin(const Launch &L, KState *st, const PState *P, int maxit);
-void launch_ksp_end(const Launch &L, PState *P, const KState *st, int body_iters);
+// The conditional nodes' values are set by these kernels and by those that end a solve or a step,
+// so that no kernel stands between a node and the decision it takes.
+void launch_picard_start(const Launch &L, PState *P, cudaGraphConditionalHandle picard_loop);
+// a Picard pass begins: zero-diagonal marker reset, the pass's KSP tolerance; st: the FP64
+// solve's state, made ready from the tolerance (null: mixed precision, refine_loop is entered)
+void launch_picard_begin(const Launch &L, PState *P, const PicardConst &c, int *zero_diag_cell,
+                         cudaGraphConditionalHandle refine_loop, KState *st, int maxit);
 // the end of one refinement step of the mixed-precision solve (go = apply its correction)
 void launch_refine_end(const Launch &L, PState *P, const KState *st, int max_refine);
-void launch_picard_after_solve(const Launch &L, PState *P, const int *zero_diag_cell);
-void launch_picard_test(const Launch &L, PState *P, const double *norm2, const PicardConst &c);
-// a conditional node's value from a flag: flag != 0 (or == 0 when negate)
-void launch_flag_condition(const Launch &L, cudaGraphConditionalHandle cond, const int *flag, bool negate);
+// st: the FP64 solve's outcome (null: the refinement's, in P)
+void launch_picard_after_solve(const Launch &L, PState *P, const int *zero_diag_cell, const KState *st,
+                               int body_iters);
+void launch_picard_test(const Launch &L, PState *P, const double *norm2, const PicardConst &c,
+                        cudaGraphConditionalHandle picard_loop);
+// a conditional node's value from a flag
+void launch_flag_condition(const Launch &L, cudaGraphConditionalHandle cond, const int *flag);
 // launch_mixed_init with the outer tolerance read from the device
 void launch_mixed_init_dev(const Launch &L, int N, const Krylov32 &K, const double *res2, const double *outer_rtol,
-                           double inner_min, int maxit);
+                           double inner_min, int maxit, cudaGraphConditionalHandle inner_loop);
 
 // the loop condition of a graph-resident Krylov loop: continue while st->done is 0
 void launch_loop_condition(const Launch &L, cudaGraphConditionalHandle cond, const KState *st);
@@ -231,10 +238,17 @@ void launch_mixed_init(const Launch &L, int N, const Krylov32 &K, const double *
 void launch_mixed_iteration(const Launch &L, const GridDev &g, const Fields &f, const MGHierarchy &H,
                             const Krylov32 &K, cudaGraphConditionalHandle cond = 0);
 // r32 = (float) (b - A x) with FP64 arithmetic; out2 = {||b - A x||^2, ||b||^2}
+// (step: the end of a refinement step inside the whole-solve graph: nothing but the loop's end
+// unless P->go, else the next step's decision with the residual)
+struct RefineStep {
+  PState *P = nullptr;
+  int max_refine = 0;
+  cudaGraphConditionalHandle refine_loop = 0;
+};
 void launch_residual32(const Launch &L, const GridDev &g, const Fields &f, const double2 *b, const double2 *x,
-                       float2 *r32, double *out2);
-// x += d
-void launch_axpy32(const Launch &L, int N, const float2 *d, double2 *x);
+                       float2 *r32, double *out2, const RefineStep &step = {});
+// x += d (P: only if P->go)
+void launch_axpy32(const Launch &L, int N, const float2 *d, double2 *x, const PState *P = nullptr);
 void launch_bfrict(const Launch &L, int N, const pism_gpu_ssa_config &c, const Fields &f, double *out);
 void launch_scale(const Launch &L, int n, double a, double *x);
 

@@ -297,7 +297,10 @@ __global__ void __launch_bounds__(NT) k_nuH(GridDev g, TileMap tm, pism_gpu_ssa_
                                             const double2 *__restrict__ hardness, const int8_t *__restrict__ mask,
                                             const double *__restrict__ tauc, const double *__restrict__ gl_mask,
                                             double2 *__restrict__ nuH, double *__restrict__ beta,
-                                            double *partials, unsigned *ticket, double *norm_out) {
+                                            double *partials, unsigned *ticket, double *norm_out, const PState *P) {
+  pdl_wait();
+  pdl_release();
+  if (P && after_wait(P)->done) return;
   const double dx = g.dx, dy = g.dy;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -529,7 +532,8 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_init(GridDev g, TileMap tm, Sten
                                                   const double2 *__restrict__ b, const double2 *__restrict__ x,
                                                   double2 *__restrict__ r, double2 *__restrict__ rhat,
                                                   double2 *__restrict__ p, double2 *__restrict__ v,
-                                                  double *partials, unsigned *ticket, KState *st) {
+                                                  double *partials, unsigned *ticket, KState *st,
+                                                  cudaGraphConditionalHandle cond) {
   double acc[2] = {0.0, 0.0};
   __shared__ HaloTile<double2> xT, nT;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -561,6 +565,7 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_init(GridDev g, TileMap tm, Sten
     const double tol = st->rtol * sqrt(tot[1]);
     st->done = (sqrt(tot[0]) <= tol || tot[1] == 0.0) ? 1 : 0;
     if (!isfinite(tot[0])) { st->done = 1; st->status = KSP_NAN; }
+    if (cond) cudaGraphSetConditional(cond, st->done ? 0u : 1u);
   }
 }
 
@@ -937,7 +942,14 @@ __global__ void __launch_bounds__(NT, 4) k_residual32(GridDev g, TileMap tm, Ste
                                                       const double2 *__restrict__ nuH, const double *__restrict__ beta,
                                                       const double2 *__restrict__ b, const double2 *__restrict__ x,
                                                       float2 *__restrict__ r32, double *partials, unsigned *ticket,
-                                                      double *out2) {
+                                                      double *out2, RefineStep step) {
+  pdl_wait();
+  x = after_wait(x);
+  PState *const P = step.P ? after_wait(step.P) : nullptr;
+  if (P && !P->go) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(step.refine_loop, 0u);
+    return;
+  }
   double acc[2] = {0.0, 0.0};
   __shared__ HaloTile<double2> xT, nT;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -956,10 +968,14 @@ __global__ void __launch_bounds__(NT, 4) k_residual32(GridDev g, TileMap tm, Ste
   if (grid_reduce<2>(acc, partials, ticket, tot)) {
     out2[0] = tot[0];
     out2[1] = tot[1];
+    if (P) cudaGraphSetConditional(step.refine_loop, refine_more(*P, tot[0], tot[1], step.max_refine) ? 1u : 0u);
   }
 }
 
-__global__ void k_axpy32(int N, const float2 *__restrict__ d, double2 *__restrict__ x) {
+__global__ void k_axpy32(int N, const float2 *__restrict__ d, double2 *__restrict__ x, const PState *P) {
+  pdl_wait();
+  pdl_release();
+  if (P && !after_wait(P)->go) return;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const float2 dk = d[k];
     double2 xk = x[k];
@@ -1019,7 +1035,7 @@ void launch_hardness(const Launch &L, const GridDev &g, const pism_gpu_ssa_confi
 }
 
 void launch_nuH(const Launch &L, const GridDev &g, const pism_gpu_ssa_config &c, const Fields &f, double reg,
-                double underrelax, bool with_norm, double *norm_out) {
+                double underrelax, bool with_norm, double *norm_out, const PState *P) {
   L.tick();
   TileMap tm = make_tiles(g);
   NuHParams p;
@@ -1035,12 +1051,13 @@ void launch_nuH(const Launch &L, const GridDev &g, const pism_gpu_ssa_config &c,
   p.B_area = g.dx * g.dy;
   p.with_norm = with_norm ? 1 : 0;
   int blocks = grid_for_tiles(L, tm.tiles);
-  if (c.calving_front_stress_boundary_condition)
-    k_nuH<true><<<blocks, NT, 0, L.stream>>>(g, tm, c, p, f.vel, f.H, f.hardness, f.mask, f.tauc, f.gl_mask, f.nuH,
-                                             f.beta, L.partials, L.ticket, norm_out);
+  const auto kernel = c.calving_front_stress_boundary_condition ? k_nuH<true> : k_nuH<false>;
+  if (P)
+    launch_pdl(L, kernel, blocks, NT, 0, g, tm, c, p, f.vel, f.H, f.hardness, f.mask, f.tauc, f.gl_mask, f.nuH, f.beta,
+               L.partials, L.ticket, norm_out, P);
   else
-    k_nuH<false><<<blocks, NT, 0, L.stream>>>(g, tm, c, p, f.vel, f.H, f.hardness, f.mask, f.tauc, f.gl_mask, f.nuH,
-                                              f.beta, L.partials, L.ticket, norm_out);
+    kernel<<<blocks, NT, 0, L.stream>>>(g, tm, c, p, f.vel, f.H, f.hardness, f.mask, f.tauc, f.gl_mask, f.nuH, f.beta,
+                                        L.partials, L.ticket, norm_out, nullptr);
 }
 
 void launch_apply(const Launch &L, const GridDev &g, const Fields &f, const double2 *x, double2 *y) {
@@ -1057,11 +1074,12 @@ void launch_diag_setup(const Launch &L, const GridDev &g, const Fields &f, doubl
 }
 
 void launch_bicg_init(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, const double2 *b,
-                      const double2 *x) {
+                      const double2 *x, cudaGraphConditionalHandle cond) {
   L.tick();
   TileMap tm = make_tiles(g);
   k_bicg_init<<<grid_for_tiles(L, tm.tiles), NT, 0, L.stream>>>(g, tm, stencil_const(g, f), f.flags, f.nuH, f.beta, b,
-                                                                x, K.r, K.rhat, K.p, K.v, L.partials, L.ticket, K.st);
+                                                                x, K.r, K.rhat, K.p, K.v, L.partials, L.ticket, K.st,
+                                                                cond);
 }
 
 void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
@@ -1084,19 +1102,30 @@ void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, c
   launch_pdl(L, k_bicg_x, bv, NT, 0, N, K.phat, K.shat, K.s, K.t, K.rhat, x, K.r, L.partials, L.ticket, K.st, cond);
 }
 
-bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
-                          KrylovExchange &E) {
-  const int N = g.Mx * g.My;
-  TileMap tm = make_tiles(g);
+static size_t bicg_exchange_words(const GridDev &g, int tiles) {
+  return 3 * ex_slot_words(tiles) + 3 * ex_node_words(g.Mx * g.My);
+}
+
+bool bicg_resident_fits(const Launch &L, const GridDev &g, KrylovExchange &E) {
+  const TileMap tm = make_tiles(g);
   if (!E.capacity) E.capacity = std::max(1, resident_blocks((const void *)k_bicg_resident, NT, 0));
   // one cell a thread in both orders: below L.max_blocks blocks the five kernels add alike
   if (tm.tiles > E.capacity || tm.tiles > L.max_blocks) return false;
-  const size_t slots = ex_slot_words(tm.tiles), nodes = ex_node_words(N), words = 3 * slots + 3 * nodes;
-  if (!E.w && cudaMalloc((void **)&E.w, sizeof(unsigned long long) * words) != cudaSuccess) {
+  if (!E.w &&
+      cudaMalloc((void **)&E.w, sizeof(unsigned long long) * bicg_exchange_words(g, tm.tiles)) != cudaSuccess) {
     E.w = nullptr;
     cudaGetLastError();
     return false;
   }
+  return true;
+}
+
+bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+                          KrylovExchange &E) {
+  const int N = g.Mx * g.My;
+  if (!bicg_resident_fits(L, g, E)) return false;
+  TileMap tm = make_tiles(g);
+  const size_t slots = ex_slot_words(tm.tiles), nodes = ex_node_words(N), words = bicg_exchange_words(g, tm.tiles);
   if (cudaMemsetAsync(E.w, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
   BicgResident ex;
   ex.a.w = E.w;
@@ -1123,16 +1152,22 @@ bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, co
 }
 
 void launch_residual32(const Launch &L, const GridDev &g, const Fields &f, const double2 *b, const double2 *x,
-                       float2 *r32, double *out2) {
+                       float2 *r32, double *out2, const RefineStep &step) {
   L.tick();
   TileMap tm = make_tiles(g);
-  k_residual32<<<grid_for_tiles(L, tm.tiles), NT, 0, L.stream>>>(g, tm, stencil_const(g, f), f.flags, f.nuH, f.beta, b,
-                                                                 x, r32, L.partials, L.ticket, out2);
+  const int blocks = grid_for_tiles(L, tm.tiles);
+  if (step.P)
+    launch_pdl(L, k_residual32, blocks, NT, 0, g, tm, stencil_const(g, f), f.flags, f.nuH, f.beta, b, x, r32, L.partials,
+               L.ticket, out2, step);
+  else
+    k_residual32<<<blocks, NT, 0, L.stream>>>(g, tm, stencil_const(g, f), f.flags, f.nuH, f.beta, b, x, r32, L.partials,
+                                              L.ticket, out2, step);
 }
 
-void launch_axpy32(const Launch &L, int N, const float2 *d, double2 *x) {
+void launch_axpy32(const Launch &L, int N, const float2 *d, double2 *x, const PState *P) {
   L.tick();
-  k_axpy32<<<grid_for(L, N), NT, 0, L.stream>>>(N, d, x);
+  if (P) launch_pdl(L, k_axpy32, grid_for(L, N), NT, 0, N, d, x, P);
+  else k_axpy32<<<grid_for(L, N), NT, 0, L.stream>>>(N, d, x, nullptr);
 }
 
 void launch_bfrict(const Launch &L, int N, const pism_gpu_ssa_config &c, const Fields &f, double *out) {

@@ -145,6 +145,21 @@ PISM_HD void refine_end(PState &P, const KState &st, int max_refine) {
   }
 }
 
+// After a refinement step's correction, with r2 = ||b - A x||^2 and b2 = ||b||^2: true when
+// another inner solve is due, else the refinement ends as the pass whose inner solve finds the
+// tolerance met would end it (that pass is not taken)
+PISM_HD bool refine_more(PState &P, double r2, double b2, int max_refine) {
+  const double rn = sqrt(r2), bn = sqrt(b2);
+  if (rn > P.rtol * bn && bn != 0.0) return true;
+  KState met{};
+  met.outer_r2 = r2;
+  met.outer_b2 = b2;
+  met.status = KSP_OUTER_DONE;
+  refine_end(P, met, max_refine);
+  P.refine_passes -= 1;
+  return false;
+}
+
 // picard_manager after a linear solve: the zero-diagonal and KSP checks
 PISM_HD void picard_after_solve(PState &P, int zero_diag_cell) {
   P.ksp_total += P.ksp_its;
