@@ -999,6 +999,15 @@ void bias_grad(pism_gpu_unet *h, cudaStream_t s, const bf16 *dy, int C, long lon
   k_reduce_few<<<1, 256, 0, s>>>(h->bias_part, ctas, C, db);
 }
 
+// the second stream and its events, from the first backward on: a network that only predicts has none
+bool side_stream(pism_gpu_unet *h) {
+  if (h->side_done) return true;
+  bool ok = h->side || cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t &e : h->ready)
+    ok = ok && (e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess);
+  return ok && cudaEventCreateWithFlags(&h->side_done, cudaEventDisableTiming) == cudaSuccess;
+}
+
 // Layer l backward: X input, dY given, masked by the layer's ReLU; dX (masked by xmask, its own
 // layer's output, where given) on the handle's stream, dW and db beside it on the second one: the
 // data gradients are the only chain.
@@ -1134,12 +1143,7 @@ int pism_gpu_unet_create(int device, int max_batch, int max_h, int max_w, pism_g
   A(&h->de2a, P(1) * 64);
   A(&h->dp1, P(1) * 32);
   A(&h->de1a, P(0) * 32);
-  if (rc == PISM_GPU_SSA_OK) {
-    bool ok = allow_kernels() && cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaEventCreateWithFlags(&h->side_done, cudaEventDisableTiming) == cudaSuccess;
-    for (cudaEvent_t &e : h->ready) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    if (!ok) rc = PISM_GPU_SSA_ECUDA;
-  }
+  if (rc == PISM_GPU_SSA_OK && !allow_kernels()) rc = PISM_GPU_SSA_ECUDA;
   if (rc != PISM_GPU_SSA_OK) {
     pism_gpu_unet_destroy(h);
     return rc;
@@ -1251,6 +1255,7 @@ int pism_gpu_unet_backward(pism_gpu_unet *h, const float *target, const float *w
   if (!h || !target) return PISM_GPU_SSA_EINVAL;
   if (!h->have_forward) return ufail(h, PISM_GPU_SSA_ESTATE, "backward needs a forward first");
   UDevice dg(h->device);
+  if (!side_stream(h)) return ufail(h, PISM_GPU_SSA_ECUDA, "no stream for the weight gradients");
   const int B = h->B, H = h->H, W = h->W;
   const long long P0 = (long long)B * H * W;
   // weights of the backward-data convolutions
