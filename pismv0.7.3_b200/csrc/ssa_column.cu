@@ -10,10 +10,11 @@
 // The 3-D fields are [i][j][k] (a column's Mz levels contiguous).  One thread per column:
 // the horizontal velocity is constant in each column, so u_z = v_z = 0 exactly and the
 // horizontal derivatives, D^2 and its power are the column's, computed once; the thread then
-// walks up its column, summing w by the trapezoid rule in the reference's order of operations
-// and scaling the strain heating by each level's hardness.
+// walks up its column, scaling the strain heating by each level's hardness and summing w by the
+// trapezoid rule in the reference's order of operations.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <map>
 #include <mutex>
 
@@ -23,7 +24,7 @@ namespace pism_gpu {
 
 namespace {
 
-constexpr int NTC = 256;
+constexpr int NTC = 128;   // small blocks: more of the tiles fit an SM
 
 __device__ __forceinline__ bool icy(int m) { return m == 2 || m == 3; }   // Mask.hh:46-48
 
@@ -61,11 +62,40 @@ __device__ __forceinline__ int k_below_height(const double *__restrict__ z, int 
   return lo;
 }
 
-// One warp per 32 consecutive columns (whose [i][j][k] data are 32 Mz consecutive doubles):
-// lane r computes column c0 + r level by level into a shared-memory tile (rows padded to an
-// odd length, so the lanes' writes at one level fall in different banks), then the warp
-// copies the tile out with consecutive lanes on consecutive addresses.  One field at a time.
-__global__ void __launch_bounds__(NTC) k_stress_balance_3d(GridDev g, pism_gpu_ssa_config c, int Mz, int S,
+// The hardness of the flow laws whose softness is Paterson and Budd's A exp(-Q / (R T)) with one
+// exponential: (A exp(-Q / (R T)))^(-1/n) = A^(-1/n) exp(Q / (n R T)).  `melting` is the value at the
+// melting point.
+struct ColdLaw {
+  double A_cold, Q_cold, A_warm, Q_warm;   // A^(-1/n), Q / (n R)
+  double melting;
+};
+
+// hardness_parameter() for the GPBLD and Paterson-Budd laws through ColdLaw
+__device__ __forceinline__ double cold_hardness(const pism_gpu_ssa_config &c, const ColdLaw &l, double E, double P) {
+  const double T = ec_pressure_adjusted_temperature(c, E, P);
+  const bool cold = T < c.Paterson_Budd_critical_temperature;
+  double B = (cold ? l.A_cold : l.A_warm) * exp((cold ? l.Q_cold : l.Q_warm) / T);
+  if (c.flow_law == PISM_FLOW_LAW_GPBLD && !(E < ec_enthalpy_cts(c, P))) {   // temperate: softened by its water
+    const double omega = fmin(ec_water_fraction(c, E, P), c.gpbld_water_frac_observed_limit);
+    B = l.melting * pow(1.0 + c.gpbld_water_frac_coeff * omega, -1.0 / c.ssa_Glen_exponent);
+  }
+  return B;
+}
+
+// One warp per 32 consecutive columns (whose [i][j][k] data are 32 Mz consecutive doubles).  The
+// horizontal velocity goes out with consecutive lanes on consecutive addresses, the column's value
+// taken from its lane.  The strain heating and w are computed column by column (lane r: column
+// c0 + r) in a shared-memory tile, rows padded to an odd length so that the lanes' accesses at one
+// level fall in different banks: the enthalpy is copied in while the velocity goes out (levels in
+// the ice only), the heating takes its place, and the tile is copied out in address order.  pairs:
+// two elements a lane at a time (every array 16-byte aligned).
+//
+// Bound: memory, 1.07 GB for 801 x 801 x 41 with GPBLD (164 us at 6.5 TB/s); the FP64 exponentials
+// next to it.  With 8-warp blocks, every field through the tile, enthalpy read by columns and
+// pow(exp()) a level: 461 us (12 warps an SM, 0.39 instructions a cycle and scheduler, 203 M
+// instructions); one element a lane 267 us (175 M), two 187 us (93 M).
+template <bool COLD>
+__global__ void __launch_bounds__(NTC) k_stress_balance_3d(GridDev g, pism_gpu_ssa_config c, ColdLaw law, int Mz, int S, bool pairs,
                                                            double e_to_a_power, double exponent, double B_iso,
                                                            const double2 *__restrict__ vel,
                                                            const int8_t *__restrict__ mask,
@@ -75,87 +105,159 @@ __global__ void __launch_bounds__(NTC) k_stress_balance_3d(GridDev g, pism_gpu_s
                                                            const double *__restrict__ bmr, double *__restrict__ u3,
                                                            double *__restrict__ v3, double *__restrict__ w3,
                                                            double *__restrict__ sigma) {
-  extern __shared__ double tiles[];
+  extern __shared__ __align__(16) double tiles[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   double *const tile = tiles + (size_t)warp * 32 * S;
   const int N = g.Mx * g.My;
-  for (int c0 = (blockIdx.x * wpb + warp) * 32; c0 < N; c0 += gridDim.x * wpb * 32) {
-    const int col = c0 + lane, ncol = min(32, N - c0);
-    const bool mine = col < N;
-    const int i = mine ? col / g.My : 0, j = mine ? col - i * g.My : 0;
-    const double2 U = mine ? vel[col] : make_double2(0.0, 0.0);
-    // the tile of field q out to dst: columns c0 .. c0 + ncol - 1, all Mz levels
-    auto flush = [&](double *dst) {
-      __syncwarp();
-      const int n = ncol * Mz;
-      double *const out = dst + (size_t)c0 * Mz;
-      int r = lane / Mz, k = lane - r * Mz;   // (column, level) of element e, advanced by 32
-      for (int e = lane; e < n; e += 32) {
-        out[e] = tile[r * S + k];
-        k += 32;
-        while (k >= Mz) {
-          k -= Mz;
-          ++r;
-        }
+  const int c0 = (blockIdx.x * wpb + warp) * 32;
+  if (c0 >= N) return;
+  const int col = c0 + lane, ncol = min(32, N - c0), n = ncol * Mz;
+  const bool mine = col < N;
+  const int i = mine ? col / g.My : 0, j = mine ? col - i * g.My : 0;
+  const double2 U = mine ? vel[col] : make_double2(0.0, 0.0);
+  const double Hc = mine ? H[col] : 0.0;
+  const int ks = mine && sigma ? k_below_height(z, Mz, Hc) : -1;
+  // f(e, r, k) for every element e = r Mz + k of the columns, consecutive lanes on consecutive
+  // elements; all lanes call f (e >= n where there is none left)
+  auto elements = [&](auto f) {
+    int r = lane / Mz, k = lane - r * Mz;
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      f(e0 + lane, r, k);
+      k += 32;
+      while (k >= Mz) {
+        k -= Mz;
+        ++r;
       }
-      __syncwarp();
+    }
+  };
+  // the same for pairs of elements; column of element e by a multiplication (e < 2^15: exact)
+  const unsigned inv = 0xffffffffu / (unsigned)Mz + 1u;
+  auto column_of = [&](int e) { return (int)__umulhi((unsigned)e, inv); };
+  auto lane_of = [&](int e) { return min(column_of(e), 31); };
+  // where the tile has element e, and e + 1 behind it: both are of one column where Mz is even, and
+  // with an odd Mz the rows have no padding
+  const bool linear = S == Mz;
+  auto at = [&](int e) { return linear ? e : e + column_of(e); };
+  auto flush = [&](double *dst) {
+    __syncwarp();
+    double *const out = dst + (size_t)c0 * Mz;
+    if (pairs) {
+      for (int e = 2 * lane; e + 1 < n; e += 64) {
+        const int q = at(e);
+        *reinterpret_cast<double2 *>(out + e) =
+            linear ? *reinterpret_cast<const double2 *>(tile + q) : make_double2(tile[q], tile[q + 1]);
+      }
+      if ((n & 1) && lane == 0) out[n - 1] = tile[n - 1];
+    } else {
+      elements([&](int e, int r, int k) {
+        if (e < n) out[e] = tile[r * S + k];
+      });
+    }
+    __syncwarp();
+  };
+  if (sigma && E) {
+    const double *const Ec = E + (size_t)c0 * Mz;
+    auto copy = [&](int e, double *to) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(Ec + e)
+                   : "memory");
     };
-    if (u3) {
-      if (mine)
-        for (int k = 0; k < Mz; ++k) tile[lane * S + k] = U.x;
-      flush(u3);
+    if (pairs) {
+      for (int e0 = 0; e0 < n; e0 += 64) {
+        const int e = e0 + 2 * lane, r = lane_of(e), k = e - r * Mz;
+        // a pair across two columns begins the next one's, which has ice at its base
+        const int top = __shfl_sync(0xffffffffu, ks, r);
+        if (!linear && e < n && k <= top) {
+          copy(e, tile + at(e));
+          copy(e + 1, tile + at(e) + 1);
+        } else if (linear && e + 1 < n && (k <= top || k + 1 == Mz))
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(tile + e)),
+                       "l"(Ec + e)
+                       : "memory");
+        else if (linear && e + 1 == n && k <= top)
+          copy(e, tile + e);
+      }
+    } else {
+      elements([&](int e, int r, int k) {
+        const int top = __shfl_sync(0xffffffffu, ks, r & 31);
+        if (e < n && k <= top) copy(e, tile + r * S + k);
+      });
     }
-    if (v3) {
-      if (mine)
-        for (int k = 0; k < Mz; ++k) tile[lane * S + k] = U.y;
-      flush(v3);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  if (u3 || v3) {
+    double *const u = u3 ? u3 + (size_t)c0 * Mz : nullptr, *const v = v3 ? v3 + (size_t)c0 * Mz : nullptr;
+    auto of = [&](double x, int r) { return __shfl_sync(0xffffffffu, x, r); };
+    if (pairs) {
+      for (int e0 = 0; e0 < n; e0 += 64) {
+        const int e = e0 + 2 * lane, r = lane_of(e), q = lane_of(e + 1);
+        const double2 x = make_double2(of(U.x, r), of(U.x, q)), y = make_double2(of(U.y, r), of(U.y, q));
+        if (e + 1 < n) {
+          if (u) *reinterpret_cast<double2 *>(u + e) = x;
+          if (v) *reinterpret_cast<double2 *>(v + e) = y;
+        } else if (e < n) {
+          if (u) u[e] = x.x;
+          if (v) v[e] = y.x;
+        }
+      }
+    } else {
+      elements([&](int e, int r, int k) {
+        const double x = of(U.x, r & 31), y = of(U.y, r & 31);
+        if (e < n) {
+          if (u) u[e] = x;
+          if (v) v[e] = y;
+        }
+      });
     }
-    if (!w3 && !sigma) continue;
-    double u_x = 0.0, v_y = 0.0, u_y = 0.0, v_x = 0.0;
+  }
+  if (!w3 && !sigma) return;
+  double u_x = 0.0, v_y = 0.0, u_y = 0.0, v_x = 0.0;
+  if (mine) {
+    const ColumnDiff d = column_diff(g, mask, i, j);
+    const double2 Uw = vel[nbr(g, i, j, -1, 0)], Ue = vel[nbr(g, i, j, 1, 0)], Us = vel[nbr(g, i, j, 0, -1)],
+                  Un = vel[nbr(g, i, j, 0, 1)];
+    u_x = d.D_x * (d.west * (U.x - Uw.x) + d.east * (Ue.x - U.x));
+    v_y = d.D_y * (d.south * (U.y - Us.y) + d.north * (Un.y - U.y));
+    u_y = d.D_y * (d.south * (U.x - Us.x) + d.north * (Un.x - U.x));
+    v_x = d.D_x * (d.west * (U.y - Uw.y) + d.east * (Ue.y - U.y));
+  }
+  if (sigma) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
     if (mine) {
-      const ColumnDiff d = column_diff(g, mask, i, j);
-      const double2 Uw = vel[nbr(g, i, j, -1, 0)], Ue = vel[nbr(g, i, j, 1, 0)], Us = vel[nbr(g, i, j, 0, -1)],
-                    Un = vel[nbr(g, i, j, 0, 1)];
-      u_x = d.D_x * (d.west * (U.x - Uw.x) + d.east * (Ue.x - U.x));
-      v_y = d.D_y * (d.south * (U.y - Us.y) + d.north * (Un.y - U.y));
-      u_y = d.D_y * (d.south * (U.x - Us.x) + d.north * (Un.x - U.x));
-      v_x = d.D_x * (d.west * (U.y - Uw.y) + d.east * (Ue.y - U.y));
-    }
-    if (w3) {
-      // w(0) = -bmr (or 0); w(k) = w(k-1) - (integrand(k) + integrand(k-1)) / 2 dz, the
-      // integrand u_x + v_y the same at every level; the products and sums in that order
-      if (mine) {
-        const double integrand = __dadd_rn(u_x, v_y);
-        const double half_sum = __dmul_rn(0.5, __dadd_rn(integrand, integrand));
-        double w = bmr ? -bmr[col] : 0.0;
-        tile[lane * S] = w;
-        for (int k = 1; k < Mz; ++k) {
-          w = __dsub_rn(w, __dmul_rn(half_sum, __dsub_rn(z[k], z[k - 1])));
-          tile[lane * S + k] = w;
-        }
+      const double a = u_x + v_y, b = u_y + v_x;   // u_z = v_z = 0
+      // D2(), PISMStressBalance.cc:309-311
+      const double D2 = 0.5 * (a * a + u_x * u_x + v_y * v_y + 0.5 * (b * b));
+      const double two_e = 2.0 * e_to_a_power, D2e = pow(D2, exponent);
+      double *const row = tile + lane * S;
+#pragma unroll 2
+      for (int k = 0; k <= ks; ++k) {
+        double B = B_iso;
+        if constexpr (COLD) B = cold_hardness(c, law, row[k], ec_pressure(c, Hc - z[k]));
+        else if (E) B = hardness_parameter(c, row[k], ec_pressure(c, Hc - z[k]));
+        row[k] = two_e * B * D2e;   // the reference's order: (2 e^(-1/n) B) D^(1/n + 1)
       }
-      flush(w3);
+      for (int k = ks + 1; k < Mz; ++k) row[k] = 0.0;
     }
-    if (sigma) {
-      if (mine) {
-        const double Hc = H[col];
-        const int ks = k_below_height(z, Mz, Hc);
-        const double a = u_x + v_y, b = u_y + v_x;   // u_z = v_z = 0
-        // D2(), PISMStressBalance.cc:309-311
-        const double D2 = 0.5 * (a * a + u_x * u_x + v_y * v_y + 0.5 * (b * b));
-        const double two_e = 2.0 * e_to_a_power, D2e = pow(D2, exponent);
-        const double *const Ec = E ? E + (size_t)col * Mz : nullptr;
-        for (int k = 0; k < Mz; ++k) {
-          double s = 0.0;
-          if (k <= ks) {
-            const double B = Ec ? hardness_parameter(c, Ec[k], ec_pressure(c, Hc - z[k])) : B_iso;
-            s = two_e * B * D2e;   // the reference's order: (2 e^(-1/n) B) D^(1/n + 1)
-          }
-          tile[lane * S + k] = s;
-        }
+    flush(sigma);
+  }
+  if (w3) {
+    // w(0) = -bmr (or 0); w(k) = w(k-1) - (integrand(k) + integrand(k-1)) / 2 dz, the
+    // integrand u_x + v_y the same at every level; the products and sums in that order
+    if (mine) {
+      const double integrand = __dadd_rn(u_x, v_y);
+      const double half_sum = __dmul_rn(0.5, __dadd_rn(integrand, integrand));
+      double w = bmr ? -bmr[col] : 0.0, below = z[0];
+      double *const row = tile + lane * S;
+      row[0] = w;
+#pragma unroll 4
+      for (int k = 1; k < Mz; ++k) {
+        const double zk = z[k];
+        w = __dsub_rn(w, __dmul_rn(half_sum, __dsub_rn(zk, below)));
+        row[k] = w;
+        below = zk;
       }
-      flush(sigma);
     }
+    flush(w3);
   }
 }
 
@@ -174,17 +276,35 @@ void launch_stress_balance_3d(const Launch &L, const GridDev &g, const pism_gpu_
   const int N = g.Mx * g.My;
   int warps = 0;
   const int smem = stress_balance_3d_smem(Mz, &warps);
-  const int blocks = std::max(1, std::min((N + 32 * warps - 1) / (32 * warps), 4 * L.max_blocks));
+  const int blocks = (N + 32 * warps - 1) / (32 * warps);
   // PISMStressBalance.cc:384-387: the flow law's exponent and enhancement factor; an
   // isothermal flow law's hardness A^(-1/n) is the same at every level
   const double n = c.ssa_Glen_exponent, exponent = 0.5 * (1.0 / n + 1.0);
   const double e_to_a_power = std::pow(c.ssa_enhancement_factor, -1.0 / n);
   const bool iso = c.flow_law == PISM_FLOW_LAW_ISOTHERMAL_GLEN;
   const double B_iso = iso ? std::pow(c.ice_softness, -1.0 / n) : 0.0;
+  // the laws with one exponential a level; the others as in ssa_device.cuh
+  const bool cold = c.flow_law == PISM_FLOW_LAW_GPBLD || c.flow_law == PISM_FLOW_LAW_PB;
+  ColdLaw law{};
+  if (cold) {
+    law.A_cold = std::pow(c.Paterson_Budd_A_cold, -1.0 / n);
+    law.Q_cold = c.Paterson_Budd_Q_cold / (n * c.ideal_gas_constant);
+    law.A_warm = std::pow(c.Paterson_Budd_A_warm, -1.0 / n);
+    law.Q_warm = c.Paterson_Budd_Q_warm / (n * c.ideal_gas_constant);
+    const double Tm = c.water_melting_point_temperature;
+    const bool below = Tm < c.Paterson_Budd_critical_temperature;
+    law.melting = (below ? law.A_cold : law.A_warm) * std::exp((below ? law.Q_cold : law.Q_warm) / Tm);
+  }
+  // rows of an odd length: with an odd number of levels the tile is the columns' memory as it is
+  const double *const E = iso ? nullptr : f.enthalpy;
+  const int S = Mz | 1;
+  bool pairs = true;
+  for (const double *q : {(const double *)u3, (const double *)v3, (const double *)w3, (const double *)sigma, E})
+    pairs = pairs && reinterpret_cast<uintptr_t>(q) % 16 == 0;
   L.tick();
-  k_stress_balance_3d<<<blocks, 32 * warps, smem, L.stream>>>(g, c, Mz, Mz | 1, e_to_a_power, exponent, B_iso, f.vel,
-                                                               f.mask, f.H, iso ? nullptr : f.enthalpy, z, bmr, u3,
-                                                               v3, w3, sigma);
+  const auto kernel = cold ? k_stress_balance_3d<true> : k_stress_balance_3d<false>;
+  kernel<<<blocks, 32 * warps, smem, L.stream>>>(g, c, law, Mz, S, pairs, e_to_a_power, exponent, B_iso, f.vel, f.mask, f.H, E, z,
+                                                 bmr, u3, v3, w3, sigma);
 }
 
 // the kernel's dynamic shared-memory limit for Mz levels on the current device: a function
@@ -199,9 +319,8 @@ int stress_balance_3d_prepare(int Mz) {
   std::lock_guard<std::mutex> guard(lock);
   auto it = raised.find(dev);
   if (it != raised.end() && smem <= it->second) return 0;
-  if (cudaFuncSetAttribute((const void *)k_stress_balance_3d, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-      cudaSuccess)
-    return 1;
+  for (const void *kernel : {(const void *)k_stress_balance_3d<true>, (const void *)k_stress_balance_3d<false>})
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 1;
   raised[dev] = smem;
   return 0;
 }
