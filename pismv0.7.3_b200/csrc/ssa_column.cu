@@ -63,18 +63,29 @@ __device__ __forceinline__ int k_below_height(const double *__restrict__ z, int 
 }
 
 // The hardness of the flow laws whose softness is Paterson and Budd's A exp(-Q / (R T)) with one
-// exponential: (A exp(-Q / (R T)))^(-1/n) = A^(-1/n) exp(Q / (n R T)).  `melting` is the value at the
-// melting point.
+// exponential: with p = 1/n as rounded, (A exp(-x))^(-p) = A^(-p) exp(x p).  The exponent x p is near
+// 9, so its rounding would be several of the result's: what the product loses is put back as a
+// factor (exp(y + r) = exp(y) (1 + r), r below 1e-15), with what A^(-p) and the last product lose.
+// `melting` is the value at the melting point.
 struct ColdLaw {
-  double A_cold, Q_cold, A_warm, Q_warm;   // A^(-1/n), Q / (n R)
+  double A_cold, Q_cold, A_warm, Q_warm;   // A^(-p), Q
+  double lost_cold, lost_warm;             // the relative rounding of A^(-p)
+  double R, p;
   double melting;
 };
+
+__host__ __device__ inline double paterson_budd_hardness(const ColdLaw &l, bool cold, double T) {
+  const double x = (cold ? l.Q_cold : l.Q_warm) / (l.R * T), y = x * l.p;
+  const double r = fma(x, l.p, -y) + (cold ? l.lost_cold : l.lost_warm);
+  const double A = cold ? l.A_cold : l.A_warm, e = exp(y), B = A * e;
+  const double lost = fma(A, e, -B);
+  return B > 0.0 && B < INFINITY ? B + fma(B, r, lost) : B;   // an exponent out of range leaves no remainder
+}
 
 // hardness_parameter() for the GPBLD and Paterson-Budd laws through ColdLaw
 __device__ __forceinline__ double cold_hardness(const pism_gpu_ssa_config &c, const ColdLaw &l, double E, double P) {
   const double T = ec_pressure_adjusted_temperature(c, E, P);
-  const bool cold = T < c.Paterson_Budd_critical_temperature;
-  double B = (cold ? l.A_cold : l.A_warm) * exp((cold ? l.Q_cold : l.Q_warm) / T);
+  double B = paterson_budd_hardness(l, T < c.Paterson_Budd_critical_temperature, T);
   if (c.flow_law == PISM_FLOW_LAW_GPBLD && !(E < ec_enthalpy_cts(c, P))) {   // temperate: softened by its water
     const double omega = fmin(ec_water_fraction(c, E, P), c.gpbld_water_frac_observed_limit);
     B = l.melting * pow(1.0 + c.gpbld_water_frac_coeff * omega, -1.0 / c.ssa_Glen_exponent);
@@ -287,13 +298,19 @@ void launch_stress_balance_3d(const Launch &L, const GridDev &g, const pism_gpu_
   const bool cold = c.flow_law == PISM_FLOW_LAW_GPBLD || c.flow_law == PISM_FLOW_LAW_PB;
   ColdLaw law{};
   if (cold) {
-    law.A_cold = std::pow(c.Paterson_Budd_A_cold, -1.0 / n);
-    law.Q_cold = c.Paterson_Budd_Q_cold / (n * c.ideal_gas_constant);
-    law.A_warm = std::pow(c.Paterson_Budd_A_warm, -1.0 / n);
-    law.Q_warm = c.Paterson_Budd_Q_warm / (n * c.ideal_gas_constant);
+    law.p = 1.0 / n;
+    law.R = c.ideal_gas_constant;
+    law.Q_cold = c.Paterson_Budd_Q_cold;
+    law.Q_warm = c.Paterson_Budd_Q_warm;
+    const auto power = [&](double A, double *rounded, double *lost) {
+      const long double v = std::pow((long double)A, -(long double)law.p);
+      *rounded = (double)v;
+      *lost = std::isfinite(*rounded) && *rounded > 0.0 ? (double)((v - *rounded) / v) : 0.0;
+    };
+    power(c.Paterson_Budd_A_cold, &law.A_cold, &law.lost_cold);
+    power(c.Paterson_Budd_A_warm, &law.A_warm, &law.lost_warm);
     const double Tm = c.water_melting_point_temperature;
-    const bool below = Tm < c.Paterson_Budd_critical_temperature;
-    law.melting = (below ? law.A_cold : law.A_warm) * std::exp((below ? law.Q_cold : law.Q_warm) / Tm);
+    law.melting = paterson_budd_hardness(law, Tm < c.Paterson_Budd_critical_temperature, Tm);
   }
   // rows of an odd length: with an odd number of levels the tile is the columns' memory as it is
   const double *const E = iso ? nullptr : f.enthalpy;
