@@ -955,11 +955,15 @@ int prepare(pism_gpu_ssa *h) {
 // staging of the strain rates and eigen-calving, in doubles from h->ec: strain rates 2 N at
 // EC_EDOT, stresses 3 N at EC_STRESS, the caller's mask N at EC_MASK; eigen-calving's Href,
 // thickness and per-cell loss N each at EC_HREF, EC_H, EC_LOSS (over the strain-rate slots,
-// which it does not use); 8 scalars at EC_SCALARS.  Plus 2 N bytes of masks in h->ec_mask.
+// which it does not use); 8 scalars at EC_SCALARS (the time step's statistics, from 3 on the
+// sweeps' flags, at 7 the rates' maximum, 0 between calls).  Plus 2 N bytes of masks in h->ec_mask.
 enum : size_t { EC_EDOT = 0, EC_STRESS = 2, EC_MASK = 5, EC_HREF = 0, EC_H = 1, EC_LOSS = 2, EC_SCALARS = 6 };
 
 int ec_buffers(pism_gpu_ssa *h) {
-  if (!h->ec) RET(dalloc(h, &h->ec, EC_SCALARS * (size_t)h->N + 8));
+  if (!h->ec) {
+    RET(dalloc(h, &h->ec, EC_SCALARS * (size_t)h->N + 8));
+    CK(h, cudaMemsetAsync(h->ec + EC_SCALARS * (size_t)h->N, 0, 8 * sizeof(double), h->stream));
+  }
   if (!h->ec_mask) RET(dalloc(h, &h->ec_mask, 2 * (size_t)h->N));
   return PISM_GPU_SSA_OK;
 }
@@ -1382,19 +1386,14 @@ int pism_gpu_ssa_strain_rates(pism_gpu_ssa *h, const double *mask, double *edot,
   if (!h->inputs_set) return fail(h, PISM_GPU_SSA_ESTATE, "pism_gpu_ssa_set_inputs was not called");
   const size_t N = h->N;
   RET(ec_buffers(h));
-  const int8_t *m = h->mask;
-  if (mask) {
-    const double *dm = mask;
-    if (where == PISM_MEM_HOST) {
-      RET(copy_in(h, h->ec + EC_MASK * N, mask, sizeof(double) * N, PISM_MEM_HOST));
-      dm = h->ec + EC_MASK * N;
-    }
-    launch_mask_from_doubles(h->L, h->N, dm, h->ec_mask, nullptr);
-    m = h->ec_mask;
+  const double *dm = mask;
+  if (mask && where == PISM_MEM_HOST) {
+    RET(copy_in(h, h->ec + EC_MASK * N, mask, sizeof(double) * N, PISM_MEM_HOST));
+    dm = h->ec + EC_MASK * N;
   }
   double *de = (edot && where == PISM_MEM_HOST) ? h->ec + EC_EDOT * N : edot;
   double *ds = (stresses && where == PISM_MEM_HOST) ? h->ec + EC_STRESS * N : stresses;
-  launch_strain_rates(h->L, h->g, h->cfg, h->vel, m, de, ds);
+  launch_strain_rates(h->L, h->g, h->cfg, h->vel, h->mask, dm, de, ds);
   CK(h, cudaGetLastError());
   if (edot && where == PISM_MEM_HOST) RET(copy_out(h, edot, de, sizeof(double) * 2 * N, PISM_MEM_HOST));
   if (stresses && where == PISM_MEM_HOST) RET(copy_out(h, stresses, ds, sizeof(double) * 3 * N, PISM_MEM_HOST));
@@ -1422,21 +1421,18 @@ int pism_gpu_ssa_eigen_calving(pism_gpu_ssa *h, double dt, double K, double *mas
   }
   int8_t *m0 = h->ec_mask, *live = h->ec_mask + N;
   int *changed = reinterpret_cast<int *>(h->ec + EC_SCALARS * N + 3);
-  launch_mask_from_doubles(h->L, h->N, dm, m0, live);
-  launch_eigen_calving_passes(h->L, h->g, h->vel, K, dt, dH, dHref, h->ec + EC_LOSS * N, m0, live);
+  launch_eigen_calving(h->L, h->g, h->vel, K, dt, dm, dH, dHref, h->ec + EC_LOSS * N, m0, live, changed);
   // remove_narrow_tongues: sweep until no cell changes; a chain of dependent cells is at
   // most N long, so N + 1 sweeps always reach the fixed point
-  for (size_t sweep = 0;; ++sweep) {
-    if (sweep > N) return fail(h, PISM_GPU_SSA_ECUDA, "remove_narrow_tongues did not settle");
-    CK(h, cudaMemsetAsync(changed, 0, sizeof(int), h->stream));
-    launch_tongue_sweep(h->L, h->g, m0, live, changed);
+  for (size_t sweeps = TONGUE_SWEEPS;; sweeps += TONGUE_SWEEPS) {
     CK(h, cudaGetLastError());
     int flag = 0;
-    RET(copy_out(h, &flag, changed, sizeof(int), PISM_MEM_HOST));
+    RET(copy_out(h, &flag, changed + TONGUE_SWEEPS - 1, sizeof(int), PISM_MEM_HOST));
     if (!flag) break;
+    if (sweeps > N) return fail(h, PISM_GPU_SSA_ECUDA, "remove_narrow_tongues did not settle");
+    CK(h, cudaMemsetAsync(changed, 0, TONGUE_SWEEPS * sizeof(int), h->stream));
+    launch_tongue_sweeps(h->L, h->g, dm, dH, m0, live, changed);
   }
-  launch_eigen_calving_finish(h->L, h->N, m0, live, dH, dm);
-  CK(h, cudaGetLastError());
   if (where == PISM_MEM_HOST) {
     RET(copy_out(h, mask, dm, sizeof(double) * N, PISM_MEM_HOST));
     RET(copy_out(h, Href, dHref, sizeof(double) * N, PISM_MEM_HOST));
@@ -1461,10 +1457,7 @@ int pism_gpu_ssa_eigen_calving_max_timestep(pism_gpu_ssa *h, double K, const dou
     dm = h->ec + EC_MASK * N;
   }
   double *stats = h->ec + EC_SCALARS * N;   // count, sum of rates, maximum rate (bits)
-  CK(h, cudaMemsetAsync(stats, 0, 3 * sizeof(double), h->stream));
-  launch_mask_from_doubles(h->L, h->N, dm, h->ec_mask, nullptr);
-  launch_eigen_calving_rates(h->L, h->g, h->vel, h->ec_mask, K, stats,
-                             reinterpret_cast<unsigned long long *>(stats + 2));
+  launch_eigen_calving_rates(h->L, h->g, h->vel, dm, K, stats, reinterpret_cast<unsigned long long *>(stats + 7));
   CK(h, cudaGetLastError());
   double s[3];
   RET(copy_out(h, s, stats, sizeof(s), PISM_MEM_HOST));

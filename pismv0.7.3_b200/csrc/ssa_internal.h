@@ -184,15 +184,19 @@ void launch_mass_continuity(const Launch &L, const GridDev &g, const pism_gpu_ss
                             const double *bmr, const double *area, double *Hnew, double *fdiv, double *mask_new,
                             double *surface_new, double *totals);
 // ---- strain rates, 2-D stresses and eigen-calving (ssa_calving.cu) ----
+// the mask: the caller's where it is given
 void launch_strain_rates(const Launch &L, const GridDev &g, const pism_gpu_ssa_config &c, const double2 *vel,
-                         const int8_t *mask, double *edot, double *stress);
-void launch_mask_from_doubles(const Launch &L, int N, const double *in, int8_t *a, int8_t *b);
-void launch_eigen_calving_passes(const Launch &L, const GridDev &g, const double2 *vel, double K, double dt,
-                                 double *H, double *Href, double *loss, int8_t *m0, int8_t *live);
-void launch_tongue_sweep(const Launch &L, const GridDev &g, const int8_t *m0, int8_t *live, int *changed);
-void launch_eigen_calving_finish(const Launch &L, int N, const int8_t *m0, const int8_t *live, double *H,
-                                 double *mask_out);
-void launch_eigen_calving_rates(const Launch &L, const GridDev &g, const double2 *vel, const int8_t *mask, double K,
+                         const int8_t *mask, const double *caller_mask, double *edot, double *stress);
+// An eigen-calving step and a first batch of remove_narrow_tongues' sweeps.  changed: TONGUE_SWEEPS
+// flags; the step is done (mask and H written) where the last one is 0, else further batches
+// follow, with the flags cleared.  Four: the sweeps of a mask without long tongues, the one that
+// finds nothing to do among them; a sweep too many costs a launch, a batch too many a round trip.
+constexpr int TONGUE_SWEEPS = 4;
+void launch_eigen_calving(const Launch &L, const GridDev &g, const double2 *vel, double K, double dt, double *mask,
+                          double *H, double *Href, double *loss, int8_t *m0, int8_t *live, int *changed);
+void launch_tongue_sweeps(const Launch &L, const GridDev &g, double *mask, double *H, const int8_t *m0, int8_t *live,
+                          int *changed);
+void launch_eigen_calving_rates(const Launch &L, const GridDev &g, const double2 *vel, const double *mask, double K,
                                 double *out, unsigned long long *rmax);
 constexpr int SB3D_MAX_LEVELS = 800;   // the column kernel's shared-memory tile holds 32 columns
 int stress_balance_3d_prepare(int Mz);
