@@ -34,6 +34,7 @@ constexpr int PH = TH + 2, PW = TW + 2;   // input patch with the 3 x 3 halo
 constexpr int THREADS = 256;              // 8 warps, one or two tile rows each
 constexpr int WG_THREADS = 288;           // weight gradient: 9 warps = 9 taps
 constexpr int WG_MAX_CTAS = 64;           // pixel-range partial sums per weight gradient
+constexpr int BIAS_MAX_CTAS = 256;        // and per bias gradient
 
 // ---- the network ----
 struct LayerDef {
@@ -372,12 +373,19 @@ __global__ void k_reduce_parts(const float *__restrict__ part, int nparts, int n
   }
 }
 
-// the same for few outputs (n <= 128): one block brings the parts to shared memory in rows of
-// 64, then a thread adds an output's in order
-constexpr int RS_ROWS = 64, RS_MAX = 128;
-__global__ void __launch_bounds__(256) k_reduce_few(const float *__restrict__ part, int nparts, int n,
-                                                    float *__restrict__ out) {
+// The same for few outputs (n <= 128), a block per sum: it brings the parts to shared memory in
+// rows of 64, then a thread adds an output's in order.  All bias gradients and the head's in one
+// launch: one block each, 9 us one after the other on the weight gradients' stream.
+constexpr int RS_ROWS = 64, RS_MAX = 128, FEW_SUMS = NLAYERS + 1;
+struct FewSums {
+  const float *part[FEW_SUMS];
+  float *out[FEW_SUMS];
+  int nparts[FEW_SUMS], n[FEW_SUMS];
+};
+__global__ void __launch_bounds__(256) k_reduce_few(FewSums f) {
   __shared__ float rows[RS_ROWS * RS_MAX];
+  const float *__restrict__ const part = f.part[blockIdx.x];
+  const int nparts = f.nparts[blockIdx.x], n = f.n[blockIdx.x];
   float s = 0.0f;
   for (int q0 = 0; q0 < nparts; q0 += RS_ROWS) {
     const int nq = min(RS_ROWS, nparts - q0);
@@ -390,7 +398,7 @@ __global__ void __launch_bounds__(256) k_reduce_few(const float *__restrict__ pa
       for (int q = 0; q < nq; ++q) s += rows[q * n + threadIdx.x];
     }
   }
-  if ((int)threadIdx.x < n) out[threadIdx.x] = s;
+  if ((int)threadIdx.x < n) f.out[blockIdx.x][threadIdx.x] = s;
 }
 
 // part[cta][c] = sum over the CTA's pixels of dy[p, c]
@@ -855,7 +863,8 @@ struct pism_gpu_unet {
   float *wg_part = nullptr;   // weight-gradient partial sums
   size_t wg_part_n = 0;
   float *small_part = nullptr;   // head / loss partial sums
-  float *bias_part = nullptr;    // bias partial sums
+  float *bias_part = nullptr;    // bias partial sums, BIAS_MAX_CTAS x RS_MAX a layer
+  FewSums few = {};              // the sums of a backward's last launch
   cudaStream_t side = nullptr;   // the weight gradients, beside the data gradients
   cudaEvent_t ready[NLAYERS] = {}, side_done = nullptr;
   float *sums = nullptr;
@@ -993,10 +1002,16 @@ void conv_wgrad(pism_gpu_unet *h, cudaStream_t s, const bf16 *x, int Cin, const 
   k_reduce_parts<<<grid_for(n), 256, 0, s>>>(h->wg_part, ctas, n, dW);
 }
 
-void bias_grad(pism_gpu_unet *h, cudaStream_t s, const bf16 *dy, int C, long long P, float *db) {
-  const int ctas = (int)std::min<long long>(256, std::max(1LL, P / 64));
-  k_bias_grad<<<ctas, 256, 0, s>>>(dy, C, P, h->bias_part);
-  k_reduce_few<<<1, 256, 0, s>>>(h->bias_part, ctas, C, db);
+// layer l's partial bias gradients; the sums follow in one launch for all layers
+void bias_grad(pism_gpu_unet *h, int l, const bf16 *dy, long long P) {
+  const int C = LAYERS[l].cout;
+  FewSums &f = h->few;
+  f.nparts[l] = (int)std::min<long long>(BIAS_MAX_CTAS, std::max(1LL, P / 64));
+  f.n[l] = C;
+  f.out[l] = h->grad + h->b_off[l];
+  float *const part = h->bias_part + (size_t)l * BIAS_MAX_CTAS * RS_MAX;
+  f.part[l] = part;
+  k_bias_grad<<<f.nparts[l], 256, 0, h->stream>>>(dy, C, P, part);
 }
 
 // the second stream and its events, from the first backward on: a network that only predicts has none
@@ -1009,8 +1024,9 @@ bool side_stream(pism_gpu_unet *h) {
 }
 
 // Layer l backward: X input, dY given, masked by the layer's ReLU; dX (masked by xmask, its own
-// layer's output, where given) on the handle's stream, dW and db beside it on the second one: the
-// data gradients are the only chain.
+// layer's output, where given) and db on the handle's stream, dW beside them on the second one: the
+// data gradients are the only chain, and with db behind them the streams are about as long
+// (16 x 128 x 128, kernel time: 450 and 410 us; 360 and 590 with all that is not a chain on the second).
 cudaError_t layer_back(pism_gpu_unet *h, int l, const bf16 *X, const bf16 *dY, bf16 *dX, const bf16 *xmask, int B, int H,
                        int W) {
   const LayerDef &L = LAYERS[l];
@@ -1019,7 +1035,7 @@ cudaError_t layer_back(pism_gpu_unet *h, int l, const bf16 *X, const bf16 *dY, b
   if (e != cudaSuccess) return e;
   if (dX) conv(h->stream, dY, L.cout, h->flip + h->flip_off[l], nullptr, 0, xmask, dX, L.cin, B, H, W);
   conv_wgrad(h, h->side, X, L.cin, dY, L.cout, B, H, W, h->grad + h->w_off[l]);
-  bias_grad(h, h->side, dY, L.cout, (long long)B * H * W, h->grad + h->b_off[l]);
+  bias_grad(h, l, dY, (long long)B * H * W);
   return cudaSuccess;
 }
 
@@ -1114,7 +1130,7 @@ int pism_gpu_unet_create(int device, int max_batch, int max_h, int max_w, pism_g
   A(&h->flip, h->flip_n);
   AF(&h->wg_part, h->wg_part_n);
   AF(&h->small_part, 256 * 130);
-  AF(&h->bias_part, 256 * 130);
+  AF(&h->bias_part, (size_t)NLAYERS * BIAS_MAX_CTAS * RS_MAX);
   AF(&h->sums, 4);
   if (rc == PISM_GPU_SSA_OK && cudaMallocHost((void **)&h->sums_host, 4 * sizeof(float)) != cudaSuccess)
     rc = PISM_GPU_SSA_ENOMEM;
@@ -1275,7 +1291,10 @@ int pism_gpu_unet_backward(pism_gpu_unet *h, const float *target, const float *w
   constexpr int NG = HEAD_COUT * HEAD_CIN + HEAD_COUT;
   k_head_back<<<hctas, 256, 0, h->stream>>>(h->act[9], h->y, target, weight, h->sums, h->p32 + h->head_off, P0, h->dd1,
                                             h->small_part);
-  k_reduce_few<<<1, 256, 0, h->stream>>>(h->small_part, hctas, NG, h->grad + h->head_off);
+  h->few.part[NLAYERS] = h->small_part;
+  h->few.nparts[NLAYERS] = hctas;
+  h->few.n[NLAYERS] = NG;
+  h->few.out[NLAYERS] = h->grad + h->head_off;
   // decoder (every gradient masked by its layer's ReLU where it is made)
   UCK(h, layer_back(h, 9, h->c1, h->dd1, h->dc1, nullptr, B, H, W));
   k_upcat_back<<<grid_for(P0 * 12), 256, 0, h->stream>>>(h->dc1, 64, 32, B, H, W, h->act[8], h->dd2, h->de1);
@@ -1298,6 +1317,7 @@ int pism_gpu_unet_backward(pism_gpu_unet *h, const float *target, const float *w
   k_pool_back_add<<<grid_for(P0 * 4), 256, 0, h->stream>>>(h->dp1, 32, B, H, W, h->act[1], h->de1);
   UCK(h, layer_back(h, 1, h->act[0], h->de1, h->de1a, h->act[0], B, H, W));
   UCK(h, layer_back(h, 0, h->in16, h->de1a, nullptr, nullptr, B, H, W));
+  k_reduce_few<<<FEW_SUMS, 256, 0, h->stream>>>(h->few);
   UCK(h, cudaEventRecord(h->side_done, h->side));
   UCK(h, cudaStreamWaitEvent(h->stream, h->side_done, 0));
   UCK(h, cudaGetLastError());
