@@ -120,24 +120,43 @@ __device__ __forceinline__ void copy_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// A layer's input, [b, i, j, channel]: x, or the concatenation [up[b, i/2, j/2, 0:Cu], x[b, i, j, :]]
+// of the decoder, read where its parts are (as an array of its own it was written and read again,
+// 45 us of kernels in a 16 x 128 x 128 step).  Cu and x's C are
+// multiples of the kernels' channel slices, so a slice is in one of them.
+struct ConvIn {
+  const bf16 *x, *up;
+  int C, Cu;
+  __host__ __device__ int channels() const { return C + Cu; }
+};
+
 // Copy the ROWS x (TW+2) patch of channels [c0, c0 + CS) around the tile at (i0, j0) of image b;
 // zero outside the image.
 template <int CS, int NTHR, int ROWS>
-__device__ __forceinline__ void copy_patch(bf16 *patch, const bf16 *__restrict__ x, int C, int c0, int b, int i0, int j0,
-                                           int H, int W) {
+__device__ __forceinline__ void copy_patch(bf16 *patch, const ConvIn &in, int c0, int b, int i0, int j0, int H, int W) {
   constexpr int CP = CS + 8, CH = CS / 8;
+  const int half = c0 < in.Cu ? 1 : 0, C = half ? in.Cu : in.C, Hs = H >> half, Ws = W >> half;
+  const bf16 *__restrict__ const x = half ? in.up + c0 : in.x + (c0 - in.Cu);
   for (int q = threadIdx.x; q < ROWS * PW * CH; q += NTHR) {
     const int pix = q / CH, ch = q - pix * CH;
     const int pi = pix / PW, pj = pix - pi * PW;
     const int ii = i0 - 1 + pi, jj = j0 - 1 + pj;
     const bool inside = ii >= 0 && ii < H && jj >= 0 && jj < W;
-    copy16(patch + pix * CP + ch * 8, inside ? x + (((size_t)b * H + ii) * W + jj) * C + c0 + ch * 8 : x, inside);
+    copy16(patch + pix * CP + ch * 8, inside ? x + (((size_t)b * Hs + (ii >> half)) * Ws + (jj >> half)) * C + ch * 8 : x,
+           inside);
   }
 }
 
 // ---- 3x3 convolution (forward, and backward data on flipped weights) ----
 // y[b, i, j, co] = act(bias[co] + sum_{tap, ci} w[tap, co, ci] * x[b, i + ky - 1, j + kx - 1, ci]),
 // zero where omask[b, i, j, co] <= 0 (backward data: the ReLU of the layer that made the input).
+//
+// With QUADS (and MR = 2: a warp has both rows of a 2 x 2 block, the columns are four lanes apart)
+// the kernel also makes the sums over 2 x 2 blocks that follow it, of the outputs as rounded: the
+// mean that the next level reads, or the gradient of the upsampled part of a concatenation; the
+// gradient of its other part goes out in place.  As kernels of their own these read and wrote every
+// output again: 16 x 128 x 128, convolutions with concatenations and sums 600 us of kernel time a
+// step, in one 547; the step 1055 -> 988 us, the forward of 1 x 408 x 408 267 -> 235 us.
 //
 // A CTA walks pixel tiles of 8 MR x 16 pixels for NB output channels; each warp has MR rows (16
 // pixels a row) by all NB channels.  A step is one channel slice of a tile: its patch (and its
@@ -148,14 +167,24 @@ __device__ __forceinline__ void copy_patch(bf16 *patch, const bf16 *__restrict__
 // channels, the warps waited on global loads (9 of 17 stalled warps an issue, the tensor pipe
 // 28 - 36 % active).  Every output adds the same products in the same order (slices, taps, halves
 // of a slice) whatever the tile, so the tile may follow the shape.  Forward of 1 x 408 x 408 (34
-// GFLOP): 314 us then, 269 us now.
+// GFLOP): 314 us then, 269 us with the copies ahead.
+// What a kernel with QUADS adds: q[b, I, J, co] = scale x the sum of the outputs co < C over the
+// 2 x 2 block, zero where mask[b, I, J, co] <= 0; y gets the channels from y0 on, as its own
+// channels 0 and up.  C and y0 are multiples of 32.
+struct Quads {
+  bf16 *q;
+  const bf16 *mask;
+  int C, y0;
+  float scale;
+};
+
 template <int CS, int NB, int MR, bool RESIDENT>
 constexpr int conv_smem() {
   return (2 * (8 * MR + 2) * PW + (RESIDENT ? 1 : 2) * 9 * NB) * (CS + 8) * (int)sizeof(bf16);
 }
 
-template <int CS, int NB, int MR, bool RESIDENT>
-__global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x, int Cin, const bf16 *__restrict__ w,
+template <int CS, int NB, int MR, bool RESIDENT, bool QUADS>
+__global__ void __launch_bounds__(THREADS) k_conv3x3(ConvIn in, Quads quads, const bf16 *__restrict__ w,
                                                      const float *__restrict__ bias, int relu,
                                                      const bf16 *__restrict__ omask, bf16 *__restrict__ y, int Cout,
                                                      int B, int H, int W) {
@@ -163,7 +192,7 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x,
   extern __shared__ __align__(16) bf16 conv_sm[];
   bf16 *const patches = conv_sm, *const weights = conv_sm + 2 * PATCH;
   const int tiles_w = (W + TW - 1) / TW, tiles_h = (H + 8 * MR - 1) / (8 * MR), tiles = B * tiles_h * tiles_w;
-  const int co0 = blockIdx.y * NB, nslice = Cin / CS;
+  const int Cin = in.channels(), co0 = blockIdx.y * NB, nslice = Cin / CS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int steps = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * nslice;
   // ldmatrix row addresses: A (pixels x channels, row-major), B (channels x couts, stored [cout][cin])
@@ -191,7 +220,7 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x,
     int b, i0, j0;
     tile_at(step, b, i0, j0);
     const int c0 = step % nslice * CS;
-    copy_patch<CS, THREADS, ROWS>(patches + (step & 1) * PATCH, x, Cin, c0, b, i0, j0, H, W);
+    copy_patch<CS, THREADS, ROWS>(patches + (step & 1) * PATCH, in, c0, b, i0, j0, H, W);
     if (!RESIDENT) copy_weights(weights + (step & 1) * WSM, c0);
   };
   if (RESIDENT) copy_weights(weights, 0);
@@ -235,14 +264,16 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x,
     tile_at(step, b, i0, j0);
     const int g = lane >> 2, tq = lane & 3;
 #pragma unroll
-    for (int m = 0; m < MR; ++m) {
-      const int i = i0 + MR * warp + m;
+    for (int q = 0; q < NB / 32; ++q) {
+      const int co = co0 + 32 * q + 8 * tq;
+      const bool own = !QUADS || co0 + 32 * q >= quads.y0, sums = QUADS && co0 + 32 * q < quads.C;
 #pragma unroll
-      for (int q = 0; q < NB / 32; ++q) {
-        const int co = co0 + 32 * q + 8 * tq;
+      for (int hh = 0; hh < 2; ++hh) {
+        const int j = j0 + g + 8 * hh;
+        uint4 out[MR];
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          const int j = j0 + g + 8 * hh;
+        for (int m = 0; m < MR; ++m) {
+          const int i = i0 + MR * warp + m;
           float v[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
@@ -250,11 +281,36 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x,
             acc[m][4 * q + u / 2][2 * hh + (u & 1)] = 0.0f;   // the next tile's
             if (relu) v[u] = fmaxf(v[u], 0.0f);
           }
-          if (i >= H || j >= W) continue;
-          const size_t off = (((size_t)b * H + i) * W + j) * Cout + co;
-          uint4 out = pack8(v);
-          if (omask) out = relu_mask8(out, *reinterpret_cast<const uint4 *>(omask + off));
-          *reinterpret_cast<uint4 *>(y + off) = out;
+          out[m] = pack8(v);
+          if (!own || i >= H || j >= W) continue;
+          const int Cy = QUADS ? Cout - quads.y0 : Cout;
+          const size_t off = (((size_t)b * H + i) * W + j) * Cy + (QUADS ? co - quads.y0 : co);
+          if (omask) out[m] = relu_mask8(out[m], *reinterpret_cast<const uint4 *>(omask + off));
+          *reinterpret_cast<uint4 *>(y + off) = out[m];
+        }
+        if constexpr (QUADS) {
+          static_assert(MR == 2, "a warp has both rows of a block");
+          if (!sums) continue;
+          // (row, column) in the order (0, 0), (0, 1), (1, 0), (1, 1)
+          float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const uint4 o = make_uint4(__shfl_down_sync(0xffffffffu, out[m].x, 4), __shfl_down_sync(0xffffffffu, out[m].y, 4),
+                                       __shfl_down_sync(0xffffffffu, out[m].z, 4), __shfl_down_sync(0xffffffffu, out[m].w, 4));
+            float f[8], r[8];
+            unpack8(out[m], f);
+            unpack8(o, r);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s[u] = s[u] + f[u] + r[u];
+          }
+          const int i = i0 + 2 * warp;
+          if ((g & 1) || i >= H || j >= W) continue;   // H and W are even: the block is all inside
+#pragma unroll
+          for (int u = 0; u < 8; ++u) s[u] *= quads.scale;
+          const size_t off = (((size_t)b * (H / 2) + i / 2) * (W / 2) + j / 2) * quads.C + co;
+          uint4 sum = pack8(s);
+          if (quads.mask) sum = relu_mask8(sum, *reinterpret_cast<const uint4 *>(quads.mask + off));
+          *reinterpret_cast<uint4 *>(quads.q + off) = sum;
         }
       }
     }
@@ -268,8 +324,8 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(const bf16 *__restrict__ x,
 // of their sums do not depend on CO and CI, which follow from how many CTAs they leave.
 //
 // Bound: the chain of a CTA's tiles (its sum's order is fixed).  Waiting for each tile's loads
-// took 4.3 us a tile.  Forward, backward and Adam of 16 x 128 x 128: 1.87 ms then, 1.13 ms now, of
-// which the gradients on a stream of their own, one launch for all flipped weights and the masks
+// took 4.3 us a tile.  Forward, backward and Adam of 16 x 128 x 128: 1.87 ms then, 1.13 ms with the
+// copies ahead, of which the gradients on a stream of their own, one launch for all flipped weights and the masks
 // made by their producers are a part.
 constexpr int WG_STAGES = 3;
 template <int CI, int CO>
@@ -278,12 +334,11 @@ constexpr int wgrad_smem() {
 }
 
 template <int CI, int CO>
-__global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(const bf16 *__restrict__ x, int Cin,
-                                                              const bf16 *__restrict__ dy, int Cout, int B, int H,
-                                                              int W, float *__restrict__ part) {
+__global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(ConvIn in, const bf16 *__restrict__ dy,
+                                                              int Cout, int B, int H, int W, float *__restrict__ part) {
   constexpr int CP = CI + 8, DP = CO + 8, PATCH = PH * PW * CP, DYS = TH * TW * DP;
   extern __shared__ __align__(16) bf16 wg_sm[];
-  const int nci = Cin / CI;
+  const int Cin = in.channels(), nci = Cin / CI;
   const int co0 = (blockIdx.y / nci) * CO, ci0 = (blockIdx.y % nci) * CI;
   const int tiles_w = (W + TW - 1) / TW, tiles_h = (H + TH - 1) / TH, tiles = B * tiles_h * tiles_w;
   const int tap = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -302,7 +357,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(const bf16 *__rest
     const int b = r / (tiles_h * tiles_w);
     r -= b * tiles_h * tiles_w;
     const int i0 = (r / tiles_w) * TH, j0 = (r % tiles_w) * TW;
-    copy_patch<CI, WG_THREADS, PH>(patch, x, Cin, ci0, b, i0, j0, H, W);
+    copy_patch<CI, WG_THREADS, PH>(patch, in, ci0, b, i0, j0, H, W);
     for (int q = threadIdx.x; q < TH * TW * (CO / 8); q += WG_THREADS) {
       const int pix = q / (CO / 8), ch = q - pix * (CO / 8);
       const int ii = i0 + pix / TW, jj = j0 + pix % TW;
@@ -445,7 +500,7 @@ __global__ void k_flip_weights(const bf16 *__restrict__ p16, FlipLayers F, bf16 
   }
 }
 
-// ---- pooling, upsampling + concatenation ----
+// ---- pooling, and the gradients of the concatenation's parts ----
 // y[b, I, J, :] = mean of x over the 2 x 2 block; 8 channels per thread
 __global__ void k_pool(const bf16 *__restrict__ x, int C, int B, int H, int W, bf16 *__restrict__ y) {
   const int h = H / 2, w = W / 2, CH = C / 8;
@@ -490,25 +545,6 @@ __global__ void k_pool_back_add(const bf16 *__restrict__ dy, int C, int B, int H
 #pragma unroll
     for (int q = 0; q < 8; ++q) a[q] += 0.25f * d[q];
     *reinterpret_cast<uint4 *>(dst) = relu_mask8(pack8(a), *reinterpret_cast<const uint4 *>(ymask + (dst - dx)));
-  }
-}
-
-// c[b, i, j, :] = [u[b, i/2, j/2, 0:Cu], s[b, i, j, 0:Cs]]
-__global__ void k_upcat(const bf16 *__restrict__ u, int Cu, const bf16 *__restrict__ s, int Cs, int B, int H, int W,
-                        bf16 *__restrict__ c) {
-  const int C = Cu + Cs, CH = C / 8, h = H / 2, w = W / 2;
-  const long long n = (long long)B * H * W * CH;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int ch = (int)(k % CH);
-    long long p = k / CH;
-    const int j = (int)(p % W);
-    p /= W;
-    const int i = (int)(p % H);
-    const int b = (int)(p / H);
-    const int c0 = ch * 8;
-    const uint4 v = c0 < Cu ? *reinterpret_cast<const uint4 *>(u + (((size_t)b * h + i / 2) * w + j / 2) * Cu + c0)
-                            : *reinterpret_cast<const uint4 *>(s + (((size_t)b * H + i) * W + j) * Cs + c0 - Cu);
-    *reinterpret_cast<uint4 *>(c + (((size_t)b * H + i) * W + j) * C + c0) = v;
   }
 }
 
@@ -872,7 +908,7 @@ struct pism_gpu_unet {
   // activations (bf16) and their gradients
   bf16 *in16 = nullptr;
   bf16 *act[NLAYERS] = {};
-  bf16 *p1 = nullptr, *p2 = nullptr, *p3 = nullptr, *c3 = nullptr, *c2 = nullptr, *c1 = nullptr;
+  bf16 *p1 = nullptr, *p2 = nullptr, *p3 = nullptr;
   float *y = nullptr;
   bf16 *dd1 = nullptr, *dc1 = nullptr, *dd2 = nullptr, *de1 = nullptr, *dc2 = nullptr, *dd3 = nullptr,
        *de2 = nullptr, *dc3 = nullptr, *dbt = nullptr, *de3 = nullptr, *dp3 = nullptr, *de3a = nullptr,
@@ -929,15 +965,15 @@ inline long long pixels(int B, int H, int W, int l) { return (long long)B * (H >
 constexpr int UNET_SMS = 148;
 
 // one kernel form: its dynamic shared memory (granted when a handle is created) and its launch
-template <int CS, int NB, int MR, bool RESIDENT>
+template <int CS, int NB, int MR, bool RESIDENT, bool QUADS = false>
 struct Conv {
   static constexpr int smem = conv_smem<CS, NB, MR, RESIDENT>();
   static bool allow() {
-    return cudaFuncSetAttribute((const void *)k_conv3x3<CS, NB, MR, RESIDENT>,
+    return cudaFuncSetAttribute((const void *)k_conv3x3<CS, NB, MR, RESIDENT, QUADS>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
   }
-  static void launch(cudaStream_t s, const bf16 *x, int Cin, const bf16 *w, const float *bias, int relu,
-                     const bf16 *omask, bf16 *y, int Cout, int B, int H, int W) {
+  static void launch(cudaStream_t s, const ConvIn &in, const Quads &quads, const bf16 *w, const float *bias, int relu, const bf16 *omask,
+                     bf16 *y, int Cout, int B, int H, int W) {
     const int tiles = B * ((H + 8 * MR - 1) / (8 * MR)) * ((W + TW - 1) / TW), ny = Cout / NB;
     // Where the weights stay, as many CTAs as are resident at once, each with the same number of
     // tiles (a first tile cannot overlap its loads).  Several slices pipeline within a tile and
@@ -945,7 +981,8 @@ struct Conv {
     // neighbours' (forward of 1 x 408 x 408: 269 us; equal shares 289, pairs of tiles 310).
     const int most = std::max(1, UNET_SMS * std::min(3, (220 * 1024) / smem) / ny);
     const int per = RESIDENT ? (tiles + most - 1) / most : 1, ctas = (tiles + per - 1) / per;
-    k_conv3x3<CS, NB, MR, RESIDENT><<<dim3(ctas, ny), THREADS, smem, s>>>(x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    k_conv3x3<CS, NB, MR, RESIDENT, QUADS><<<dim3(ctas, ny), THREADS, smem, s>>>(in, quads, w, bias, relu, omask, y, Cout,
+                                                                                 B, H, W);
   }
 };
 template <int CI, int CO>
@@ -955,51 +992,80 @@ struct Wgrad {
     return cudaFuncSetAttribute((const void *)k_conv3x3_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem) == cudaSuccess;
   }
-  static void launch(cudaStream_t s, const bf16 *x, int Cin, const bf16 *dy, int Cout, int B, int H, int W, int ctas,
+  static void launch(cudaStream_t s, const ConvIn &in, const bf16 *dy, int Cout, int B, int H, int W, int ctas,
                      float *part) {
-    k_conv3x3_wgrad<CI, CO><<<dim3(ctas, (Cout / CO) * (Cin / CI)), WG_THREADS, smem, s>>>(x, Cin, dy, Cout, B, H, W,
-                                                                                          part);
+    k_conv3x3_wgrad<CI, CO><<<dim3(ctas, (Cout / CO) * (in.channels() / CI)), WG_THREADS, smem, s>>>(in, dy, Cout, B, H,
+                                                                                                    W, part);
   }
 };
 bool allow_kernels() {
   return Conv<32, 32, 2, true>::allow() && Conv<32, 32, 2, false>::allow() && Conv<32, 32, 1, true>::allow() &&
-         Conv<32, 32, 1, false>::allow() && Conv<16, 32, 2, true>::allow() && Conv<16, 32, 1, true>::allow() &&
+         Conv<32, 32, 2, true, true>::allow() && Conv<32, 32, 2, false, true>::allow() && Conv<32, 32, 1, false>::allow() && Conv<16, 32, 2, true>::allow() && Conv<16, 32, 1, true>::allow() &&
          Wgrad<32, 32>::allow() && Wgrad<32, 16>::allow() && Wgrad<16, 16>::allow();
 }
 
-// 16 x 16 pixels where that leaves every SM a CTA, else 8 x 16; the weights stay in shared memory
-// where the layer is one slice
-void conv(cudaStream_t s, const bf16 *x, int Cin, const bf16 *w, const float *bias, int relu, const bf16 *omask,
+// whether a layer's tiles are 16 x 16 pixels: where that leaves every SM a CTA; else 8 x 16
+bool tall_tiles(int Cout, int B, int H, int W) {
+  return (long long)B * ((H + 15) / 16) * ((W + TW - 1) / TW) * (Cout / 32) >= UNET_SMS;
+}
+
+// the weights stay in shared memory where the layer is one slice
+void conv(cudaStream_t s, const ConvIn &in, const bf16 *w, const float *bias, int relu, const bf16 *omask,
           bf16 *y, int Cout, int B, int H, int W) {
-  const bool tall = (long long)B * ((H + 15) / 16) * ((W + TW - 1) / TW) * (Cout / 32) >= UNET_SMS;
+  const int Cin = in.channels();
+  const bool tall = tall_tiles(Cout, B, H, W);
+  const Quads none{};
   if (Cin == 16) {
-    if (tall) Conv<16, 32, 2, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
-    else Conv<16, 32, 1, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    if (tall) Conv<16, 32, 2, true>::launch(s, in, none, w, bias, relu, omask, y, Cout, B, H, W);
+    else Conv<16, 32, 1, true>::launch(s, in, none, w, bias, relu, omask, y, Cout, B, H, W);
   } else if (Cin == 32) {
-    if (tall) Conv<32, 32, 2, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
-    else Conv<32, 32, 1, true>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    if (tall) Conv<32, 32, 2, true>::launch(s, in, none, w, bias, relu, omask, y, Cout, B, H, W);
+    else Conv<32, 32, 1, true>::launch(s, in, none, w, bias, relu, omask, y, Cout, B, H, W);
   } else {
-    if (tall) Conv<32, 32, 2, false>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
-    else Conv<32, 32, 1, false>::launch(s, x, Cin, w, bias, relu, omask, y, Cout, B, H, W);
+    if (tall) Conv<32, 32, 2, false>::launch(s, in, none, w, bias, relu, omask, y, Cout, B, H, W);
+    else Conv<32, 32, 1, false>::launch(s, in, none, w, bias, relu, omask, y, Cout, B, H, W);
   }
 }
 
+// a layer of 32 channels or more with tall tiles, and the 2 x 2 sums behind it
+void conv_quads(cudaStream_t s, const ConvIn &in, const Quads &quads, const bf16 *w, const float *bias, int relu, bf16 *y,
+                int Cout, int B, int H, int W) {
+  if (in.channels() == 32) Conv<32, 32, 2, true, true>::launch(s, in, quads, w, bias, relu, nullptr, y, Cout, B, H, W);
+  else Conv<32, 32, 2, false, true>::launch(s, in, quads, w, bias, relu, nullptr, y, Cout, B, H, W);
+}
+
 // dW: the channel blocks are halved while that still leaves SMs without a CTA
-void conv_wgrad(pism_gpu_unet *h, cudaStream_t s, const bf16 *x, int Cin, const bf16 *dy, int Cout, int B, int H, int W,
+void conv_wgrad(pism_gpu_unet *h, cudaStream_t s, const ConvIn &in, const bf16 *dy, int Cout, int B, int H, int W,
                 float *dW) {
+  const int Cin = in.channels();
   const int tiles = B * ((H + TH - 1) / TH) * ((W + TW - 1) / TW);
   const int ctas = std::min(tiles, WG_MAX_CTAS);
   const int blocks = ctas * (Cout / 32) * std::max(1, Cin / 32);   // with blocks of 32 x 32
   const bool half = blocks < 2 * UNET_SMS, quarter = blocks < UNET_SMS;
   if (Cin % 32 != 0 || quarter) {   // 16 input channels: the first layer only, one block of 32 x 32
-    Wgrad<16, 16>::launch(s, x, Cin, dy, Cout, B, H, W, ctas, h->wg_part);
+    Wgrad<16, 16>::launch(s, in, dy, Cout, B, H, W, ctas, h->wg_part);
   } else if (half) {
-    Wgrad<32, 16>::launch(s, x, Cin, dy, Cout, B, H, W, ctas, h->wg_part);
+    Wgrad<32, 16>::launch(s, in, dy, Cout, B, H, W, ctas, h->wg_part);
   } else {
-    Wgrad<32, 32>::launch(s, x, Cin, dy, Cout, B, H, W, ctas, h->wg_part);
+    Wgrad<32, 32>::launch(s, in, dy, Cout, B, H, W, ctas, h->wg_part);
   }
   const int n = 9 * Cout * Cin;
   k_reduce_parts<<<grid_for(n), 256, 0, s>>>(h->wg_part, ctas, n, dW);
+}
+
+// what layer l reads: an activation, pooled where a level begins, or the decoder's concatenation of
+// the level below and the skip
+ConvIn input_of(const pism_gpu_unet *h, int l) {
+  switch (l) {
+    case 0: return {h->in16, nullptr, LAYERS[0].cin, 0};
+    case 2: return {h->p1, nullptr, LAYERS[2].cin, 0};
+    case 4: return {h->p2, nullptr, LAYERS[4].cin, 0};
+    case 6: return {h->p3, nullptr, LAYERS[6].cin, 0};
+    case 7: return {h->act[5], h->act[6], LAYERS[5].cout, LAYERS[6].cout};
+    case 8: return {h->act[3], h->act[7], LAYERS[3].cout, LAYERS[7].cout};
+    case 9: return {h->act[1], h->act[8], LAYERS[1].cout, LAYERS[8].cout};
+    default: return {h->act[l - 1], nullptr, LAYERS[l].cin, 0};
+  }
 }
 
 // layer l's partial bias gradients; the sums follow in one launch for all layers
@@ -1014,6 +1080,24 @@ void bias_grad(pism_gpu_unet *h, int l, const bf16 *dy, long long P) {
   k_bias_grad<<<f.nparts[l], 256, 0, h->stream>>>(dy, C, P, part);
 }
 
+cudaError_t layer_back(pism_gpu_unet *h, int l, const bf16 *dY, bf16 *dX, const bf16 *xmask, int B, int H, int W,
+                       const Quads *split);
+
+// Layer l backward where its input is a concatenation: the gradients of the upsampled part (du, masked
+// by its layer's ReLU) and of the skip (ds); dc takes the concatenation's where the tiles are not tall
+cudaError_t concat_back(pism_gpu_unet *h, int l, const bf16 *dY, bf16 *du, bf16 *ds, bf16 *dc, int B, int H, int W) {
+  const ConvIn in = input_of(h, l);
+  if (tall_tiles(in.channels(), B, H, W)) {
+    const Quads split{du, in.up, in.Cu, in.Cu, 1.0f};
+    return layer_back(h, l, dY, ds, nullptr, B, H, W, &split);
+  }
+  const cudaError_t e = layer_back(h, l, dY, dc, nullptr, B, H, W, nullptr);
+  if (e != cudaSuccess) return e;
+  k_upcat_back<<<grid_for((long long)B * H * W * in.channels() / 8), 256, 0, h->stream>>>(dc, in.Cu, in.C, B, H, W, in.up, du,
+                                                                                     ds);
+  return cudaSuccess;
+}
+
 // the second stream and its events, from the first backward on: a network that only predicts has none
 bool side_stream(pism_gpu_unet *h) {
   if (h->side_done) return true;
@@ -1023,18 +1107,20 @@ bool side_stream(pism_gpu_unet *h) {
   return ok && cudaEventCreateWithFlags(&h->side_done, cudaEventDisableTiming) == cudaSuccess;
 }
 
-// Layer l backward: X input, dY given, masked by the layer's ReLU; dX (masked by xmask, its own
+// Layer l backward: dY given, masked by the layer's ReLU; dX (masked by xmask, its own
 // layer's output, where given) and db on the handle's stream, dW beside them on the second one: the
 // data gradients are the only chain, and with db behind them the streams are about as long
-// (16 x 128 x 128, kernel time: 450 and 410 us; 360 and 590 with all that is not a chain on the second).
-cudaError_t layer_back(pism_gpu_unet *h, int l, const bf16 *X, const bf16 *dY, bf16 *dX, const bf16 *xmask, int B, int H,
-                       int W) {
+// (with split, dX is the gradient of the skip and the other part's is made beside it; 16 x 128 x 128, kernel time: 450 and 410 us; 360 and 590 with all that is not a chain on the second).
+cudaError_t layer_back(pism_gpu_unet *h, int l, const bf16 *dY, bf16 *dX, const bf16 *xmask, int B, int H, int W,
+                       const Quads *split) {
   const LayerDef &L = LAYERS[l];
   cudaError_t e = cudaEventRecord(h->ready[l], h->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ready[l], 0);
   if (e != cudaSuccess) return e;
-  if (dX) conv(h->stream, dY, L.cout, h->flip + h->flip_off[l], nullptr, 0, xmask, dX, L.cin, B, H, W);
-  conv_wgrad(h, h->side, X, L.cin, dY, L.cout, B, H, W, h->grad + h->w_off[l]);
+  if (dX && split)
+    conv_quads(h->stream, {dY, nullptr, L.cout, 0}, *split, h->flip + h->flip_off[l], nullptr, 0, dX, L.cin, B, H, W);
+  else if (dX) conv(h->stream, {dY, nullptr, L.cout, 0}, h->flip + h->flip_off[l], nullptr, 0, xmask, dX, L.cin, B, H, W);
+  conv_wgrad(h, h->side, input_of(h, l), dY, L.cout, B, H, W, h->grad + h->w_off[l]);
   bias_grad(h, l, dY, (long long)B * H * W);
   return cudaSuccess;
 }
@@ -1139,9 +1225,6 @@ int pism_gpu_unet_create(int device, int max_batch, int max_h, int max_w, pism_g
   A(&h->p1, P(1) * 32);
   A(&h->p2, P(2) * 64);
   A(&h->p3, P(3) * 96);
-  A(&h->c3, P(2) * 224);
-  A(&h->c2, P(1) * 160);
-  A(&h->c1, P(0) * 96);
   AF(&h->y, P(0) * 2);
   A(&h->dd1, P(0) * 32);
   A(&h->dc1, P(0) * 96);
@@ -1187,7 +1270,7 @@ int pism_gpu_unet_destroy(pism_gpu_unet *h) {
   for (cudaEvent_t e : h->ready)
     if (e) cudaEventDestroy(e);
   for (float *p : {h->p32, h->grad, h->m, h->v, h->wg_part, h->small_part, h->bias_part, h->sums, h->y}) cudaFree(p);
-  for (bf16 *p : {h->p16, h->flip, h->in16, h->p1, h->p2, h->p3, h->c3, h->c2, h->c1, h->dd1, h->dc1, h->dd2, h->de1,
+  for (bf16 *p : {h->p16, h->flip, h->in16, h->p1, h->p2, h->p3, h->dd1, h->dc1, h->dd2, h->de1,
                   h->dc2, h->dd3, h->de2, h->dc3, h->dbt, h->de3, h->dp3, h->de3a, h->dp2, h->de2a, h->dp1, h->de1a})
     cudaFree(p);
   for (bf16 *p : h->act) cudaFree(p);
@@ -1235,26 +1318,30 @@ int pism_gpu_unet_forward(pism_gpu_unet *h, const float *input, int B, int H, in
   const long long P0 = (long long)B * H * W;
   const bf16 *w = h->p16;
   const float *p = h->p32;
-  auto L = [&](int l, const bf16 *x, int Hl, int Wl) {
-    conv(h->stream, x, LAYERS[l].cin, w + h->w_off[l], p + h->b_off[l], 1, nullptr, h->act[l], LAYERS[l].cout, B, Hl, Wl);
+  auto L = [&](int l) {
+    const int lev = LAYERS[l].level;
+    conv(h->stream, input_of(h, l), w + h->w_off[l], p + h->b_off[l], 1, nullptr, h->act[l], LAYERS[l].cout, B, H >> lev,
+         W >> lev);
+  };
+  // a level's last layer before the next one, and its 2 x 2 means
+  auto L_pooled = [&](int l, bf16 *pooled) {
+    const int lev = LAYERS[l].level, C = LAYERS[l].cout, Hl = H >> lev, Wl = W >> lev;
+    if (tall_tiles(C, B, Hl, Wl)) {
+      conv_quads(h->stream, input_of(h, l), {pooled, nullptr, C, 0, 0.25f}, w + h->w_off[l], p + h->b_off[l], 1, h->act[l], C,
+                 B, Hl, Wl);
+      return;
+    }
+    L(l);
+    k_pool<<<grid_for(pixels(B, H, W, lev + 1) * (C / 8)), 256, 0, h->stream>>>(h->act[l], C, B, Hl, Wl, pooled);
   };
   k_pack_input<<<grid_for(P0), 256, 0, h->stream>>>(input, P0, h->in16);
-  L(0, h->in16, H, W);
-  L(1, h->act[0], H, W);
-  k_pool<<<grid_for(pixels(B, H, W, 1) * 4), 256, 0, h->stream>>>(h->act[1], 32, B, H, W, h->p1);
-  L(2, h->p1, H / 2, W / 2);
-  L(3, h->act[2], H / 2, W / 2);
-  k_pool<<<grid_for(pixels(B, H, W, 2) * 8), 256, 0, h->stream>>>(h->act[3], 64, B, H / 2, W / 2, h->p2);
-  L(4, h->p2, H / 4, W / 4);
-  L(5, h->act[4], H / 4, W / 4);
-  k_pool<<<grid_for(pixels(B, H, W, 3) * 12), 256, 0, h->stream>>>(h->act[5], 96, B, H / 4, W / 4, h->p3);
-  L(6, h->p3, H / 8, W / 8);
-  k_upcat<<<grid_for(pixels(B, H, W, 2) * 28), 256, 0, h->stream>>>(h->act[6], 128, h->act[5], 96, B, H / 4, W / 4, h->c3);
-  L(7, h->c3, H / 4, W / 4);
-  k_upcat<<<grid_for(pixels(B, H, W, 1) * 20), 256, 0, h->stream>>>(h->act[7], 96, h->act[3], 64, B, H / 2, W / 2, h->c2);
-  L(8, h->c2, H / 2, W / 2);
-  k_upcat<<<grid_for(P0 * 12), 256, 0, h->stream>>>(h->act[8], 64, h->act[1], 32, B, H, W, h->c1);
-  L(9, h->c1, H, W);
+  L(0);
+  L_pooled(1, h->p1);
+  L(2);
+  L_pooled(3, h->p2);
+  L(4);
+  L_pooled(5, h->p3);
+  for (int l = 6; l < NLAYERS; ++l) L(l);
   k_head<<<grid_for(P0), 256, 0, h->stream>>>(h->act[9], p + h->head_off, P0, h->y);
   UCK(h, cudaGetLastError());
   if (output != h->y)
@@ -1296,27 +1383,22 @@ int pism_gpu_unet_backward(pism_gpu_unet *h, const float *target, const float *w
   h->few.n[NLAYERS] = NG;
   h->few.out[NLAYERS] = h->grad + h->head_off;
   // decoder (every gradient masked by its layer's ReLU where it is made)
-  UCK(h, layer_back(h, 9, h->c1, h->dd1, h->dc1, nullptr, B, H, W));
-  k_upcat_back<<<grid_for(P0 * 12), 256, 0, h->stream>>>(h->dc1, 64, 32, B, H, W, h->act[8], h->dd2, h->de1);
-  UCK(h, layer_back(h, 8, h->c2, h->dd2, h->dc2, nullptr, B, H / 2, W / 2));
-  k_upcat_back<<<grid_for(pixels(B, H, W, 1) * 20), 256, 0, h->stream>>>(h->dc2, 96, 64, B, H / 2, W / 2, h->act[7],
-                                                                       h->dd3, h->de2);
-  UCK(h, layer_back(h, 7, h->c3, h->dd3, h->dc3, nullptr, B, H / 4, W / 4));
-  k_upcat_back<<<grid_for(pixels(B, H, W, 2) * 28), 256, 0, h->stream>>>(h->dc3, 128, 96, B, H / 4, W / 4, h->act[6],
-                                                                       h->dbt, h->de3);
+  UCK(h, concat_back(h, 9, h->dd1, h->dd2, h->de1, h->dc1, B, H, W));
+  UCK(h, concat_back(h, 8, h->dd2, h->dd3, h->de2, h->dc2, B, H / 2, W / 2));
+  UCK(h, concat_back(h, 7, h->dd3, h->dbt, h->de3, h->dc3, B, H / 4, W / 4));
   // bottleneck and encoder
-  UCK(h, layer_back(h, 6, h->p3, h->dbt, h->dp3, nullptr, B, H / 8, W / 8));
+  UCK(h, layer_back(h, 6, h->dbt, h->dp3, nullptr, B, H / 8, W / 8, nullptr));
   k_pool_back_add<<<grid_for(pixels(B, H, W, 2) * 12), 256, 0, h->stream>>>(h->dp3, 96, B, H / 4, W / 4, h->act[5],
                                                                           h->de3);
-  UCK(h, layer_back(h, 5, h->act[4], h->de3, h->de3a, h->act[4], B, H / 4, W / 4));
-  UCK(h, layer_back(h, 4, h->p2, h->de3a, h->dp2, nullptr, B, H / 4, W / 4));
+  UCK(h, layer_back(h, 5, h->de3, h->de3a, h->act[4], B, H / 4, W / 4, nullptr));
+  UCK(h, layer_back(h, 4, h->de3a, h->dp2, nullptr, B, H / 4, W / 4, nullptr));
   k_pool_back_add<<<grid_for(pixels(B, H, W, 1) * 8), 256, 0, h->stream>>>(h->dp2, 64, B, H / 2, W / 2, h->act[3],
                                                                          h->de2);
-  UCK(h, layer_back(h, 3, h->act[2], h->de2, h->de2a, h->act[2], B, H / 2, W / 2));
-  UCK(h, layer_back(h, 2, h->p1, h->de2a, h->dp1, nullptr, B, H / 2, W / 2));
+  UCK(h, layer_back(h, 3, h->de2, h->de2a, h->act[2], B, H / 2, W / 2, nullptr));
+  UCK(h, layer_back(h, 2, h->de2a, h->dp1, nullptr, B, H / 2, W / 2, nullptr));
   k_pool_back_add<<<grid_for(P0 * 4), 256, 0, h->stream>>>(h->dp1, 32, B, H, W, h->act[1], h->de1);
-  UCK(h, layer_back(h, 1, h->act[0], h->de1, h->de1a, h->act[0], B, H, W));
-  UCK(h, layer_back(h, 0, h->in16, h->de1a, nullptr, nullptr, B, H, W));
+  UCK(h, layer_back(h, 1, h->de1, h->de1a, h->act[0], B, H, W, nullptr));
+  UCK(h, layer_back(h, 0, h->de1a, nullptr, nullptr, B, H, W, nullptr));
   k_reduce_few<<<FEW_SUMS, 256, 0, h->stream>>>(h->few);
   UCK(h, cudaEventRecord(h->side_done, h->side));
   UCK(h, cudaStreamWaitEvent(h->stream, h->side_done, 0));
