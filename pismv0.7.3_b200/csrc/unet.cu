@@ -183,8 +183,17 @@ constexpr int conv_smem() {
   return (2 * (8 * MR + 2) * PW + (RESIDENT ? 1 : 2) * 9 * NB) * (CS + 8) * (int)sizeof(bf16);
 }
 
+// As many CTAs an SM as the shared memory takes, at most three, and registers for them: unbounded, the
+// layers whose weights stay took 93 - 96, two CTAs of the three that their grid counts on, so a
+// second wave of long CTAs (32 to 96 channels of 16 x 128 x 128: 75 us, bounded 63); those with
+// several slices now use up to 120 registers.
+template <int CS, int NB, int MR, bool RESIDENT>
+constexpr int conv_ctas() {
+  return conv_smem<CS, NB, MR, RESIDENT>() * 3 <= 220 * 1024 ? 3 : 2;
+}
+
 template <int CS, int NB, int MR, bool RESIDENT, bool QUADS>
-__global__ void __launch_bounds__(THREADS) k_conv3x3(ConvIn in, Quads quads, const bf16 *__restrict__ w,
+__global__ void __launch_bounds__(THREADS, (conv_ctas<CS, NB, MR, RESIDENT>())) k_conv3x3(ConvIn in, Quads quads, const bf16 *__restrict__ w,
                                                      const float *__restrict__ bias, int relu,
                                                      const bf16 *__restrict__ omask, bf16 *__restrict__ y, int Cout,
                                                      int B, int H, int W) {
@@ -381,7 +390,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(ConvIn in, const b
     if (++fill == WG_STAGES) fill = 0;
     const bf16 *const patch = wg_sm + use * (PATCH + DYS), *const dys = patch + PATCH;
     if (++use == WG_STAGES) use = 0;
-#pragma unroll 2
+#pragma unroll 4
     for (int row = 0; row < TH; ++row) {
       uint32_t a[CO / 16][4];
 #pragma unroll
