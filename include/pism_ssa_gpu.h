@@ -232,6 +232,12 @@ const char *pism_gpu_ssa_last_error(const pism_gpu_ssa *h);
 /* Run the handle's work on a caller-owned cudaStream_t (NULL = the handle's own). */
 int pism_gpu_ssa_set_stream(pism_gpu_ssa *h, void *cuda_stream);
 
+/* The linear solves that run as one kernel (block-Jacobi BiCGStab with graphs >= 2, SSAFEM's
+ * conjugate gradients) wait between their blocks by reading a word until it is there.  A wait gives
+ * up after `reads` reads (1 .. 2^20, the default, about a second), and the solve then ends as a
+ * failed linear solve (PISM_GPU_SSA_EKSP).  For a program that wants such a failure sooner. */
+int pism_gpu_ssa_set_wait_limit(pism_gpu_ssa *h, int reads);
+
 /* Replace the configuration (e.g. epsilon_ssa set after init, as ssa_testi.cc:99-100). */
 int pism_gpu_ssa_set_config(pism_gpu_ssa *h, const pism_gpu_ssa_config *cfg);
 

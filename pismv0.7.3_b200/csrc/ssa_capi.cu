@@ -1174,6 +1174,17 @@ int pism_gpu_ssa_set_stream(pism_gpu_ssa *h, void *s) {
   return PISM_GPU_SSA_OK;
 }
 
+int pism_gpu_ssa_set_wait_limit(pism_gpu_ssa *h, int reads) {
+  if (!h) return PISM_GPU_SSA_EINVAL;
+  if (reads < 1 || reads > EX_SPIN_LIMIT)
+    return fail(h, PISM_GPU_SSA_EINVAL, "the wait limit must be in [1, %d]", EX_SPIN_LIMIT);
+  h->L.wait_limit = reads;
+  DeviceGuard dg(h->device);
+  if (h->sgraph.exec) cudaGraphExecDestroy(h->sgraph.exec);   // it holds the limit by value
+  h->sgraph = {};
+  return PISM_GPU_SSA_OK;
+}
+
 int pism_gpu_ssa_set_config(pism_gpu_ssa *h, const pism_gpu_ssa_config *cfg) {
   if (!h) return PISM_GPU_SSA_EINVAL;
   RET(check_config(h, cfg));

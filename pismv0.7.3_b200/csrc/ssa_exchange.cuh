@@ -12,7 +12,9 @@
 // decisions.
 //
 // The blocks wait for one another: the kernel is launched cooperatively, with no more blocks
-// than are resident at once, and every wait gives up after a bounded number of reads.
+// than are resident at once, and every wait gives up after a bounded number of reads.  A block that
+// gives up posts nothing more, a leading block no sum of a part it has not seen whole, so no block
+// takes a sum with a part missing for a sum: the others run out of reads in their turn.
 #pragma once
 
 #include "ssa_reduce.cuh"
@@ -20,7 +22,6 @@
 namespace pism_gpu {
 
 constexpr int EX_WORDS = 4;              // a slot: two values, 32 bytes
-constexpr int EX_SPIN_LIMIT = 1 << 20;   // reads of a word before a wait gives up (about a second)
 constexpr int EX_GROUPS = RED_THREADS / 32;
 
 // The slots of one kind of exchange: one per block, then EX_GROUPS for the leading blocks' sums.
@@ -28,6 +29,7 @@ constexpr int EX_GROUPS = RED_THREADS / 32;
 // has read this one's.  Zeroed before the kernel; rounds count from 1.
 struct ExSlots {
   unsigned long long *w;
+  int limit;   // reads of a word before a wait gives up
   __device__ __forceinline__ unsigned long long *block(int b) const { return w + (size_t)b * EX_WORDS; }
   __device__ __forceinline__ unsigned long long *group(int g) const { return w + (size_t)(gridDim.x + g) * EX_WORDS; }
 };
@@ -42,8 +44,8 @@ __device__ __forceinline__ void ex_put(unsigned long long *p, double v, unsigned
 }
 // the NV doubles of a slot, their loads in flight together; false when the wait gave up
 template <int NV>
-__device__ __forceinline__ bool ex_get(const unsigned long long *p, unsigned round, double (&v)[NV]) {
-  for (int it = 0; it < EX_SPIN_LIMIT; ++it) {
+__device__ __forceinline__ bool ex_get(const unsigned long long *p, unsigned round, int limit, double (&v)[NV]) {
+  for (int it = 0; it < limit; ++it) {
     unsigned long long w[NV][2];
 #pragma unroll
     for (int k = 0; k < NV; ++k)
@@ -69,6 +71,7 @@ __device__ __forceinline__ bool ex_get(const unsigned long long *p, unsigned rou
 struct ExNodes {
   unsigned long long *w;
   int nodes;
+  int limit;   // as for the slots
   __device__ __forceinline__ void put(int n, const double2 &v, unsigned round) const {
     ex_put(w + 2 * (size_t)n, v.x, round);
     ex_put(w + 2 * ((size_t)nodes + n), v.y, round);
@@ -76,7 +79,7 @@ struct ExNodes {
   // the values of M nodes, their loads in flight together; false when the wait gave up
   template <int M>
   __device__ __forceinline__ bool get(const int (&n)[M], unsigned round, double2 (&v)[M]) const {
-    for (int it = 0; it < EX_SPIN_LIMIT; ++it) {
+    for (int it = 0; it < limit; ++it) {
       unsigned long long q[M][4];
 #pragma unroll
       for (int m = 0; m < M; ++m)
@@ -132,7 +135,7 @@ __device__ __forceinline__ bool exchange_sum(double (&val)[NV], const ExSlots &s
     for (int v = 0; v < NV; ++v) acc[v] = 0.0;
     for (int b = 32 * g + lane; b < nb; b += RED_THREADS) {
       double x[NV] = {};
-      ok = ex_get<NV>(slots.block(b), round, x) && ok;
+      ok = ex_get<NV>(slots.block(b), round, slots.limit, x) && ok;
 #pragma unroll
       for (int v = 0; v < NV; ++v) acc[v] += x[v];
     }
@@ -152,13 +155,15 @@ __device__ __forceinline__ bool exchange_sum(double (&val)[NV], const ExSlots &s
     if (warp == 1 && (int)blockIdx.x < groups) {
       double acc[NV];
       gather(blockIdx.x, acc);
+      if (__all_sync(0xffffffffu, ok)) {   // else a slot is missing, and its zero is in the sum
 #pragma unroll
-      for (int v = 0; v < NV; ++v)
-        if (lane == v) ex_put(slots.group(blockIdx.x) + 2 * v, acc[v], round);
+        for (int v = 0; v < NV; ++v)
+          if (lane == v) ex_put(slots.group(blockIdx.x) + 2 * v, acc[v], round);
+      }
     }
     if (warp == 0) {
       double x[NV] = {};
-      if (lane < groups) ok = ex_get<NV>(slots.group(lane), round, x) && ok;
+      if (lane < groups) ok = ex_get<NV>(slots.group(lane), round, slots.limit, x) && ok;
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         double s = 0.0;

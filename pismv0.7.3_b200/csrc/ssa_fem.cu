@@ -675,8 +675,8 @@ bool launch_fem_cg_resident(const Launch &L, const FemProblem &P, FemState &S) {
   }
   if (cudaMemsetAsync(S.ex, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
   FemGrid G = fem_grid(P);
-  ExSlots sq{S.ex}, sr{S.ex + ws};
-  ExNodes zex{S.ex + 2 * ws, S.N};
+  ExSlots sq{S.ex, L.wait_limit}, sr{S.ex + ws, L.wait_limit};
+  ExNodes zex{S.ex + 2 * ws, S.N, L.wait_limit};
   const double *J = S.J;
   const double4 *dinv = S.dinv;
   const double2 *r = S.r, *z = S.z;

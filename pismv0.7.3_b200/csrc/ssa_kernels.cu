@@ -1128,12 +1128,12 @@ bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, co
   const size_t slots = ex_slot_words(tm.tiles), nodes = ex_node_words(N), words = bicg_exchange_words(g, tm.tiles);
   if (cudaMemsetAsync(E.w, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
   BicgResident ex;
-  ex.a.w = E.w;
-  ex.b.w = E.w + slots;
-  ex.c.w = E.w + 2 * slots;
-  ex.v = ExNodes{E.w + 3 * slots, N};
-  ex.t = ExNodes{E.w + 3 * slots + nodes, N};
-  ex.terms = ExNodes{E.w + 3 * slots + 2 * nodes, N};
+  ex.a = ExSlots{E.w, L.wait_limit};
+  ex.b = ExSlots{E.w + slots, L.wait_limit};
+  ex.c = ExSlots{E.w + 2 * slots, L.wait_limit};
+  ex.v = ExNodes{E.w + 3 * slots, N, L.wait_limit};
+  ex.t = ExNodes{E.w + 3 * slots + nodes, N, L.wait_limit};
+  ex.terms = ExNodes{E.w + 3 * slots + 2 * nodes, N, L.wait_limit};
   GridDev gd = g;
   StencilConst s = stencil_const(g, f);
   const uint32_t *flags = f.flags;
