@@ -16,6 +16,7 @@
 #include "pism_unet_gpu.h"
 #include "ssa_internal.h"
 #include "ssa_fem.h"
+#include "ssa_march_plan.h"
 #include "unet_internal.h"
 
 using namespace pism_gpu;
@@ -1106,7 +1107,8 @@ int pism_gpu_ssa_create(const pism_gpu_grid *grid, const pism_gpu_ssa_config *cf
     if (mg_allocate(h->mg, h->N) != 0) return bail(PISM_GPU_SSA_ENOMEM);
     if (cudaMemsetAsync(h->mg.singular, 0, sizeof(int), h->stream) != cudaSuccess) return bail(PISM_GPU_SSA_ECUDA);
   }
-  AL(h->partials, (size_t)h->L.max_blocks * 8); AL(h->ticket, 1); AL(h->norm_dev, 2); AL(h->zd_dev, 1);
+  AL(h->partials, std::max((size_t)h->L.max_blocks * 8, (size_t)march_partials(grid->Mx, grid->My, sms)));
+  AL(h->ticket, 1); AL(h->norm_dev, 2); AL(h->zd_dev, 1);
 #undef AL
   if (cudaMallocHost((void **)&h->st_host, sizeof(KState)) != cudaSuccess ||
       cudaMallocHost((void **)&h->norm_host, 2 * sizeof(double)) != cudaSuccess ||

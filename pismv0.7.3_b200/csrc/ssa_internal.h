@@ -60,7 +60,7 @@ constexpr int EX_SPIN_LIMIT = 1 << 20;   // reads of a word: about a second
 struct Launch {
   cudaStream_t stream;
   int max_blocks;        // resident blocks (SM count x blocks per SM)
-  double *partials;      // per-block partial sums (>= max_blocks * 8)
+  double *partials;      // per-block partial sums (max_blocks * 8, or march_partials() where that is more)
   unsigned *ticket;      // last-block ticket, kept at 0 between kernels
   long long *count;      // kernel-launch counter (may be null)
   int wait_limit = EX_SPIN_LIMIT;   // reads of an exchange word before a block's wait gives up (ssa_exchange.cuh)

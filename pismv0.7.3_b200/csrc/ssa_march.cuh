@@ -20,44 +20,12 @@
 
 #include "ssa_fine32.cuh"
 #include "ssa_krylov32.cuh"
+#include "ssa_march_plan.h"
 #include "ssa_pdl.cuh"
 
 namespace pism_gpu {
 
-constexpr int MARCH_WARPS = 4, MARCH_THREADS = 32 * MARCH_WARPS;
-
-// strips of W = 32 - 2 halo columns, chunks of R rows; one strip's chunk is one warp's work
-struct MarchPlan {
-  int strips, R, chunks, blocks;
-};
-
-// All warps are resident at once (k blocks of four warps on each SM), so a pass takes R + extra
-// rows, each of latency + k issue (relative units, fitted to the passes' times at 801^2 with k
-// = 1 .. 4: 26.9, 14.0, 11.2, 9.0 us for the restriction, 45.7, 27.8, 21.3, 17.4 us for the
-// smoothing with the apply).  A row is a chain of about 200 - 300 dependent instructions, so
-// more warps cost a row little and shorten the chunks: k is 4 but on small grids, where R is
-// already at its least.
-inline MarchPlan march_plan(int Mx, int My, int halo, int extra, int align, int sms, int latency, int issue) {
-  const int W = 32 - 2 * halo;
-  MarchPlan best{};
-  long long least = -1;
-  for (int k = 1; k <= 4; ++k) {
-    MarchPlan p;
-    p.strips = (My + W - 1) / W;
-    const int most = k * sms * MARCH_WARPS / p.strips;   // chunks that fit in one wave
-    if (most < 1 && k < 4) continue;
-    const int chunks = most < 1 ? 1 : (most < Mx ? most : Mx);
-    p.R = ((Mx + chunks - 1) / chunks + align - 1) / align * align;
-    p.chunks = (Mx + p.R - 1) / p.R;
-    p.blocks = (p.strips * p.chunks + MARCH_WARPS - 1) / MARCH_WARPS;
-    const long long cost = (p.R + extra) * (long long)(latency + k * issue);
-    if (least < 0 || cost < least) {
-      least = cost;
-      best = p;
-    }
-  }
-  return best;
-}
+constexpr int MARCH_THREADS = 32 * MARCH_WARPS;
 
 // this warp's strip and chunk
 struct MarchTask {

@@ -1716,7 +1716,7 @@ static void vcycle(const Launch &Lc, const GridDev &g, const Fields &f, const MG
 #undef MG0P
     } else {
       static_assert(std::is_same<ZV, float2>::value, "the fused pass produces FP32 iterates");
-      const MarchPlan m = march_plan(g.Mx, g.My, 2, 4, 1, sms, 16, 1);
+      const MarchPlan m = march_plan_apply(g.Mx, g.My, sms);
 #define MG0PA(AX, AY) [&] { launch_pdl(Lc, k_mg0_post_apply<AX, AY, BA, EPI>, m.blocks, MARCH_THREADS, 0, F, b, omega, corr, C.My, C.x, m, z, epi); }
       dispatch_ax(H.fine_ax, H.fine_ay, MG0PA(2, 2), MG0PA(2, 1), MG0PA(1, 2), MG0PA(1, 1));
 #undef MG0PA
