@@ -21,15 +21,27 @@
 
 namespace pism_gpu {
 
+// How many reads of a word a wait takes before it gives up: the default, known to the compiler, or a
+// caller's.  With every wait on a number it does not know, the resident conjugate gradients on 241^2
+// nodes (227 blocks, two an SM) took 2.1 ms in place of 1.3, so a kernel has both forms.
+struct ExDefaultLimit {
+  static __device__ __forceinline__ constexpr int reads() { return EX_SPIN_LIMIT; }
+};
+struct ExGivenLimit {
+  int n;
+  __device__ __forceinline__ int reads() const { return n; }
+};
+
 constexpr int EX_WORDS = 4;              // a slot: two values, 32 bytes
 constexpr int EX_GROUPS = RED_THREADS / 32;
 
 // The slots of one kind of exchange: one per block, then EX_GROUPS for the leading blocks' sums.
 // Kinds alternate within an iteration, so that a block may post the next round's before another
 // has read this one's.  Zeroed before the kernel; rounds count from 1.
+template <class Limit>
 struct ExSlots {
   unsigned long long *w;
-  int limit;   // reads of a word before a wait gives up
+  Limit limit;
   __device__ __forceinline__ unsigned long long *block(int b) const { return w + (size_t)b * EX_WORDS; }
   __device__ __forceinline__ unsigned long long *group(int g) const { return w + (size_t)(gridDim.x + g) * EX_WORDS; }
 };
@@ -43,9 +55,9 @@ __device__ __forceinline__ void ex_put(unsigned long long *p, double v, unsigned
                : "memory");
 }
 // the NV doubles of a slot, their loads in flight together; false when the wait gave up
-template <int NV>
-__device__ __forceinline__ bool ex_get(const unsigned long long *p, unsigned round, int limit, double (&v)[NV]) {
-  for (int it = 0; it < limit; ++it) {
+template <int NV, class Limit>
+__device__ __forceinline__ bool ex_get(const unsigned long long *p, unsigned round, Limit limit, double (&v)[NV]) {
+  for (int it = 0; it < limit.reads(); ++it) {
     unsigned long long w[NV][2];
 #pragma unroll
     for (int k = 0; k < NV; ++k)
@@ -68,10 +80,11 @@ __device__ __forceinline__ bool ex_get(const unsigned long long *p, unsigned rou
 
 // Vector values (two doubles) by node, in two planes of tagged words, so that a warp's nodes are
 // whole sectors: the components of node n at w[2 n] and w[2 (nodes + n)].
+template <class Limit>
 struct ExNodes {
   unsigned long long *w;
   int nodes;
-  int limit;   // as for the slots
+  Limit limit;
   __device__ __forceinline__ void put(int n, const double2 &v, unsigned round) const {
     ex_put(w + 2 * (size_t)n, v.x, round);
     ex_put(w + 2 * ((size_t)nodes + n), v.y, round);
@@ -79,7 +92,7 @@ struct ExNodes {
   // the values of M nodes, their loads in flight together; false when the wait gave up
   template <int M>
   __device__ __forceinline__ bool get(const int (&n)[M], unsigned round, double2 (&v)[M]) const {
-    for (int it = 0; it < limit; ++it) {
+    for (int it = 0; it < limit.reads(); ++it) {
       unsigned long long q[M][4];
 #pragma unroll
       for (int m = 0; m < M; ++m)
@@ -110,8 +123,8 @@ inline size_t ex_node_words(int nodes) { return 4 * (size_t)nodes; }
 
 // Sum NV values over the first nb blocks of the grid; every thread of the grid gets the totals.
 // False (in every thread of the block) when a wait gave up; the other blocks then give up too.
-template <int NV>
-__device__ __forceinline__ bool exchange_sum(double (&val)[NV], const ExSlots &slots, unsigned round,
+template <int NV, class Limit>
+__device__ __forceinline__ bool exchange_sum(double (&val)[NV], const ExSlots<Limit> &slots, unsigned round,
                                              double (&tot)[NV], int nb = gridDim.x) {
   static_assert(2 * NV <= EX_WORDS, "a slot holds two values");
   constexpr int WARPS = RED_THREADS / 32;

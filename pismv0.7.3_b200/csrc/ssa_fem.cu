@@ -14,6 +14,7 @@
 // its four nodes.  The Jacobian is stored as 9 neighbour blocks of 2 x 2 per node,
 // structure-of-arrays ([36][N]), which the CG apply reads coalesced.
 #include <algorithm>
+#include <climits>
 
 #include "ssa_exchange.cuh"
 #include "ssa_fem.h"
@@ -382,11 +383,12 @@ __global__ void __launch_bounds__(NTF) k_cg_direction(int N, const double2 *z, d
 constexpr int CG_RUN = NTF + 2;
 constexpr int CG_SMEM = 36 * NTF * (int)sizeof(double) + 3 * CG_RUN * (int)sizeof(double2);
 
+template <class Limit>
 __global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double *__restrict__ J,
                                                         const double4 *__restrict__ dinv,
                                                         const double2 *__restrict__ r0, const double2 *__restrict__ z0,
-                                                        double2 *__restrict__ x_out, ExNodes zex, FemCG *cg,
-                                                        ExSlots slots_q, ExSlots slots_r) {
+                                                        double2 *__restrict__ x_out, ExNodes<Limit> zex, FemCG *cg,
+                                                        ExSlots<Limit> slots_q, ExSlots<Limit> slots_r) {
   extern __shared__ __align__(16) double Js[];   // [36][NTF], then the three runs of p
   double2 *const P = reinterpret_cast<double2 *>(Js + 36 * NTF);
   const int N = G.Mx * G.My, tid = threadIdx.x, s0 = blockIdx.x * NTF, n = s0 + tid;
@@ -503,7 +505,7 @@ __global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double 
       const int nodes[5] = {above, below, apart[0] >= 0 ? apart[0] : above, apart[1] >= 0 ? apart[1] : above,
                             end >= 0 ? end : above};
       double2 v[5];
-      ok = zex.get<5>(nodes, round, v);
+      ok = zex.template get<5>(nodes, round, v);
       P[tid] = direction(v[0], P[tid]);
       P[2 * CG_RUN + tid] = direction(v[1], P[2 * CG_RUN + tid]);
       pa = direction(v[2], pa);
@@ -512,7 +514,7 @@ __global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double 
     } else {
       const int nodes[2] = {above, below};
       double2 v[2];
-      ok = zex.get<2>(nodes, round, v);
+      ok = zex.template get<2>(nodes, round, v);
       P[tid] = direction(v[0], P[tid]);
       P[2 * CG_RUN + tid] = direction(v[1], P[2 * CG_RUN + tid]);
     }
@@ -660,11 +662,26 @@ void launch_fem_cg_iterations(const Launch &L, const FemProblem &P, const FemSta
   }
 }
 
+template <class Limit>
+static cudaError_t run_cg_resident(const Launch &L, FemGrid G, FemState &S, int nb, Limit limit) {
+  const size_t ws = ex_slot_words(nb);
+  ExSlots<Limit> sq{S.ex, limit}, sr{S.ex + ws, limit};
+  ExNodes<Limit> zex{S.ex + 2 * ws, S.N, limit};
+  const double *J = S.J;
+  const double4 *dinv = S.dinv;
+  const double2 *r = S.r, *z = S.z;
+  void *args[] = {&G, &J, &dinv, &r, &z, &S.du, &zex, &S.cg, &sq, &sr};
+  return cudaLaunchCooperativeKernel((const void *)k_cg_resident<Limit>, dim3(nb), dim3(NTF), args, CG_SMEM, L.stream);
+}
+
 bool launch_fem_cg_resident(const Launch &L, const FemProblem &P, FemState &S) {
   const int nb = (S.N + NTF - 1) / NTF;
   if (!S.cg_resident_blocks) {   // once per grid: what the device holds at once
-    cudaFuncSetAttribute((const void *)k_cg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM);
-    S.cg_resident_blocks = std::max(1, resident_blocks((const void *)k_cg_resident, NTF, CG_SMEM));
+    S.cg_resident_blocks = INT_MAX;
+    for (const void *k : {(const void *)k_cg_resident<ExDefaultLimit>, (const void *)k_cg_resident<ExGivenLimit>}) {
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_SMEM);
+      S.cg_resident_blocks = std::min(S.cg_resident_blocks, std::max(1, resident_blocks(k, NTF, CG_SMEM)));
+    }
   }
   // one thread a node: the order of the sums is that of the kernels below L.max_blocks blocks
   if (nb > S.cg_resident_blocks || nb > L.max_blocks) return false;
@@ -674,15 +691,9 @@ bool launch_fem_cg_resident(const Launch &L, const FemProblem &P, FemState &S) {
     return false;
   }
   if (cudaMemsetAsync(S.ex, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
-  FemGrid G = fem_grid(P);
-  ExSlots sq{S.ex, L.wait_limit}, sr{S.ex + ws, L.wait_limit};
-  ExNodes zex{S.ex + 2 * ws, S.N, L.wait_limit};
-  const double *J = S.J;
-  const double4 *dinv = S.dinv;
-  const double2 *r = S.r, *z = S.z;
-  void *args[] = {&G, &J, &dinv, &r, &z, &S.du, &zex, &S.cg, &sq, &sr};
-  if (cudaLaunchCooperativeKernel((const void *)k_cg_resident, dim3(nb), dim3(NTF), args, CG_SMEM, L.stream) !=
-      cudaSuccess) {
+  const cudaError_t e = L.wait_limit == EX_SPIN_LIMIT ? run_cg_resident(L, fem_grid(P), S, nb, ExDefaultLimit{})
+                                                      : run_cg_resident(L, fem_grid(P), S, nb, ExGivenLimit{L.wait_limit});
+  if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -740,18 +740,20 @@ __global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *phat_, cons
 // 22 Picard steps), one B200: 27.2 ms with the five kernels, 10.2 ms with this one.  Grids of
 // more tiles than SMs (37 888 cells at most) keep the five kernels.
 // ---------------------------------------------------------------------------
+template <class Limit>
 struct BicgResident {
-  ExSlots a, b, c;      // the slots of (rhat, v); (t, s), (t, t); (rhat, r), (r, r)
-  ExNodes v, t, terms;  // v and t of the tiles' border cells; the last sum's terms by cell
+  ExSlots<Limit> a, b, c;      // the slots of (rhat, v); (t, s), (t, t); (rhat, r), (r, r)
+  ExNodes<Limit> v, t, terms;  // v and t of the tiles' border cells; the last sum's terms by cell
 };
 
+template <class Limit>
 __global__ void __launch_bounds__(NT, 1) k_bicg_resident(GridDev g, TileMap tm, StencilConst sc,
                                                          const uint32_t *__restrict__ flags,
                                                          const double2 *__restrict__ nuH,
                                                          const double *__restrict__ beta_,
                                                          const double4 *__restrict__ dinv,
-                                                         const double2 *__restrict__ r0, double2 *x_, BicgResident ex,
-                                                         KState *st) {
+                                                         const double2 *__restrict__ r0, double2 *x_,
+                                                         BicgResident<Limit> ex, KState *st) {
   __shared__ HaloTile<double2> xT, nT;
   const int N = g.Mx * g.My, tid = threadIdx.x, ti = tid >> 5, tj = tid & 31;
   const int i0 = (blockIdx.x / tm.tiles_j) * TI, j0 = (blockIdx.x % tm.tiles_j) * TJ, i = i0 + ti, j = j0 + tj;
@@ -790,17 +792,17 @@ __global__ void __launch_bounds__(NT, 1) k_bicg_resident(GridDev g, TileMap tm, 
   const int maxit = st->maxit, nlin = (N + NT - 1) / NT;
   int its = st->iter, done = st->done, status = st->status;
   // the owners' values of the cells this thread keeps: past the edge (own), in the halo (halo)
-  auto copies = [&](const ExNodes &e, unsigned round, double2 &own, double2 &halo) {
+  auto copies = [&](const ExNodes<Limit> &e, unsigned round, double2 &own, double2 &halo) {
     bool ok = true;
     double2 w[1];
     if (need_k) {
       const int q[1] = {k};
-      ok = e.get<1>(q, round, w);
+      ok = e.template get<1>(q, round, w);
       own = w[0];
     }
     if (need_h) {
       const int q[1] = {h};
-      ok = e.get<1>(q, round, w) && ok;
+      ok = e.template get<1>(q, round, w) && ok;
       halo = w[0];
     }
     return ok;
@@ -899,7 +901,7 @@ __global__ void __launch_bounds__(NT, 1) k_bicg_resident(GridDev g, TileMap tm, 
     if (kl < N) {
       const int q[1] = {kl};
       double2 w[1];
-      ok = ex.terms.get<1>(q, round, w) && ok;
+      ok = ex.terms.template get<1>(q, round, w) && ok;
       acc2[0] = w[0].x;
       acc2[1] = w[0].y;
     }
@@ -1108,7 +1110,9 @@ static size_t bicg_exchange_words(const GridDev &g, int tiles) {
 
 bool bicg_resident_fits(const Launch &L, const GridDev &g, KrylovExchange &E) {
   const TileMap tm = make_tiles(g);
-  if (!E.capacity) E.capacity = std::max(1, resident_blocks((const void *)k_bicg_resident, NT, 0));
+  if (!E.capacity)
+    E.capacity = std::max(1, std::min(resident_blocks((const void *)k_bicg_resident<ExDefaultLimit>, NT, 0),
+                                      resident_blocks((const void *)k_bicg_resident<ExGivenLimit>, NT, 0)));
   // one cell a thread in both orders: below L.max_blocks blocks the five kernels add alike
   if (tm.tiles > E.capacity || tm.tiles > L.max_blocks) return false;
   if (!E.w &&
@@ -1120,20 +1124,18 @@ bool bicg_resident_fits(const Launch &L, const GridDev &g, KrylovExchange &E) {
   return true;
 }
 
-bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
-                          KrylovExchange &E) {
+template <class Limit>
+static cudaError_t run_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+                                     unsigned long long *w, Limit limit) {
   const int N = g.Mx * g.My;
-  if (!bicg_resident_fits(L, g, E)) return false;
   TileMap tm = make_tiles(g);
-  const size_t slots = ex_slot_words(tm.tiles), nodes = ex_node_words(N), words = bicg_exchange_words(g, tm.tiles);
-  if (cudaMemsetAsync(E.w, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
-  BicgResident ex;
-  ex.a = ExSlots{E.w, L.wait_limit};
-  ex.b = ExSlots{E.w + slots, L.wait_limit};
-  ex.c = ExSlots{E.w + 2 * slots, L.wait_limit};
-  ex.v = ExNodes{E.w + 3 * slots, N, L.wait_limit};
-  ex.t = ExNodes{E.w + 3 * slots + nodes, N, L.wait_limit};
-  ex.terms = ExNodes{E.w + 3 * slots + 2 * nodes, N, L.wait_limit};
+  const size_t slots = ex_slot_words(tm.tiles), nodes = ex_node_words(N);
+  BicgResident<Limit> ex{{w, limit},
+                         {w + slots, limit},
+                         {w + 2 * slots, limit},
+                         {w + 3 * slots, N, limit},
+                         {w + 3 * slots + nodes, N, limit},
+                         {w + 3 * slots + 2 * nodes, N, limit}};
   GridDev gd = g;
   StencilConst s = stencil_const(g, f);
   const uint32_t *flags = f.flags;
@@ -1142,8 +1144,17 @@ bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, co
   const double4 *dinv = K.dinv;
   KState *st = K.st;
   void *args[] = {&gd, &tm, &s, &flags, &nuH, &beta, &dinv, &r, &x, &ex, &st};
-  if (cudaLaunchCooperativeKernel((const void *)k_bicg_resident, dim3(tm.tiles), dim3(NT), args, 0, L.stream) !=
-      cudaSuccess) {
+  return cudaLaunchCooperativeKernel((const void *)k_bicg_resident<Limit>, dim3(tm.tiles), dim3(NT), args, 0, L.stream);
+}
+
+bool launch_bicg_resident(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+                          KrylovExchange &E) {
+  if (!bicg_resident_fits(L, g, E)) return false;
+  const size_t words = bicg_exchange_words(g, make_tiles(g).tiles);
+  if (cudaMemsetAsync(E.w, 0, sizeof(unsigned long long) * words, L.stream) != cudaSuccess) return false;
+  const cudaError_t e = L.wait_limit == EX_SPIN_LIMIT ? run_bicg_resident(L, g, f, K, x, E.w, ExDefaultLimit{})
+                                                      : run_bicg_resident(L, g, f, K, x, E.w, ExGivenLimit{L.wait_limit});
+  if (e != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

@@ -17,8 +17,8 @@ __device__ double value_of(int block, int thread, int v, unsigned round) {
   return (double)((block + 1) * (v + 1) * (int)round + thread);   // whole numbers: every order adds alike
 }
 
-template <int NV>
-__global__ void __launch_bounds__(RED_THREADS) k_check(ExSlots a, ExSlots b, int absent, int *rounds, double *sums) {
+template <int NV, class Limit>
+__global__ void __launch_bounds__(RED_THREADS) k_check(ExSlots<Limit> a, ExSlots<Limit> b, int absent, int *rounds, double *sums) {
   if ((int)blockIdx.x == absent) return;
   for (unsigned round = 1; round <= ROUNDS; ++round) {
     double x[NV], tot[NV];
@@ -31,8 +31,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_check(ExSlots a, ExSlots b, int
   }
 }
 
-template <int NV>
-static int run(int blocks, int absent, int limit) {
+template <int NV, class Limit>
+static int run(int blocks, int absent, Limit limit) {
   const size_t words = ex_slot_words(blocks);
   unsigned long long *w = nullptr;
   int *rounds = nullptr;
@@ -43,10 +43,11 @@ static int run(int blocks, int absent, int limit) {
     return 1;
   cudaMemset(w, 0, 2 * words * sizeof(*w));
   cudaMemset(rounds, 0, blocks * sizeof(int));
-  ExSlots a{w, limit}, b{w + words, limit};
+  ExSlots<Limit> a{w, limit}, b{w + words, limit};
   void *args[] = {&a, &b, &absent, &rounds, &sums};
-  if (blocks > resident_blocks((const void *)k_check<NV>, RED_THREADS, 0) ||
-      cudaLaunchCooperativeKernel((const void *)k_check<NV>, dim3(blocks), dim3(RED_THREADS), args, 0, 0) != cudaSuccess ||
+  const void *kernel = (const void *)k_check<NV, Limit>;
+  if (blocks > resident_blocks(kernel, RED_THREADS, 0) ||
+      cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(RED_THREADS), args, 0, 0) != cudaSuccess ||
       cudaDeviceSynchronize() != cudaSuccess)
     return 1;
   int done[ROUNDS] = {}, right = 1;
@@ -72,6 +73,8 @@ static int run(int blocks, int absent, int limit) {
 int main() {
   int blocks, absent, limit, one;
   while (scanf("%d %d %d %d", &blocks, &absent, &limit, &one) == 4)
-    if (one ? run<1>(blocks, absent, limit) : run<2>(blocks, absent, limit)) return 1;
+    if (limit == EX_SPIN_LIMIT ? (one ? run<1>(blocks, absent, ExDefaultLimit{}) : run<2>(blocks, absent, ExDefaultLimit{}))
+                               : (one ? run<1>(blocks, absent, ExGivenLimit{limit}) : run<2>(blocks, absent, ExGivenLimit{limit})))
+      return 1;
   return 0;
 }
