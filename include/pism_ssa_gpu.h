@@ -130,8 +130,10 @@ typedef struct pism_gpu_ssa_config {
   double ksp_rtol_max;
   double ksp_rtol_factor;
   /* launch mode of the Krylov iterations: 2 a graph-resident loop per solve (a CUDA graph
-     with a conditional WHILE node), 1 captured graphs of a few iterations, 0 direct launches
-     (kernel profilers that cannot look into conditional graphs need 0 or 1).
+     with a conditional WHILE node) or one kernel (block-Jacobi BiCGStab and SSAFEM's conjugate
+     gradients, on grids that fit the device at once), 1 captured graphs of a few iterations,
+     0 direct launches (kernel profilers that cannot look into conditional graphs need 0 or 1);
+     the same results, bit for bit.
      3 (BiCGStab only, otherwise as 2): the whole Picard loop of a solve is one CUDA graph
      with nested conditional nodes, its decisions taken on the device, one launch and one
      read-back per solve; the same results as 2, bit for bit */

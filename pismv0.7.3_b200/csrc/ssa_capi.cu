@@ -1564,11 +1564,11 @@ int pism_gpu_ssafem_solve(pism_gpu_ssa *h, const pism_gpu_ssafem_options *o, pis
       rc = fail(h, PISM_GPU_SSA_EZERODIAG, "SSAFEM: singular diagonal block at node %d", zp - 1);
       break;
     }
-    // conjugate gradients: the whole solve in one kernel where the grid fits the device, else in
-    // batches of FEM_CG_BATCH iterations, each skipped on the device once done; the batch is
+    // conjugate gradients: the whole solve in one kernel where the grid fits the device (graphs >= 2;
+    // the same bits), else in batches of FEM_CG_BATCH iterations, each skipped on the device once done; the batch is
     // captured into a CUDA graph on first use (its buffers never move) and replayed, with
     // direct launches if the capture fails
-    const bool resident = launch_fem_cg_resident(L, P, S);
+    const bool resident = h->cfg.graphs >= 2 && launch_fem_cg_resident(L, P, S);
     if (resident) {
       CK(h, cudaGetLastError());
       RET(copy_out(h, &cg, S.cg, sizeof(cg), PISM_MEM_HOST));

@@ -270,8 +270,18 @@ __global__ void __launch_bounds__(NTF) k_fem_node(FemProblem P, FemGrid G, FemCo
 }
 
 // ---- conjugate gradients on J du = -F, preconditioned by the inverse diagonal blocks ----
-__device__ __forceinline__ double2 bmul(double4 A, double2 x) {
-  return make_double2(A.x * x.x + A.y * x.y, A.z * x.x + A.w * x.y);
+// Which product of a sum is rounded by itself is written out, so that the kernels of an iteration
+// and the one of a whole solve give the same bits (left to the compiler they did not: 289 and 287
+// iterations of the first linear solve on 5 x 481 nodes): a b + c d with c d rounded first.
+__device__ __forceinline__ double two(double a, double b, double c, double d) {
+  return __fma_rn(a, b, __dmul_rn(c, d));
+}
+__device__ __forceinline__ double dot(const double2 &a, const double2 &b) { return two(a.x, b.x, a.y, b.y); }
+__device__ __forceinline__ double2 axpy(double s, const double2 &x, const double2 &y) {
+  return make_double2(__fma_rn(s, x.x, y.x), __fma_rn(s, x.y, y.y));
+}
+__device__ __forceinline__ double2 bmul(const double4 &A, const double2 &x) {
+  return make_double2(two(A.x, x.x, A.y, x.y), two(A.z, x.x, A.w, x.y));
 }
 
 __global__ void __launch_bounds__(NTF) k_cg_init(int N, const double2 *F, const double4 *dinv, double2 *x,
@@ -279,13 +289,15 @@ __global__ void __launch_bounds__(NTF) k_cg_init(int N, const double2 *F, const 
                                                  int maxit, double *partials, unsigned *ticket) {
   double acc[2] = {0.0, 0.0};
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
-    const double2 rn = make_double2(-F[n].x, -F[n].y), zn = bmul(dinv[n], rn);
+    const double2 rn = make_double2(-F[n].x, -F[n].y);
+    const double4 A = dinv[n];   // (the other product first, as the first z has always been rounded)
+    const double2 zn = make_double2(two(A.y, rn.y, A.x, rn.x), two(A.w, rn.y, A.z, rn.x));
     x[n] = make_double2(0.0, 0.0);
     r[n] = rn;
     z[n] = zn;
     p[n] = zn;
-    acc[0] += rn.x * zn.x + rn.y * zn.y;
-    acc[1] += rn.x * rn.x + rn.y * rn.y;
+    acc[0] += dot(rn, zn);
+    acc[1] += dot(rn, rn);
   }
   double tot[2];
   if (grid_reduce<2>(acc, partials, ticket, tot)) {
@@ -309,12 +321,12 @@ __global__ void __launch_bounds__(NTF) k_cg_apply(FemGrid G, const double *J, co
     double2 y = make_double2(0.0, 0.0);
     for (int b = 0; b < 9; ++b) {
       const double2 x = p[fem_node(G, i + b / 3 - 1, j + b % 3 - 1)];
-      y.x += J[(size_t)(b * 4 + 0) * N + n] * x.x + J[(size_t)(b * 4 + 1) * N + n] * x.y;
-      y.y += J[(size_t)(b * 4 + 2) * N + n] * x.x + J[(size_t)(b * 4 + 3) * N + n] * x.y;
+      y.x += two(J[(size_t)(b * 4 + 0) * N + n], x.x, J[(size_t)(b * 4 + 1) * N + n], x.y);
+      y.y += two(J[(size_t)(b * 4 + 2) * N + n], x.x, J[(size_t)(b * 4 + 3) * N + n], x.y);
     }
     q[n] = y;
     const double2 pn = p[n];
-    acc[0] += pn.x * y.x + pn.y * y.y;
+    acc[0] += dot(pn, y);
   }
   double tot[1];
   if (grid_reduce<1>(acc, partials, ticket, tot)) {
@@ -332,17 +344,12 @@ __global__ void __launch_bounds__(NTF) k_cg_update(int N, const double4 *dinv, c
   double acc[2] = {0.0, 0.0};
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
     const double2 pn = p[n], qn = q[n];
-    double2 xn = x[n], rn = r[n];
-    xn.x += alpha * pn.x;
-    xn.y += alpha * pn.y;
-    rn.x -= alpha * qn.x;
-    rn.y -= alpha * qn.y;
-    const double2 zn = bmul(dinv[n], rn);
-    x[n] = xn;
+    const double2 rn = axpy(-alpha, qn, r[n]), zn = bmul(dinv[n], rn);
+    x[n] = axpy(alpha, pn, x[n]);
     r[n] = rn;
     z[n] = zn;
-    acc[0] += rn.x * zn.x + rn.y * zn.y;
-    acc[1] += rn.x * rn.x + rn.y * rn.y;
+    acc[0] += dot(rn, zn);
+    acc[1] += dot(rn, rn);
   }
   double tot[2];
   if (grid_reduce<2>(acc, partials, ticket, tot)) {
@@ -359,8 +366,7 @@ __global__ void __launch_bounds__(NTF) k_cg_direction(int N, const double2 *z, d
   if (cg->done) return;
   const double beta = cg->beta;
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
-    const double2 zn = z[n], pn = p[n];
-    p[n] = make_double2(zn.x + beta * pn.x, zn.y + beta * pn.y);
+    p[n] = axpy(beta, p[n], z[n]);
   }
 }
 
@@ -454,10 +460,10 @@ __global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double 
 #pragma unroll
       for (int b = 0; b < 9; ++b) {
         const double2 pb = b == 4 ? pn : (at[b] >= 0 ? P[at[b]] : at[b] == -1 ? pa : pa2);
-        y.x += Js[(b * 4 + 0) * NTF + tid] * pb.x + Js[(b * 4 + 1) * NTF + tid] * pb.y;
-        y.y += Js[(b * 4 + 2) * NTF + tid] * pb.x + Js[(b * 4 + 3) * NTF + tid] * pb.y;
+        y.x += two(Js[(b * 4 + 0) * NTF + tid], pb.x, Js[(b * 4 + 1) * NTF + tid], pb.y);
+        y.y += two(Js[(b * 4 + 2) * NTF + tid], pb.x, Js[(b * 4 + 3) * NTF + tid], pb.y);
       }
-      acc[0] += pn.x * y.x + pn.y * y.y;
+      acc[0] += dot(pn, y);
     }
     double tq[1];
     if (!exchange_sum<1>(acc, slots_q, round, tq)) {
@@ -472,16 +478,13 @@ __global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double 
     alpha = rz / pq;
     double acc2[2] = {0.0, 0.0};
     if (mine) {
-      x.x += alpha * pn.x;
-      x.y += alpha * pn.y;
-      r.x -= alpha * y.x;
-      r.y -= alpha * y.y;
+      x = axpy(alpha, pn, x);
+      r = axpy(-alpha, y, r);
       z = bmul(d, r);
-      asm volatile("" : "+d"(z.x), "+d"(z.y));   // rounded here, as the other blocks' copies are
       // every owner has posted its (p, q) of this round, so none still reads the last round's z
       zex.put(n, z, round);
-      acc2[0] += r.x * z.x + r.y * z.y;
-      acc2[1] += r.x * r.x + r.y * r.y;
+      acc2[0] += dot(r, z);
+      acc2[1] += dot(r, r);
     }
     double tr[2];
     if (!exchange_sum<2>(acc2, slots_r, round, tr)) {
@@ -497,9 +500,7 @@ __global__ void __launch_bounds__(NTF, 2) k_cg_resident(FemGrid G, const double 
     if (done) break;
     // read after the sums, when the words are there: reads before them, repeated by every thread
     // until the owners have written, hold the sums up
-    auto direction = [&](const double2 &zn, const double2 &p) {
-      return make_double2(zn.x + beta * p.x, zn.y + beta * p.y);
-    };
+    auto direction = [&](const double2 &zn, const double2 &p) { return axpy(beta, p, zn); };
     bool ok;
     if (more) {   // warps that also read rows' ends or runs' ends
       const int nodes[5] = {above, below, apart[0] >= 0 ? apart[0] : above, apart[1] >= 0 ? apart[1] : above,
