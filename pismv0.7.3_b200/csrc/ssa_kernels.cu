@@ -569,38 +569,48 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_init(GridDev g, TileMap tm, Sten
   }
 }
 
-// p = r + beta (p - omega v);  phat = M^-1 p (block Jacobi; with multigrid phat is
-// written by the V-cycle instead)
-template <bool JAC>
-__global__ void __launch_bounds__(NT) k_bicg_p(int N, const double2 *r_, const double2 *v_,
-                                               const double4 *__restrict__ dinv, double2 *p_, double2 *phat_,
-                                               const KState *st_) {
-  pdl_wait();
-  const KState *st = after_wait(st_);
+// The five kernels of an iteration.  EARLY: with multigrid or the line solve, launched among the
+// preconditioner's short kernels while the one before still runs (ssa_pdl.cuh).  Block Jacobi
+// (!EARLY) has these five alone, on grids too large for k_bicg_resident: an early start takes SMs
+// from the kernel before, and vectors read through after_wait() are not read-only loads.  One B200,
+// us an iteration early / not: 94 x 400 cells 21.2 / 21.6, 240 x 330 24.9 / 23.8, 401^2 31.5 / 29.1,
+// 601^2 48.3 / 39.2, 801^2 77.8 / 73.1, 1201^2 159.0 / 153.8.  With the line solve 101^2 25.9 / 27.3,
+// 301^2 40.9 / 42.3, 401^2 49.1 / 48.8, 801^2 140.5 / 140.6.
+
+// p = r + beta (p - omega v);  phat = M^-1 p (block Jacobi; otherwise phat is written by the
+// preconditioner)
+template <bool EARLY>
+__global__ void __launch_bounds__(NT) k_bicg_p(int N, const double2 *__restrict__ r_, const double2 *__restrict__ v_,
+                                               const double4 *__restrict__ dinv, double2 *__restrict__ p_,
+                                               double2 *__restrict__ phat_, const KState *st_) {
+  if (EARLY) pdl_wait();
+  const KState *st = after_wait<EARLY>(st_);
   if (st->done) return;
-  pdl_release();
-  const double2 *__restrict__ r = after_wait(r_), *__restrict__ v = after_wait(v_);
-  double2 *__restrict__ p = after_wait(p_), *__restrict__ phat = after_wait(phat_);
+  if (EARLY) pdl_release();
+  const double2 *__restrict__ r = after_wait<EARLY>(r_), *__restrict__ v = after_wait<EARLY>(v_);
+  double2 *__restrict__ p = after_wait<EARLY>(p_), *__restrict__ phat = after_wait<EARLY>(phat_);
   const double bta = st->beta, om = st->omega;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 rk = r[k], pk = p[k], vk = v[k];
     const double2 pn = make_double2(rk.x + bta * (pk.x - om * vk.x), rk.y + bta * (pk.y - om * vk.y));
     p[k] = pn;
-    if (JAC) phat[k] = dmul(dinv[k], pn);
+    if (!EARLY) phat[k] = dmul(dinv[k], pn);
   }
 }
 
 // v = A phat; alpha = rho / (rhat . v)
+template <bool EARLY>
 __global__ void __launch_bounds__(NT, 4) k_bicg_v(GridDev g, TileMap tm, StencilConst s, const uint32_t *__restrict__ flags,
                                                const double2 *__restrict__ nuH, const double *__restrict__ beta,
-                                               const double2 *phat_, const double2 *rhat_, double2 *v_,
-                                               double *partials, unsigned *ticket, KState *st_) {
-  pdl_wait();
-  KState *st = after_wait(st_);
+                                               const double2 *__restrict__ phat_, const double2 *__restrict__ rhat_,
+                                               double2 *__restrict__ v_, double *partials, unsigned *ticket,
+                                               KState *st_) {
+  if (EARLY) pdl_wait();
+  KState *st = after_wait<EARLY>(st_);
   if (st->done) return;
-  pdl_release();
-  const double2 *__restrict__ phat = after_wait(phat_), *__restrict__ rhat = after_wait(rhat_);
-  double2 *__restrict__ v = after_wait(v_);
+  if (EARLY) pdl_release();
+  const double2 *__restrict__ phat = after_wait<EARLY>(phat_), *__restrict__ rhat = after_wait<EARLY>(rhat_);
+  double2 *__restrict__ v = after_wait<EARLY>(v_);
   double acc[1] = {0.0};
   __shared__ HaloTile<double2> xT, nT;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -625,36 +635,38 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_v(GridDev g, TileMap tm, Stencil
 }
 
 // s = r - alpha v;  shat = M^-1 s
-template <bool JAC>
-__global__ void __launch_bounds__(NT) k_bicg_s(int N, const double2 *r_, const double2 *v_,
-                                               const double4 *__restrict__ dinv, double2 *sv_, double2 *shat_,
-                                               const KState *st_) {
-  pdl_wait();
-  const KState *st = after_wait(st_);
+template <bool EARLY>
+__global__ void __launch_bounds__(NT) k_bicg_s(int N, const double2 *__restrict__ r_, const double2 *__restrict__ v_,
+                                               const double4 *__restrict__ dinv, double2 *__restrict__ sv_,
+                                               double2 *__restrict__ shat_, const KState *st_) {
+  if (EARLY) pdl_wait();
+  const KState *st = after_wait<EARLY>(st_);
   if (st->done) return;
-  pdl_release();
-  const double2 *__restrict__ r = after_wait(r_), *__restrict__ v = after_wait(v_);
-  double2 *__restrict__ sv = after_wait(sv_), *__restrict__ shat = after_wait(shat_);
+  if (EARLY) pdl_release();
+  const double2 *__restrict__ r = after_wait<EARLY>(r_), *__restrict__ v = after_wait<EARLY>(v_);
+  double2 *__restrict__ sv = after_wait<EARLY>(sv_), *__restrict__ shat = after_wait<EARLY>(shat_);
   const double al = st->alpha;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 rk = r[k], vk = v[k];
     const double2 sk = make_double2(rk.x - al * vk.x, rk.y - al * vk.y);
     sv[k] = sk;
-    if (JAC) shat[k] = dmul(dinv[k], sk);
+    if (!EARLY) shat[k] = dmul(dinv[k], sk);
   }
 }
 
 // t = A shat; omega = (t . s) / (t . t)
+template <bool EARLY>
 __global__ void __launch_bounds__(NT, 4) k_bicg_t(GridDev g, TileMap tm, StencilConst s, const uint32_t *__restrict__ flags,
                                                const double2 *__restrict__ nuH, const double *__restrict__ beta,
-                                               const double2 *shat_, const double2 *sv_, double2 *tv_,
-                                               double *partials, unsigned *ticket, KState *st_) {
-  pdl_wait();
-  KState *st = after_wait(st_);
+                                               const double2 *__restrict__ shat_, const double2 *__restrict__ sv_,
+                                               double2 *__restrict__ tv_, double *partials, unsigned *ticket,
+                                               KState *st_) {
+  if (EARLY) pdl_wait();
+  KState *st = after_wait<EARLY>(st_);
   if (st->done) return;
-  pdl_release();
-  const double2 *__restrict__ shat = after_wait(shat_), *__restrict__ sv = after_wait(sv_);
-  double2 *__restrict__ tv = after_wait(tv_);
+  if (EARLY) pdl_release();
+  const double2 *__restrict__ shat = after_wait<EARLY>(shat_), *__restrict__ sv = after_wait<EARLY>(sv_);
+  double2 *__restrict__ tv = after_wait<EARLY>(tv_);
   double acc[2] = {0.0, 0.0};
   __shared__ HaloTile<double2> xT, nT;
   for (int t = blockIdx.x; t < tm.tiles; t += gridDim.x) {
@@ -674,22 +686,24 @@ __global__ void __launch_bounds__(NT, 4) k_bicg_t(GridDev g, TileMap tm, Stencil
 
 // x += alpha phat + omega shat;  r = s - omega t;  convergence test, and the WHILE condition
 // of a graph-resident loop (cond, 0: none)
-__global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *phat_, const double2 *shat_, const double2 *sv_,
-                                               const double2 *tv_, const double2 *rhat_, double2 *x_, double2 *r_,
-                                               double *partials, unsigned *ticket, KState *st_,
+template <bool EARLY>
+__global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *__restrict__ phat_, const double2 *__restrict__ shat_,
+                                               const double2 *__restrict__ sv_, const double2 *__restrict__ tv_,
+                                               const double2 *__restrict__ rhat_, double2 *__restrict__ x_,
+                                               double2 *__restrict__ r_, double *partials, unsigned *ticket, KState *st_,
                                                cudaGraphConditionalHandle cond) {
-  pdl_wait();
-  KState *st = after_wait(st_);
+  if (EARLY) pdl_wait();
+  KState *st = after_wait<EARLY>(st_);
   if (st->done) {
     if (cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
     return;
   }
-  pdl_release();
+  if (EARLY) pdl_release();
   const double al = st->alpha, om = st->omega;
-  const double2 *__restrict__ phat = after_wait(phat_), *__restrict__ shat = after_wait(shat_);
-  const double2 *__restrict__ sv = after_wait(sv_), *__restrict__ tv = after_wait(tv_);
-  const double2 *__restrict__ rhat = after_wait(rhat_);
-  double2 *__restrict__ x = after_wait(x_), *__restrict__ r = after_wait(r_);
+  const double2 *__restrict__ phat = after_wait<EARLY>(phat_), *__restrict__ shat = after_wait<EARLY>(shat_);
+  const double2 *__restrict__ sv = after_wait<EARLY>(sv_), *__restrict__ tv = after_wait<EARLY>(tv_);
+  const double2 *__restrict__ rhat = after_wait<EARLY>(rhat_);
+  double2 *__restrict__ x = after_wait<EARLY>(x_), *__restrict__ r = after_wait<EARLY>(r_);
   double acc[2] = {0.0, 0.0};
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < N; k += gridDim.x * blockDim.x) {
     const double2 ph = phat[k], sh = shat[k], sk = sv[k], tk = tv[k];
@@ -737,8 +751,10 @@ __global__ void __launch_bounds__(NT) k_bicg_x(int N, const double2 *phat_, cons
 // for bit.
 //
 // Bound: the exchanges' trips through L2 (about 1 us each).  Test I on 5 x 201 (1486 iterations in
-// 22 Picard steps), one B200: 27.2 ms with the five kernels, 10.2 ms with this one.  Grids of
-// more tiles than SMs (37 888 cells at most) keep the five kernels.
+// 22 Picard steps), one B200: 27.2 - 31 ms with the five kernels, 10.2 - 11.0 ms with this one.  It is
+// faster up to the last grid that fits, us an iteration with the five kernels / this one: 7 tiles
+// 20.0 / 5.5, 35 tiles 20.3 / 8.3, 100 tiles 21.6 / 8.6, 130 tiles 20.5 / 9.3, 144 tiles 20.7 / 9.9.
+// Grids of more tiles than SMs (37 888 cells at most) keep the five kernels.
 // ---------------------------------------------------------------------------
 template <class Limit>
 struct BicgResident {
@@ -1084,24 +1100,34 @@ void launch_bicg_init(const Launch &L, const GridDev &g, const Fields &f, const 
                                                                 cond);
 }
 
-void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+template <bool EARLY>
+static void bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
                            const MGHierarchy *mg, const LinePC *line, cudaGraphConditionalHandle cond) {
-  L.tick(5);
   TileMap tm = make_tiles(g);
   const int N = g.Mx * g.My;
   const StencilConst s = stencil_const(g, f);
   const int bt = grid_for_tiles(L, tm.tiles), bv = grid_for(L, N);
-  const bool jac = !mg && !line;
-  launch_pdl(L, jac ? k_bicg_p<true> : k_bicg_p<false>, bv, NT, 0, N, K.r, K.v, K.dinv, K.p, K.phat, K.st);
-  if (mg) mg_vcycle(L, g, f, *mg, K.p, K.phat, K.st);
-  else if (line) line_apply(L, g, *line, K.p, K.phat, K.st);
-  launch_pdl(L, k_bicg_v, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.phat, K.rhat, K.v, L.partials, L.ticket,
-             K.st);
-  launch_pdl(L, jac ? k_bicg_s<true> : k_bicg_s<false>, bv, NT, 0, N, K.r, K.v, K.dinv, K.s, K.shat, K.st);
-  if (mg) mg_vcycle(L, g, f, *mg, K.s, K.shat, K.st);
-  else if (line) line_apply(L, g, *line, K.s, K.shat, K.st);
-  launch_pdl(L, k_bicg_t, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.shat, K.s, K.t, L.partials, L.ticket, K.st);
-  launch_pdl(L, k_bicg_x, bv, NT, 0, N, K.phat, K.shat, K.s, K.t, K.rhat, x, K.r, L.partials, L.ticket, K.st, cond);
+  auto precondition = [&](const double2 *r, double2 *z) {
+    if (mg) mg_vcycle(L, g, f, *mg, r, z, K.st);
+    else if (line) line_apply(L, g, *line, r, z, K.st);
+  };
+  launch_early<EARLY>(L, k_bicg_p<EARLY>, bv, NT, 0, N, K.r, K.v, K.dinv, K.p, K.phat, K.st);
+  precondition(K.p, K.phat);
+  launch_early<EARLY>(L, k_bicg_v<EARLY>, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.phat, K.rhat, K.v, L.partials,
+                      L.ticket, K.st);
+  launch_early<EARLY>(L, k_bicg_s<EARLY>, bv, NT, 0, N, K.r, K.v, K.dinv, K.s, K.shat, K.st);
+  precondition(K.s, K.shat);
+  launch_early<EARLY>(L, k_bicg_t<EARLY>, bt, NT, 0, g, tm, s, f.flags, f.nuH, f.beta, K.shat, K.s, K.t, L.partials,
+                      L.ticket, K.st);
+  launch_early<EARLY>(L, k_bicg_x<EARLY>, bv, NT, 0, N, K.phat, K.shat, K.s, K.t, K.rhat, x, K.r, L.partials, L.ticket,
+                      K.st, cond);
+}
+
+void launch_bicg_iteration(const Launch &L, const GridDev &g, const Fields &f, const Krylov &K, double2 *x,
+                           const MGHierarchy *mg, const LinePC *line, cudaGraphConditionalHandle cond) {
+  L.tick(5);
+  if (mg || line) bicg_iteration<true>(L, g, f, K, x, mg, line, cond);
+  else bicg_iteration<false>(L, g, f, K, x, nullptr, nullptr, cond);
 }
 
 static size_t bicg_exchange_words(const GridDev &g, int tiles) {

@@ -22,15 +22,17 @@ namespace pism_gpu {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// the same pointer, as a value the compiler knows only from here on
-template <class T>
+// the same pointer, as a value the compiler knows only from here on (!EARLY: in a kernel's form
+// that is launched after its predecessor, the pointer as it is)
+template <bool EARLY = true, class T>
 __device__ __forceinline__ T *after_wait(T *p) {
-  asm volatile("" : "+l"(p)::"memory");
+  if constexpr (EARLY) asm volatile("" : "+l"(p)::"memory");
   return p;
 }
 
-template <class... P, class... A>
-inline void launch_pdl(const Launch &L, void (*kernel)(P...), int blocks, int threads, size_t smem, A &&...args) {
+// EARLY: while its predecessor still runs; else after it
+template <bool EARLY, class... P, class... A>
+inline void launch_early(const Launch &L, void (*kernel)(P...), int blocks, int threads, size_t smem, A &&...args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)blocks);
   cfg.blockDim = dim3((unsigned)threads);
@@ -40,8 +42,12 @@ inline void launch_pdl(const Launch &L, void (*kernel)(P...), int blocks, int th
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = EARLY ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline void launch_pdl(const Launch &L, void (*kernel)(P...), int blocks, int threads, size_t smem, A &&...args) {
+  launch_early<true>(L, kernel, blocks, threads, smem, std::forward<A>(args)...);
 }
 
 }  // namespace pism_gpu
