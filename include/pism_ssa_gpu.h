@@ -234,6 +234,11 @@ const char *pism_gpu_ssa_last_error(const pism_gpu_ssa *h);
 /* Run the handle's work on a caller-owned cudaStream_t (NULL = the handle's own). */
 int pism_gpu_ssa_set_stream(pism_gpu_ssa *h, void *cuda_stream);
 
+/* Order the handle's stream after the work queued so far on `cuda_stream` (NULL = the legacy
+ * default stream), without waiting on the host: for device arrays that a call is given while the
+ * kernels that fill them, or last read the memory of its outputs, may still run there. */
+int pism_gpu_ssa_wait_stream(pism_gpu_ssa *h, void *cuda_stream);
+
 /* The linear solves that run as one kernel (block-Jacobi BiCGStab with graphs >= 2, SSAFEM's
  * conjugate gradients) wait between their blocks by reading a word until it is there.  A wait gives
  * up after `reads` reads (1 .. 2^20, the default, about a second), and the solve then ends as a

@@ -22,7 +22,8 @@ MEM_HOST, MEM_DEVICE = 0, 1
 # every symbol include/pism_ssa_gpu.h declares
 EXPORTS = [
     "pism_gpu_ssa_config_defaults", "pism_gpu_ssa_create", "pism_gpu_ssa_destroy", "pism_gpu_ssa_last_error",
-    "pism_gpu_ssa_set_stream", "pism_gpu_ssa_set_wait_limit", "pism_gpu_ssa_set_config", "pism_gpu_ssa_set_inputs",
+    "pism_gpu_ssa_set_stream", "pism_gpu_ssa_wait_stream", "pism_gpu_ssa_set_wait_limit",
+    "pism_gpu_ssa_set_config", "pism_gpu_ssa_set_inputs",
     "pism_gpu_ssa_set_initial_guess", "pism_gpu_ssa_solve", "pism_gpu_ssa_get_field",
     "pism_gpu_ssa_assemble_rhs", "pism_gpu_ssa_compute_hardness", "pism_gpu_ssa_compute_nuH",
     "pism_gpu_ssa_apply", "pism_gpu_ssa_apply_preconditioner", "pism_gpu_ssa_linear_solve",
@@ -57,6 +58,7 @@ def load() -> C.CDLL:
         "pism_gpu_ssa_destroy": (I, [V]),
         "pism_gpu_ssa_last_error": (C.c_char_p, [V]),
         "pism_gpu_ssa_set_stream": (I, [V, V]),
+        "pism_gpu_ssa_wait_stream": (I, [V, V]),
         "pism_gpu_ssa_set_wait_limit": (I, [V, I]),
         "pism_gpu_ssa_set_config": (I, [V, P(CConfig)]),
         "pism_gpu_ssa_set_inputs": (I, [V, P(CInputs)]),

@@ -89,6 +89,7 @@ struct pism_gpu_ssa {
   double *norm_host = nullptr;
   int *zd_host = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t filled = nullptr;   // pism_gpu_ssa_wait_stream's, made by its first call
   bool inputs_set = false, have_melange = false, have_gl = false, have_enthalpy = false, have_hardness = false,
        have_fracture = false, prepared = false;
   int default_pc_failure_count = 0;   // SSAFD.cc:252-253 (m_default_pc_failure_*)
@@ -1156,6 +1157,7 @@ int pism_gpu_ssa_destroy(pism_gpu_ssa *h) {
   if (h->res_host) cudaFreeHost(h->res_host);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
+  if (h->filled) cudaEventDestroy(h->filled);
   for (auto &gr : h->graphs)
     if (gr.exec) cudaGraphExecDestroy(gr.exec);
   for (auto &lp : h->loops)
@@ -1173,6 +1175,22 @@ int pism_gpu_ssa_set_stream(pism_gpu_ssa *h, void *s) {
   if (!h) return PISM_GPU_SSA_EINVAL;
   h->stream = s ? (cudaStream_t)s : h->own_stream;
   h->L.stream = h->stream;
+  return PISM_GPU_SSA_OK;
+}
+
+int pism_gpu_ssa_wait_stream(pism_gpu_ssa *h, void *s) {
+  if (!h) return PISM_GPU_SSA_EINVAL;
+  if ((cudaStream_t)s == h->stream) return PISM_GPU_SSA_OK;
+  DeviceGuard dg(h->device);
+  // what a capturing stream queues has not run, and is not waited for
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing((cudaStream_t)s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return PISM_GPU_SSA_OK;
+  }
+  if (!h->filled) CK(h, cudaEventCreateWithFlags(&h->filled, cudaEventDisableTiming));
+  CK(h, cudaEventRecord(h->filled, (cudaStream_t)s));
+  CK(h, cudaStreamWaitEvent(h->stream, h->filled, 0));
   return PISM_GPU_SSA_OK;
 }
 

@@ -151,6 +151,7 @@ def features(ssa, stride: int = 1):
     import torch
     hh, ww = image_shape(*ssa.shape, stride)
     f = torch.empty((hh, ww, IN_CHANNELS), dtype=torch.float32, device=torch.device("cuda", ssa.device))
+    ssa._after_torch()
     ssa._check(ssa.lib.pism_gpu_ssa_learned_features(ssa._h, stride, _ptr(f), hh, ww), "learned_features")
     return f
 
@@ -328,6 +329,7 @@ def pc_input(ssa, r, stride: int = 1):
     img = torch.zeros((hh, ww, IN_CHANNELS), dtype=torch.float32, device=r.device)
     rho = torch.zeros((), dtype=torch.float64, device=r.device)
     rr = r.contiguous()
+    ssa._after_torch()
     ssa._check(ssa.lib.pism_gpu_ssa_learned_pc_input(ssa._h, stride, _ptr(rr), _ptr(img), hh, ww, _ptr(rho)),
                "learned_pc_input")
     return img, rho

@@ -108,6 +108,15 @@ class SSAFD:
             msg = self.lib.pism_gpu_ssa_last_error(self._h).decode() or what
             raise _EXC.get(rc, SSAError)(f"{what}: {msg} (status {rc})")
 
+    def _after_torch(self):
+        """Order the handle's stream after what torch's current stream has queued: CUDA tensors
+        are filled there (the copies and zeros made here, a caller's guess), and the memory that
+        torch gives an output may still be read there by work that came before."""
+        from torch._C import _cuda_getCurrentRawStream   # current_stream() without its object: 1.2 us a call
+        rc = self.lib.pism_gpu_ssa_wait_stream(self._h, _cuda_getCurrentRawStream(self.device))
+        if rc:
+            self._check(rc, "wait_stream")
+
     @property
     def shape(self):
         return (self.grid.Mx, self.grid.My)
@@ -165,6 +174,8 @@ class SSAFD:
 
     def _upload(self):
         ci, _keep = self._inputs(self._fields, self._bc)
+        if ci.where == _capi.MEM_DEVICE:
+            self._after_torch()
         self._check(self.lib.pism_gpu_ssa_set_inputs(self._h, C.byref(ci)), "set_inputs")
 
     def solve_batch(self, members, net=None, stride: int = 1):
@@ -196,6 +207,8 @@ class SSAFD:
             arr[q].velocity = vb.ptr
             keep += [bufs, vb]
             outs.append(vb.keep)
+        if any(b.device for b in keep[1::2]):
+            self._after_torch()
         nh = net._h if net is not None else None
         rc = self.lib.pism_gpu_ssa_solve_batch(self._h, nh, stride, n, arr, stats)
         if rc not in (_capi.OK, _capi.EKSP, _capi.EPICARD, _capi.ENAN, _capi.EZERODIAG):
@@ -205,6 +218,8 @@ class SSAFD:
     def set_initial_guess(self, guess):
         """SSA::set_initial_guess (SSA.cc:361-363)."""
         b = _Buf(guess, (*self.shape, 2))
+        if b.device:
+            self._after_torch()
         where = _capi.MEM_DEVICE if b.device else _capi.MEM_HOST
         self._check(self.lib.pism_gpu_ssa_set_initial_guess(self._h, b.ptr, where), "set_initial_guess")
 
@@ -222,6 +237,8 @@ class SSAFD:
         if out is None:
             out = np.empty((*self.shape, 2))
         b = _Buf(out, (*self.shape, 2))
+        if b.device:
+            self._after_torch()
         where = _capi.MEM_DEVICE if b.device else _capi.MEM_HOST
         rc = self.lib.pism_gpu_ssa_solve(self._h, b.ptr, where, C.byref(self._stats))
         self._check(rc, "SSAFD solve")
@@ -241,6 +258,8 @@ class SSAFD:
         if out is None:
             out = np.empty(shape)
         b = _Buf(out, shape)
+        if b.device:
+            self._after_torch()
         where = _capi.MEM_DEVICE if b.device else _capi.MEM_HOST
         self._check(self.lib.pism_gpu_ssa_get_field(self._h, field, b.ptr, where), "get_field")
         return b.keep if b.device else out
@@ -286,6 +305,8 @@ class SSAFD:
                     out[k] = torch.empty(shape, dtype=torch.float64, device=f"cuda:{self.device}")
                 else:
                     out[k] = np.empty(shape)
+        if on_device:
+            self._after_torch()
         bufs = {k: _Buf(out[k], shape) for k in names}
         bmr = _Buf(basal_melt_rate, self.shape) if basal_melt_rate is not None else None
         if bmr is not None and bmr.device != on_device:
@@ -312,6 +333,7 @@ class SSAFD:
             import torch
             out = {k: torch.empty(shape, dtype=torch.float64, device=f"cuda:{self.device}")
                    for k in ("thickness", "mask", "surface", "flux_divergence")}
+            self._after_torch()
         else:
             out = {k: np.empty(shape) for k in ("thickness", "mask", "surface", "flux_divergence")}
         ins = [_Buf(a, shape) if a is not None else None for a in (climatic_mass_balance, basal_melt_rate, cell_area)]
@@ -348,6 +370,8 @@ class SSAFD:
                 out[k] = torch.empty((*shape, d), dtype=torch.float64, device=f"cuda:{self.device}")
             else:
                 out[k] = np.empty((*shape, d))
+        if on_device:
+            self._after_torch()
         bufs = {k: _Buf(v, v.shape) for k, v in out.items()}
         where = _capi.MEM_DEVICE if on_device else _capi.MEM_HOST
         self._check(self.lib.pism_gpu_ssa_strain_rates(self._h, m.ptr, bufs["edot"].ptr if "edot" in bufs else None,
@@ -368,6 +392,7 @@ class SSAFD:
         if on_device:
             import torch
             bufs = [_Buf(a.to(torch.float64).reshape(shape).clone(), shape) for a in (mask, Href, thickness)]
+            self._after_torch()
         else:
             bufs = [_Buf(np.array(a, dtype=np.float64).reshape(shape), shape) for a in (mask, Href, thickness)]
         where = _capi.MEM_DEVICE if on_device else _capi.MEM_HOST
@@ -379,6 +404,8 @@ class SSAFD:
         """EigenCalving::max_timestep (PISMEigenCalving.cc:249-341) on the current velocity:
         "dt" (s), "max_rate", "mean_rate" (m/s) and "count" of calving cells."""
         m = _Buf(mask, self.shape)
+        if m.device:
+            self._after_torch()
         res = (C.c_double * 4)()
         where = _capi.MEM_DEVICE if m.device else _capi.MEM_HOST
         self._check(self.lib.pism_gpu_ssa_eigen_calving_max_timestep(self._h, float(K), m.ptr, C.cast(res, _D), where),
