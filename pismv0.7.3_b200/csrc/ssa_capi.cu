@@ -1405,7 +1405,7 @@ int pism_gpu_ssa_mass_continuity_step(pism_gpu_ssa *h, double dt, const double *
   CK(h, cudaGetLastError());
   for (int q = 0; q < 4; ++q)
     if (out[q] && where == PISM_MEM_HOST) RET(copy_out(h, out[q], dout[q], sizeof(double) * N, PISM_MEM_HOST));
-  if (totals) RET(copy_out(h, totals, dtot, sizeof(double) * 8, PISM_MEM_HOST));
+  if (totals) return copy_out(h, totals, dtot, sizeof(double) * 8, PISM_MEM_HOST);   // waits for the stream
   CK(h, cudaStreamSynchronize(h->stream));
   return PISM_GPU_SSA_OK;
 }
@@ -1469,8 +1469,7 @@ int pism_gpu_ssa_eigen_calving(pism_gpu_ssa *h, double dt, double K, double *mas
     RET(copy_out(h, Href, dHref, sizeof(double) * N, PISM_MEM_HOST));
     RET(copy_out(h, thickness, dH, sizeof(double) * N, PISM_MEM_HOST));
   }
-  CK(h, cudaStreamSynchronize(h->stream));
-  return PISM_GPU_SSA_OK;
+  return PISM_GPU_SSA_OK;   // the flag's read-back came after the last kernel
 }
 
 int pism_gpu_ssa_eigen_calving_max_timestep(pism_gpu_ssa *h, double K, const double *mask, double *result,

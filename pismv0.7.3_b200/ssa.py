@@ -23,6 +23,7 @@ from . import _capi
 from .config import CFemOptions, CFemStats, CInputs, CMember, CStats, GridDesc, SSAConfig
 
 _D = C.POINTER(C.c_double)
+_raw_stream = None   # torch's raw current stream of a device, once a CUDA tensor has been given
 
 
 class SSAError(RuntimeError):
@@ -112,8 +113,10 @@ class SSAFD:
         """Order the handle's stream after what torch's current stream has queued: CUDA tensors
         are filled there (the copies and zeros made here, a caller's guess), and the memory that
         torch gives an output may still be read there by work that came before."""
-        from torch._C import _cuda_getCurrentRawStream   # current_stream() without its object: 1.2 us a call
-        rc = self.lib.pism_gpu_ssa_wait_stream(self._h, _cuda_getCurrentRawStream(self.device))
+        global _raw_stream
+        if _raw_stream is None:   # current_stream() without its object, 1.2 us a call
+            from torch._C import _cuda_getCurrentRawStream as _raw_stream
+        rc = self.lib.pism_gpu_ssa_wait_stream(self._h, _raw_stream(self.device))
         if rc:
             self._check(rc, "wait_stream")
 
