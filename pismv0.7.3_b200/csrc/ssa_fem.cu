@@ -290,14 +290,14 @@ __global__ void __launch_bounds__(NTF) k_cg_init(int N, const double2 *F, const 
   double acc[2] = {0.0, 0.0};
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
     const double2 rn = make_double2(-F[n].x, -F[n].y);
-    const double4 A = dinv[n];   // (the other product first, as the first z has always been rounded)
+    const double4 A = dinv[n];   // (here the other product first, as this kernel has always rounded)
     const double2 zn = make_double2(two(A.y, rn.y, A.x, rn.x), two(A.w, rn.y, A.z, rn.x));
     x[n] = make_double2(0.0, 0.0);
     r[n] = rn;
     z[n] = zn;
     p[n] = zn;
-    acc[0] += dot(rn, zn);
-    acc[1] += dot(rn, rn);
+    acc[0] += two(rn.y, zn.y, rn.x, zn.x);
+    acc[1] += two(rn.y, rn.y, rn.x, rn.x);
   }
   double tot[2];
   if (grid_reduce<2>(acc, partials, ticket, tot)) {

@@ -7,7 +7,9 @@
 //
 // Each thread accumulates its cells' terms in FP64 in its own order; finish() adds the grid's
 // partial sums in block order (ssa_reduce.cuh) and writes the scalar to the Krylov state.  The
-// iteration reads the scalars as FP32, which rounds the order of the FP64 sums away.
+// apply kernels and the marching pass add in different orders (the pass's follows the device's
+// SMs), so their scalars may differ in the last bits; the iteration reads them as FP32, which almost
+// always rounds that away: the iterates of the two usually agree bit for bit, but need not.
 #pragma once
 
 #include "ssa_reduce.cuh"
