@@ -61,7 +61,7 @@ DEFAULT_GRAPHS = 3
 # In-solve DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum, --cache-control
 # none) of one inner iteration's kernels on the 801^2 sheet, per (grid, precision, FP32 apply
 # kernel) (profiles/inner_iteration_traffic_801.md: the per-launch averages of the kernels)
-INNER_ITERATION_TRAFFIC = {(801, "mixed", 2): 96.5e6}
+INNER_ITERATION_TRAFFIC = {(801, "mixed", 2): 71.2e6}
 
 
 def _package():
@@ -414,7 +414,8 @@ def ssafem_point(dev, stream, reps=3):
         out[name] = {"ms": float(np.median(ts)), "newton_iterations": st["newton_iterations"],
                      "cg_iterations": st["ksp_iterations"], "converged": st["converged"],
                      "maxvector_error_m_per_year": err["maxvector"]}
-    out["note"] = "wall time of the call (host loop with a read-back per Newton step and CG batch)"
+    out["note"] = ("wall time of the call (host loop, each linear solve one kernel; a read-back per residual, "
+                   "set-up and linear solve)")
     return out
 
 
@@ -541,10 +542,15 @@ def ensemble_member(q, M=401):
     return g, c, f, {"T": T, "tauc_median": med}
 
 
+# what fast_config makes of the synthetic sheets' configuration, whose preconditioner it keeps
+ENSEMBLE_SET_UP = "FP64 BiCGStab with point-block Jacobi, inexact Picard, learned guess"
+
+
 def ensemble_point(stream, flush, dev, members=16, steps=2):
     """members/s of pism_gpu_ssa_solve_batch on `members` seeded 401^2 sheets (the ensemble
-    workload's members 0 .. members-1, fast set-up, learned guess), device-timed, L2 flushed
-    before each batch: the ensemble configuration in the default bench line"""
+    workload's members 0 .. members-1, learned guess, inexact Picard; the synthetic sheets'
+    preconditioner, point-block Jacobi, so FP64 BiCGStab: FP32 inner solves need multigrid),
+    device-timed, L2 flushed before each batch: the ensemble configuration in the default bench line"""
     import torch
     from pism_b200 import learned as Lrn
     from pism_b200.ssa import SSAFD
@@ -579,14 +585,15 @@ def ensemble_point(stream, flush, dev, members=16, steps=2):
     return {"members": members, "grid": [M, M], "ms_per_batch": ms, "members_per_s": members / (ms * 1e-3),
             "converged": int(sum(st["converged"] for st in stats)),
             "picard_iterations": [st["picard_iterations"] for st in stats],
+            "set_up": ENSEMBLE_SET_UP,
             "how": "pism_gpu_ssa_solve_batch, members in turn on one handle (bench.py --workload ensemble "
                    "runs the 64-member configuration with its accuracy check)"}
 
 
 def run_ensemble(args):
-    """--workload ensemble: pism_gpu_ssa_solve_batch over the members of this rank (the
-    fast set-up with the learned guess), members/s of the whole job; each member's
-    velocity error against the plain FP64 solve of the same member."""
+    """--workload ensemble: pism_gpu_ssa_solve_batch over the members of this rank (set up
+    as in ensemble_point), members/s of the whole job; each member's velocity error against
+    the plain FP64 solve of the same member."""
     import torch
     import torch.distributed as dist
     world = int(os.environ.get("WORLD_SIZE", "1"))
@@ -657,12 +664,12 @@ def run_ensemble(args):
     s.close()
     net.close()
     line = {
-        "metric": f"ensemble members solved/s ({args.members} x {M}^2 per GPU, learned+FP32)", "value": value,
+        "metric": f"ensemble members solved/s ({args.members} x {M}^2 per GPU, learned, FP64 block Jacobi)", "value": value,
         "unit": "members/s", "n_gpus": world, "steps": args.steps, "warmup": 1, "ms_per_step": step_ms,
-        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64+f32", "data": "synthetic",
+        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": {"workload": f"ensemble of {args.members} seeded {M}x{M} sheets at 10 km per GPU, temperature "
                                "U[-20,-2] C and tau_c median U[20,200] kPa per member, solved by "
-                               "pism_gpu_ssa_solve_batch (fast set-up, learned guess)",
+                               f"pism_gpu_ssa_solve_batch ({ENSEMBLE_SET_UP})",
                    "members_per_gpu": args.members, "l2": "flushed (256 MB write) between steps",
                    "parallelism": f"members sharded over {world} GPU(s)"},
         "members": {"picard_iterations": [st["picard_iterations"] for st in stats],
@@ -966,7 +973,7 @@ def main():
                  1: "k_mg0_post, then k32_apply with bulk-copy-staged tiles",
                  0: "k_mg0_post, then k32_apply"}[c.mixed_apply_kernel]
     roof["kernel"] = (f"one inner BiCGStab + V(1,1) multigrid iteration: k32_p, k32_x + 2 x (k_mg0_restrict, "
-                      f"k_mgc_restrict x3, k_mg_small_cycle, k_mgc_post x3, {fine_last})"
+                      f"k_mgc_restrict x3, k_mg_small_resident, k_mgc_post x3, {fine_last})"
                       if c.precision == "mixed" else "one BiCGStab + V(1,1) multigrid iteration (FP64 Krylov vectors)")
     # the FP64 matrix-free apply alone, each launch timed with L2 flushed before it (HBM-bound)
     x = torch.randn((M, M, 2), dtype=torch.float64, device=dev) * 1e-5

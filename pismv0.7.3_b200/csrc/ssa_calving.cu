@@ -18,8 +18,8 @@
 // bytes.  The caller's mask is read as doubles where it is needed (no conversion pass), the
 // passes of a calving step are launched together, each while its predecessor drains, and a sweep
 // after one that changed nothing returns at once: the host reads one word a batch of sweeps.
-// Strain rates with stresses, a calving step and its time step, 801 x 801: 234 us with a pass a
-// step and a read-back a sweep, 189 now (195 before a front cell's loads were issued together).
+// Strain rates with stresses, a calving step and its time step, 801 x 801: 216 - 234 us by box with a
+// pass a step and a read-back a sweep, 190 - 203 now, 81 of them in kernels.
 #include <algorithm>
 #include <cstdint>
 
