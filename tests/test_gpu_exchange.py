@@ -25,7 +25,7 @@ SHORT = 2000   # reads: about 2 ms
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def driver(tmp_path_factory):
     if shutil.which("nvcc") is None:
         pytest.skip("needs nvcc")
     exe = str(tmp_path_factory.mktemp("exchange") / "check")
@@ -35,24 +35,24 @@ def checker(tmp_path_factory):
     return exe
 
 
-def ask(checker, *line):
-    out = subprocess.run([checker], input=" ".join(str(v) for v in line) + "\n", capture_output=True, text=True,
+def ask(driver, *line):
+    out = subprocess.run([driver], input=" ".join(str(v) for v in line) + "\n", capture_output=True, text=True,
                          check=True, timeout=60).stdout.split()
     return [int(v) for v in out[:3]], out[3] == "1"
 
 
 @pytest.mark.parametrize("one", [0, 1])
 @pytest.mark.parametrize("blocks", [1, 2, 31, 32, 33, 64, 65, 148])
-def test_sums(checker, blocks, one):
-    assert ask(checker, blocks, -1, 1 << 20, one) == ([blocks] * 3, True)
+def test_sums(driver, blocks, one):
+    assert ask(driver, blocks, -1, 1 << 20, one) == ([blocks] * 3, True)
 
 
 @pytest.mark.parametrize("one", [0, 1])
 @pytest.mark.parametrize("blocks,absent", [(2, 0), (2, 1), (32, 0), (32, 31), (33, 32), (33, 0), (64, 40), (64, 1), (148, 147),
                                            (148, 70)])
-def test_a_block_that_never_posts(checker, blocks, absent, one):
+def test_a_block_that_never_posts(driver, blocks, absent, one):
     """no block finishes a round without it"""
-    assert ask(checker, blocks, absent, SHORT, one)[0] == [0, 0, 0]
+    assert ask(driver, blocks, absent, SHORT, one)[0] == [0, 0, 0]
 
 
 @pytest.mark.parametrize("limit", [1, 4, 16, 64])
